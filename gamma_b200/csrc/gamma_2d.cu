@@ -26,19 +26,21 @@ using namespace gb::d2;
 namespace {
 
 constexpr int kThreads = 256;
-// resident blocks per SM asked of the heavy per-cell passes: their FP64 and
-// load latency needs warps more than registers (measured per pass at 512
-// tracks with grids of whole waves: 3 for the theta interfaces and the
-// transverse gradients, 4 for the r interfaces, the theta gather and the cell
-// update)
+// resident blocks per SM asked of the heavy per-cell passes.  The interface
+// passes are straight-line FP64 code (flat_ops.cuh) that overlaps its own
+// quotients and wants registers: at 512 tracks of 4,000 cells, per stage, the r
+// interfaces took 377 us at 2 blocks (3: 411, 4: 470, 1: 591) and the theta
+// interfaces 440 us at 2 (3: 538, 4: 602, 1: 615).  The transverse gradients
+// wait on loads and want warps: 484 us at 4 (3: 542, 2: 625, 1: 1078); so do the
+// theta gather and the cell update.
 #ifndef GB2_MINB_MV
-#define GB2_MINB_MV 4
+#define GB2_MINB_MV 2
 #endif
 #ifndef GB2_MINB_TG
-#define GB2_MINB_TG 3
+#define GB2_MINB_TG 4
 #endif
 #ifndef GB2_MINB_F1
-#define GB2_MINB_F1 3
+#define GB2_MINB_F1 2
 #endif
 #ifndef GB2_MINB_GA
 #define GB2_MINB_GA 4
@@ -231,7 +233,7 @@ __device__ __forceinline__ void cell_at(const Grid2 &G, long long g, int *j, int
        g_ += (long long)gridDim.x * blockDim.x)                                                     \
     if (int j = 0, i = 0; cell_at((G), g_, &j, &i), true)
 
-__global__ void __launch_bounds__(kThreads, GB2_MINB_MV) k_mv(Phys ph, Params2 P, Grid2 G) {
+__global__ void __launch_bounds__(kThreads, GB2_MINB_MV) k_mv(const __grid_constant__ Phys ph, const __grid_constant__ Params2 P, const __grid_constant__ Grid2 G) {
   const long long it = *G.it;
   FOR_LIVE_CELLS(G, j, i) mv_interface(ph, P, G, j, i, it);
 }
@@ -249,7 +251,7 @@ __global__ void k_stale(Grid2 G) {
   if (j <= G.NJ - 2) stale_append(G, j);
 }
 
-__global__ void __launch_bounds__(kThreads, GB2_MINB_TG) k_tgrad(Grid2 G) {
+__global__ void __launch_bounds__(kThreads, GB2_MINB_TG) k_tgrad(const __grid_constant__ Grid2 G) {
   FOR_LIVE_CELLS(G, j, i) trans_grad(G, j, i);
 }
 
@@ -315,7 +317,7 @@ __global__ void k_if_pref(Grid2 G) {
 }
 
 // every theta interface, one per thread (f1_if)
-__global__ void __launch_bounds__(kThreads, GB2_MINB_F1) k_f1if(Phys ph, Grid2 G) {
+__global__ void __launch_bounds__(kThreads, GB2_MINB_F1) k_f1if(const __grid_constant__ Phys ph, const __grid_constant__ Grid2 G) {
   const long long n = G.if_pref[G.NJ];
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x) {
@@ -381,7 +383,7 @@ struct LearnedStart {
 // k_guess_policy2 did not choose returns at once.
 template <bool GUESS>
 __global__ void __launch_bounds__(kThreads, GB2_MINB_UP)
-    k_update(Phys ph, Params2 P, Grid2 G, int stage, Stats2 *S, const float *guess, Policy2 *pol) {
+    k_update(const __grid_constant__ Phys ph, const __grid_constant__ Params2 P, const __grid_constant__ Grid2 G, int stage, Stats2 *S, const float *guess, Policy2 *pol) {
   if (pol && ((pol->use_guess != 0) != GUESS)) return;
   // calls, iterations, fallbacks, max, learned starts, poor warm starts
   unsigned long long c2p[6] = {0, 0, 0, 0, 0, 0};
@@ -465,6 +467,7 @@ Phys phys_of(const gamma_2d_config_t &c) {
   Phys p;
   p.gamma_ad = c.gamma_ad;
   p.kgam = c.gamma_ad / (c.gamma_ad - 1.);
+  p.rgm1 = 1. / (c.gamma_ad - 1.);
   p.cfl = c.cfl;
   p.vi = c.vi;
   p.eos = c.eos;

@@ -153,6 +153,7 @@ gb::Phys phys_of(const gamma_config_t &c) {
   gb::Phys p;
   p.gamma_ad = c.gamma_ad;
   p.kgam = c.gamma_ad / (c.gamma_ad - 1.);
+  p.rgm1 = 1. / (c.gamma_ad - 1.);
   p.cfl = c.cfl;
   p.vi = c.vi;
   p.eos = c.eos;
@@ -179,24 +180,9 @@ int configure_launch(gamma_ctx *c, int v, bool guess, int *grid, size_t *smem) {
 }
 
 template <class Cfg>
-__global__ void cons2prim_kernel(gb::Phys ph, double *cons, double *prim, int n, int *iters) {
-  constexpr int NQ = Cfg::NQ;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    double c[NQ], p[NQ];
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-      c[q] = cons[(long long)q * n + k];
-      p[q] = prim[(long long)q * n + k];
-    }
-    gb::C2PStats st;
-    gb::cons2prim<Cfg>(ph, c, p, &st);  // warm start from prim[PPP]
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-      cons[(long long)q * n + k] = c[q];
-      prim[(long long)q * n + k] = p[q];
-    }
-    if (iters) iters[k] = st.iters;
-  }
+__global__ void cons2prim_kernel(const __grid_constant__ gb::Phys ph, double *cons, double *prim, int n, int *iters) {
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
+    gb::cons2prim_at<Cfg>(ph, cons, prim, n, k, iters, -1.);  // warm start from prim[PPP]
 }
 
 // Grid::printCols' side effect with shock detection (text1d.cpp:135-141):

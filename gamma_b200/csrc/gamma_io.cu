@@ -39,6 +39,7 @@ Phys phys_1d(const gamma_config_t &c) {
   Phys p;
   p.gamma_ad = c.gamma_ad;
   p.kgam = c.gamma_ad / (c.gamma_ad - 1.);
+  p.rgm1 = 1. / (c.gamma_ad - 1.);
   p.cfl = c.cfl;
   p.vi = c.vi;
   p.eos = c.eos;
@@ -52,6 +53,7 @@ Phys phys_2d(const gamma_2d_config_t &c) {
   Phys p;
   p.gamma_ad = c.gamma_ad;
   p.kgam = c.gamma_ad / (c.gamma_ad - 1.);
+  p.rgm1 = 1. / (c.gamma_ad - 1.);
   p.cfl = c.cfl;
   p.vi = c.vi;
   p.eos = c.eos;

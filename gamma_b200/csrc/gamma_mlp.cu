@@ -35,6 +35,7 @@ gb::Phys phys_of(const gamma_config_t &c) {
   gb::Phys p;
   p.gamma_ad = c.gamma_ad;
   p.kgam = c.gamma_ad / (c.gamma_ad - 1.);
+  p.rgm1 = 1. / (c.gamma_ad - 1.);
   p.cfl = c.cfl;
   p.vi = c.vi;
   p.eos = c.eos;
@@ -72,8 +73,7 @@ __global__ void infer_kernel(const float *P, const float *x, long long n, float 
 // cons2prim started from the network's pressure (one warp per 32 cells).
 // cons/prim: [NQ rows][n] in the reference's slot order.
 template <class Cfg>
-__global__ void cons2prim_guess_kernel(gb::Phys ph, const float *P, double *cons, double *prim, int n, int *iters) {
-  constexpr int NQ = Cfg::NQ;
+__global__ void cons2prim_guess_kernel(const __grid_constant__ gb::Phys ph, const float *P, double *cons, double *prim, int n, int *iters) {
   __shared__ gb::mlp::InferSmem s;
   gb::mlp::load_infer_weights(P, s);
   __syncthreads();
@@ -82,29 +82,17 @@ __global__ void cons2prim_guess_kernel(gb::Phys ph, const float *P, double *cons
   for (int base = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32; base < n; base += warps * 32) {
     const int k = base + lane;
     const bool on = k < n;
-    double c[NQ], p[NQ];
     float f[3] = {0.f, 0.f, 0.f}, o[2] = {0.f, 0.f};
+    double D = 0.;
     if (on) {
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) {
-        c[q] = cons[(long long)q * n + k];
-        p[q] = prim[(long long)q * n + k];
-      }
-      gb::mlp::features(c[gb::DEN], c[gb::TAU], c[gb::SS1], f);
+      D = cons[(long long)gb::DEN * n + k];
+      gb::mlp::features(D, cons[(long long)gb::TAU * n + k], cons[(long long)gb::SS1 * n + k], f);
     }
     __syncwarp();
     gb::mlp::infer_warp(s, f, o);
     if (on) {
-      const double pg = gb::mlp::guess_pressure(c[gb::DEN], o[0]);
-      if (isfinite(pg) && pg > 0.) p[gb::PPP] = pg;
-      gb::C2PStats st;
-      gb::cons2prim<Cfg>(ph, c, p, &st);
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) {
-        cons[(long long)q * n + k] = c[q];
-        prim[(long long)q * n + k] = p[q];
-      }
-      if (iters) iters[k] = st.iters;
+      const double pg = gb::mlp::guess_pressure(D, o[0]);
+      gb::cons2prim_at<Cfg>(ph, cons, prim, n, k, iters, isfinite(pg) && pg > 0. ? pg : -1.);
     }
   }
 }

@@ -128,6 +128,7 @@ extern "C" GAMMA_API int gamma_gpu_step_tubes_noalloc(const gamma_config_t *cfg,
   gb::Phys ph{};
   ph.gamma_ad = cfg->gamma_ad;
   ph.kgam = cfg->gamma_ad / (cfg->gamma_ad - 1.);
+  ph.rgm1 = 1. / (cfg->gamma_ad - 1.);
   ph.cfl = cfg->cfl;
   ph.vi = cfg->vi;
   ph.eos = cfg->eos;

@@ -25,6 +25,8 @@
 #define GB_HD_OUTLINE __device__ __noinline__
 #endif
 
+#include "flat_ops.cuh"
+
 namespace gb {
 
 enum { RHO = 0, PPP = 1, UU1 = 2, UU2 = 3 };
@@ -72,13 +74,13 @@ constexpr double DT_INF = 1.e15;
 
 // cartesian + rel_cart, ideal gas, no shock detection / synchrotron: NUM_Q = 6.
 #ifndef GB_CART_MIN_BLOCKS
-#define GB_CART_MIN_BLOCKS 5
+#define GB_CART_MIN_BLOCKS 6
 #endif
 struct CfgCart {
   static constexpr bool FAST = GB_FAST_ARITH != 0;
   static constexpr bool FAST_RIEMANN = GB_FAST_ARITH == 1;
   static constexpr bool FAST_ROOT = GB_FAST_ARITH == 1;
-  static constexpr int MIN_BLOCKS = GB_CART_MIN_BLOCKS;  // 128-thread CTAs per SM (5: 96 registers)
+  static constexpr int MIN_BLOCKS = GB_CART_MIN_BLOCKS;  // 128-thread CTAs per SM (6: 80 registers)
   static constexpr int NQ = 6;
   static constexpr bool SPH = false;    // rel_sph hydro and spherical1D geometry
   static constexpr bool SHOCK = false;  // SHOCK_DETECTION_
@@ -124,6 +126,7 @@ struct RefOrder : Cfg {
 struct Phys {
   double gamma_ad;  // GAMMA_
   double kgam;      // GAMMA_ / (GAMMA_ - 1), the enthalpy factor of the ideal EOS
+  double rgm1;      // 1 / (GAMMA_ - 1)
   double cfl;       // CFL_
   double vi;        // VI
   int eos;          // 0 ideal, 1 Synge / Taub-Mathews (rel_sph.cpp:37-52)
@@ -150,34 +153,41 @@ struct FState {
   double lfac, v;
 };
 
-GB_HD double lfac_of(double uu) {
+template <class Ar>
+GB_HD double lfac_of(Ar &ar, double uu) {
   // fluid.cpp:10-22 (u = sqrt(sum uu^2) then sqrt(1+u^2))
   double u = 0.;
   u += uu * uu;
-  u = sqrt(u);
-  return sqrt(1 + u * u);
+  u = ar.root(u);
+  return ar.root(1 + u * u);
+}
+GB_HD double lfac_of(double uu) {
+  PlainOps ar;
+  return lfac_of(ar, uu);
+}
+
+// The formulas below take their quotients and roots from an operator set Ar
+// (flat_ops.cuh): PlainOps, the operators themselves, or FlatOps, the same
+// results without branches.  The forms without `ar` use PlainOps.
+
+// GAMMA_ - 1 as a divisor (its reciprocal comes from the host)
+template <class Ar>
+GB_HD typename Ar::By by_gm1(Ar &ar, const Phys &ph) {
+  return ar.by_known(ph.gamma_ad - 1., ph.rgm1);
 }
 
 // FluidState::gamma (rel_sph.cpp:37-52)
-GB_HD double eos_gamma(const Phys &ph, double rho, double p) {
+template <class Ar>
+GB_HD double eos_gamma(Ar &ar, const Phys &ph, double rho, double p) {
   const double G = ph.gamma_ad;
   if (ph.eos == 0) return G;
-  double a = p / rho / (G - 1.);
-  double e_ratio = a + sqrt(a * a + 1.);
-  return G - (G - 1.) / 2. * (1. - 1. / (e_ratio * e_ratio));
+  double a = ar.quo(ar.quo(p, ar.by(rho)), by_gm1(ar, ph));
+  double e_ratio = a + ar.root(a * a + 1.);
+  return G - (G - 1.) / 2. * (1. - ar.inv(e_ratio * e_ratio));
 }
-
-// a / b, bit for bit, for quotients whose numerator is often zero (uniform
-// tracers, flat gradients, gas at rest).  With a = +-0 the IEEE quotient is a
-// signed zero (b finite or infinite, nonzero) or NaN (b zero or NaN), which is
-// a * (1 / s) with s = +-1, +-0 or NaN as b's class; the divide then never
-// sees a zero numerator, which sends the whole warp through the division's
-// slow path.
-GB_HD double qdiv(double a, double b) {
-  const bool z = a == 0.;
-  const double s = z ? ((b != 0. && b == b) ? copysign(1., b) : b) : b;
-  const double q = (z ? 1. : a) / s;
-  return z ? a * q : q;
+GB_HD double eos_gamma(const Phys &ph, double rho, double p) {
+  PlainOps ar;
+  return eos_gamma(ar, ph, rho, p);
 }
 
 // 1/x to about 2^-22, for correction terms only
@@ -199,48 +209,67 @@ GB_HD double recip_approx(double x) {
 // to twice the precision, and Dekker's exact product (the FMA form) gives the
 // pair s*q; it is rounded once.  The correction terms need ~20 bits, hence the
 // approximate reciprocal.  Outside [2^-900, 2^900] (or NaN): pow itself.
-GB_HD double pow_3_4(double x) {
-  if (!(x >= 0x1p-900 && x <= 0x1p900)) return pow(x, 0.75);
-  const double s = sqrt(x);
+template <class Ar>
+GB_HD double pow_3_4(Ar &ar, double x) {
+  if (!Ar::FLAT && !(x >= 0x1p-900 && x <= 0x1p900)) return pow(x, 0.75);  // FlatOps::root sees the range
+  const double s = ar.root(x);
   const double sl = fma(-s, s, x) * 0.5 * recip_approx(s);  // sqrt(x) = s + sl
-  const double q = sqrt(s);
+  const double q = ar.root(s);
   const double ql = (fma(-q, q, s) + sl) * 0.5 * recip_approx(q);  // sqrt(s + sl) = q + ql
   const double ph = s * q;
   const double lo = fma(s, q, -ph) + (s * ql + sl * q);
   return ph + lo;
 }
+GB_HD double pow_3_4(double x) {
+  PlainOps ar;
+  return pow_3_4(ar, x);
+}
 
 // (p/p1)^(1/GAMMA_) of the isentrope
-GB_HD double isentrope_pow(double x, double ginv) { return ginv == 0.75 ? pow_3_4(x) : pow(x, ginv); }
+template <class Ar>
+GB_HD double isentrope_pow(Ar &ar, double x, double ginv) {
+  return ginv == 0.75 ? pow_3_4(ar, x) : pow(x, ginv);
+}
 
+template <class Cfg, class Ar>
+GB_HD double state_gamma(Ar &ar, const Phys &ph, const double *prim) {
+  return Cfg::SPH ? eos_gamma(ar, ph, prim[RHO], prim[PPP]) : ph.gamma_ad;
+}
 template <class Cfg>
 GB_HD double state_gamma(const Phys &ph, const double *prim) {
-  return Cfg::SPH ? eos_gamma(ph, prim[RHO], prim[PPP]) : ph.gamma_ad;
+  PlainOps ar;
+  return state_gamma<Cfg>(ar, ph, prim);
+}
+
+// a state's Gamma - 1 as a divisor
+template <class Cfg, class Ar>
+GB_HD typename Ar::By by_state_gm1(Ar &ar, const Phys &ph, double gma) {
+  return Cfg::SPH && ph.eos != 0 ? ar.by(gma - 1.) : by_gm1(ar, ph);
 }
 
 // gamma/(gamma-1) of a state: cached for the ideal EOS
-template <class Cfg>
-GB_HD double enth_k(const Phys &ph, const double *prim) {
+template <class Cfg, class Ar>
+GB_HD double enth_k(Ar &ar, const Phys &ph, const double *prim) {
   if (Cfg::SPH && ph.eos != 0) {
-    const double g = eos_gamma(ph, prim[RHO], prim[PPP]);
-    return g / (g - 1.);
+    const double g = eos_gamma(ar, ph, prim[RHO], prim[PPP]);
+    return ar.quo(g, ar.by(g - 1.));
   }
   return ph.kgam;
 }
 
 // prim2cons (rel_sph.cpp:55-82, rel_cart.cpp:37-64)
-template <class Cfg>
-GB_HD void prim2cons(const Phys &ph, const double *prim, double *cons) {
+template <class Cfg, class Ar>
+GB_HD void prim2cons(Ar &ar, const Phys &ph, const double *prim, double *cons) {
   double rho = prim[RHO];
   double p = prim[PPP];
   double uu = prim[UU1];
-  double lfac = lfac_of(uu);
+  double lfac = lfac_of(ar, uu);
   double h;
   if (Cfg::FAST) {
-    h = 1. + enth_k<Cfg>(ph, prim) * p / rho;
+    h = 1. + ar.quo(enth_k<Cfg>(ar, ph, prim) * p, ar.by(rho));
   } else {
-    const double gma = state_gamma<Cfg>(ph, prim);
-    h = 1. + p * gma / (gma - 1.) / rho;
+    const double gma = state_gamma<Cfg>(ar, ph, prim);
+    h = 1. + ar.quo(ar.quo(p * gma, by_state_gm1<Cfg>(ar, ph, gma)), ar.by(rho));
   }
   double D = lfac * rho;
   double tau = D * h * lfac - p - D;
@@ -252,25 +281,30 @@ GB_HD void prim2cons(const Phys &ph, const double *prim, double *cons) {
 #pragma unroll
   for (int t = TR1; t < Cfg::NQ; ++t) cons[t] = prim[t] * D;
 }
+template <class Cfg>
+GB_HD void prim2cons(const Phys &ph, const double *prim, double *cons) {
+  PlainOps ar;
+  prim2cons<Cfg>(ar, ph, prim, cons);
+}
 
 // prim2cons + state2flux of a reconstructed or cell state in one pass
 // (rel_sph.cpp:55-113): lfac and v = u/lfac are formed once.
-template <class Cfg>
-GB_HD void state2flux(const double *prim, const double *cons, double *flux);
+template <class Cfg, class Ar>
+GB_HD void state2flux(Ar &ar, const double *prim, const double *cons, double *flux);
 
-template <class Cfg>
-GB_HD void fill_state(const Phys &ph, FState<Cfg> &S) {
+template <class Cfg, class Ar>
+GB_HD void fill_state(Ar &ar, const Phys &ph, FState<Cfg> &S) {
   if (!Cfg::FAST) {
-    prim2cons<Cfg>(ph, S.prim, S.cons);
-    state2flux<Cfg>(S.prim, S.cons, S.flux);
-    S.lfac = lfac_of(S.prim[UU1]);
-    S.v = qdiv(S.prim[UU1], S.lfac);
+    prim2cons<Cfg>(ar, ph, S.prim, S.cons);
+    state2flux<Cfg>(ar, S.prim, S.cons, S.flux);
+    S.lfac = lfac_of(ar, S.prim[UU1]);
+    S.v = ar.quo0(S.prim[UU1], ar.by(S.lfac));
     return;
   }
   const double rho = S.prim[RHO], p = S.prim[PPP], uu = S.prim[UU1];
-  const double lfac = sqrt(1. + uu * uu);
-  const double v = uu / lfac;
-  const double h = 1. + enth_k<Cfg>(ph, S.prim) * p / rho;
+  const double lfac = ar.root(1. + uu * uu);
+  const double v = ar.quo(uu, ar.by(lfac));
+  const double h = 1. + ar.quo(enth_k<Cfg>(ar, ph, S.prim) * p, ar.by(rho));
   const double D = lfac * rho;
   const double Dh = D * h;
   S.lfac = lfac;
@@ -291,19 +325,19 @@ GB_HD void fill_state(const Phys &ph, FState<Cfg> &S) {
 }
 
 // state2flux (rel_sph.cpp:85-113, rel_cart.cpp:67-95)
-template <class Cfg>
-GB_HD void state2flux(const double *prim, const double *cons, double *flux) {
+template <class Cfg, class Ar>
+GB_HD void state2flux(Ar &ar, const double *prim, const double *cons, double *flux) {
   double p = prim[PPP];
   double uu = prim[UU1];
-  double lfac = lfac_of(uu);
+  const auto lfac = ar.by(lfac_of(ar, uu));
   double D = cons[DEN];
   double ss = cons[SS1];
-  flux[DEN] = qdiv(D * uu, lfac);
-  flux[SS1] = qdiv(ss * uu, lfac) + p;
+  flux[DEN] = ar.quo0(D * uu, lfac);
+  flux[SS1] = ar.quo0(ss * uu, lfac) + p;
   flux[SS2] = 0.;
-  flux[TAU] = ss - qdiv(D * uu, lfac);
+  flux[TAU] = ss - flux[DEN];
 #pragma unroll
-  for (int t = TR1; t < Cfg::NQ; ++t) flux[t] = qdiv(cons[t] * uu, lfac);
+  for (int t = TR1; t < Cfg::NQ; ++t) flux[t] = ar.quo0(cons[t] * uu, lfac);
 }
 
 // ---------------------------------------------------------------------------
@@ -371,152 +405,165 @@ GB_HD double c2p_f(const Phys &ph, double p, double D, double S2, double E, doub
   return f;
 }
 
-// f in the reference's operation order (rel_sph.cpp:198-207, rel_cart.cpp:118-120),
-// with df/dp and lfac^2 on request.
-template <class Cfg>
-GB_HD double c2p_f_ref(const Phys &ph, double p, double D, double S, double E, double *df = nullptr,
-                       double *l2out = nullptr, double *lfac_out = nullptr, bool p_may_be_zero = false) {
+// f(p) and, on request, its slope; lfac and lfac^2 at p, and whether
+// 1 - S^2/W^2 was not negative there (else lfac is that of its magnitude).
+struct C2PEval {
+  double f, df, lfac, l2;
+  bool inside;
+};
+
+// f in the reference's operation order (rel_sph.cpp:198-207, rel_cart.cpp:118-120).
+template <class Cfg, class Ar>
+GB_HD C2PEval c2p_f_ref(Ar &ar, const Phys &ph, double p, double D, double S, double E, bool slope,
+                        bool p_may_be_zero = false) {
+  C2PEval e;
   const double W = E + p;
-  const double x = qdiv(S * S, W * W);
+  const double x = ar.quo0(S * S, ar.by(W * W));
   const double arg = Cfg::SPH ? fabs(1. - x) : (1. - x);
-  const double lfac = 1. / sqrt(arg);
+  const double lfac = ar.rroot(arg);
   const bool ideal = !Cfg::SPH || ph.eos == 0;
-  const double gma = ideal ? ph.gamma_ad : eos_gamma(ph, D / lfac, p);
+  const double gma = ideal ? ph.gamma_ad : eos_gamma(ar, ph, ar.quo(D, ar.by(lfac)), p);
+  const auto gm1 = ideal ? by_gm1(ar, ph) : ar.by(gma - 1.);
   // p = 0 at the bracket's lower end p_lo, which every search evaluates
   const double kp = gma * p * lfac * lfac;
-  const double f = (E + p - D * lfac - (p_may_be_zero ? qdiv(kp, gma - 1.) : kp / (gma - 1.)));
-  if (df) {
+  e.f = (E + p - D * lfac - (p_may_be_zero ? ar.quo0(kp, gm1) : ar.quo(kp, gm1)));
+  e.l2 = lfac * lfac;
+  e.lfac = lfac;
+  e.inside = arg >= 0.;
+  e.df = 0.;
+  if (slope) {
     if (!ideal) {  // Gamma_eff(p) terms: take them from the derivative form
       double dfast;
       c2p_f<Cfg>(ph, p, D, S * S, E, &dfast);
-      *df = dfast;
+      e.df = dfast;
     } else {  // d lfac/dp = -lfac^3 x / W with the same lfac and x as f
       const double sgn = (1. - x) >= 0. ? 1. : -1.;
-      const double l2 = lfac * lfac;
-      const double dl = qdiv(-sgn * lfac * l2 * x, W);
+      const double dl = ar.quo0(-sgn * lfac * e.l2 * x, ar.by(W));
       // kgam is GAMMA_/(GAMMA_-1) rounded once on the host: gma/(gma-1) exactly
-      *df = 1. - D * dl - ph.kgam * (l2 + 2. * p * lfac * dl);
+      e.df = 1. - D * dl - ph.kgam * (e.l2 + 2. * p * lfac * dl);
     }
   }
-  if (l2out) *l2out = lfac * lfac;
-  if (lfac_out) *lfac_out = arg >= 0. ? lfac : -1.;  // -1: no lfac of fabs(1 - x) here
-  return f;
+  return e;
 }
+
+// What the root search returns: the pressure the reference would go on with
+// (the starting one where it finds none) and the Lorentz factor
+// 1/sqrt(|1 - S^2/(E+p)^2|) there when the search evaluated f at it (the same
+// rounding as f's), else -1; then its statistics (C2PStats).
+struct C2PRoot {
+  double p, lfac;
+  C2PStats st;
+};
 
 // Pressure root of the cons2prim driver (rel_sph.cpp:243-286): the bracket,
 // its no-solution tests and the warm start pCand are the reference's; the
-// Brent search is replaced by safeguarded Newton-Raphson.  Returns the
-// pressure the reference would go on with (pCand itself where it finds none).
+// Brent search is replaced by safeguarded Newton-Raphson.
 //
-// lfac_at (optional): the Lorentz factor 1/sqrt(|1 - S^2/(E+p)^2|) at the
-// returned pressure when the search evaluated f there (the same rounding as
-// f's), else -1.
-//
-// defer (with st): where a search is needed and the warm start is poor
-// (c2p_warm_start_poor), stop before it and set st->deferred; the caller then
+// defer: where a search is needed and the warm start is poor
+// (c2p_warm_start_poor), stop before it and set st.deferred; the caller then
 // starts the search again from a better pressure (the learned guess).
-template <class Cfg>
-GB_HD double c2p_pressure_body(const Phys &ph, double D, double S, double S2, double E, double pCand,
-                               C2PStats *st, double *lfac_at, bool defer) {
-  auto fval = [&](double p, double *df, double *l2, double *lf, bool p_may_be_zero = false) -> double {
-    return Cfg::FAST_ROOT ? c2p_f<Cfg>(ph, p, D, S2, E, df, l2)
-                     : c2p_f_ref<Cfg>(ph, p, D, S, E, df, l2, lf, p_may_be_zero);
+//
+// With FlatOps the result counts only if !ar.bad(); the loops stop early where
+// it is set.
+template <class Cfg, class Ar>
+GB_HD C2PRoot c2p_pressure_body(Ar &ar, const Phys &ph, double D, double S, double S2, double E, double pCand,
+                                bool defer) {
+  auto feval = [&](double p, bool slope, bool p_may_be_zero = false) -> C2PEval {
+    if (!Cfg::FAST_ROOT) return c2p_f_ref<Cfg>(ar, ph, p, D, S, E, slope, p_may_be_zero);
+    C2PEval e;
+    e.f = c2p_f<Cfg>(ph, p, D, S2, E, slope ? &e.df : nullptr, &e.l2);
+    e.lfac = sqrt(e.l2);
+    e.inside = false;
+    return e;
   };
-  int iters = 0, fallback = 0;
+  C2PRoot R;
+  R.st = C2PStats{0, 0, 0, 0};
   // f at the warm start, with its slope: the search starts there when the
   // warm start lies in the bracket (f does not depend on whether df is asked for)
-  double df0, l20, lf0 = -1.;
-  const double f_init = fval(pCand, &df0, &l20, &lf0);
-  if (lfac_at) *lfac_at = lf0;
+  C2PEval e0 = feval(pCand, true);
+  R.p = pCand;
+  R.lfac = e0.inside ? e0.lfac : -1.;
   // rel_cyl.cpp:161 searches only where |f| exceeds 1e-13 (rel_sph, rel_cart: 0)
-  int poor = 0;
-  if (fabs(f_init) > (Cfg::CYL ? 1.e-13 : 0.)) {
-    poor = c2p_warm_start_poor(f_init, df0, pCand);
-    if (defer && st && poor) {
-      st->iters = 0;
-      st->fallback = 0;
-      st->deferred = 1;
-      st->poor = 1;
-      return pCand;
+  if (fabs(e0.f) > (Cfg::CYL ? 1.e-13 : 0.)) {
+    R.st.poor = c2p_warm_start_poor(e0.f, e0.df, pCand);
+    if (defer && R.st.poor) {
+      R.st.deferred = 1;
+      return R;
     }
     double p_lo = fmax(0., (1. + 1e-13) * S - E);
     bool find_p = true;
-    if (fval(p_lo, nullptr, nullptr, nullptr, true) < 0) find_p = false;
+    if (feval(p_lo, false, true).f < 0) find_p = false;
     double p_hi;
-    if (f_init < 0) {
+    if (e0.f < 0) {
       p_hi = 1. * pCand;
     } else {
       p_hi = pCand;
       // the reference grows p_hi without bound (a zero guess would never end);
       // 400 decades reach infinity, where f is NaN and the loop stops anyway.
-      // Its first test re-evaluates f(pCand), which is f_init.
-      for (int g = 0; g < 400 && (g == 0 ? f_init : fval(p_hi, nullptr, nullptr, nullptr)) > 0; ++g) p_hi *= 10;
+      // Its first test re-evaluates f(pCand), which is e0.f.
+      for (int g = 0; g < 400 && (g == 0 ? e0.f : feval(p_hi, false).f) > 0; ++g) {
+        p_hi *= 10;
+        if (Ar::FLAT && ar.bad()) break;
+      }
     }
     if (p_hi < p_lo) find_p = false;
     if (find_p) {
       // f(lo) >= 0 >= f(hi).  The warm start tightens one side.
       double lo = p_lo, hi = p_hi;
-      if (f_init > 0.) lo = fmax(lo, pCand);
+      if (e0.f > 0.) lo = fmax(lo, pCand);
       double p = fmin(fmax(pCand, lo), hi);
-      double df = df0, l2 = l20, lf = lf0;
-      double f = f_init;
-      if (!(p == pCand)) f = fval(p, &df, &l2, &lf);
+      if (!(p == pCand)) e0 = feval(p, true);
       const int MAXIT = 100;
       const double eps = 2.220446049250313e-16;
+      int iters;
       for (iters = 1; iters <= MAXIT; ++iters) {
         // Rounding noise of f: E, p, D lfac and k p lfac^2 cancel, and lfac
         // itself carries eps*lfac^2 relative error from 1 - S^2/W^2.  Below
         // this level the sign of f is noise and p is as good as it gets.
-        const double noise = eps * (E + p + D * sqrt(l2) * (1. + l2) + 4. * p * l2 * (1. + 2. * l2));
-        if (f == 0. || fabs(f) <= noise) break;
-        double pn = p - f / df;
+        // (lfac is sqrt(l2): the root of a rounded square is exact.)
+        const double noise =
+            eps * (E + p + D * e0.lfac * (1. + e0.l2) + 4. * p * e0.l2 * (1. + 2. * e0.l2));
+        if (e0.f == 0. || fabs(e0.f) <= noise) break;
+        double pn = p - ar.quo(e0.f, ar.by(e0.df));
         if (!(pn > lo && pn < hi)) {
           // Newton left the bracket: bisect, geometrically once lo > 0
           pn = lo > 0. ? sqrt(lo) * sqrt(hi) : 0.5 * (lo + hi);
           if (!(pn > lo && pn < hi)) pn = 0.5 * (lo + hi);
         }
-        double dfn, l2n, lfn;
-        const double fn = fval(pn, &dfn, &l2n, &lfn);
-        if (fn > 0.) lo = pn;
-        else if (fn < 0.) hi = pn;
+        e0 = feval(pn, true);
+        if (e0.f > 0.) lo = pn;
+        else if (e0.f < 0.) hi = pn;
         const double step = fabs(pn - p);
         p = pn;
-        f = fn;
-        df = dfn;
-        l2 = l2n;
-        lf = lfn;
-        if (fn == 0. || step <= 1.e-14 * pn || (hi - lo) <= 1.e-14 * hi) break;
+        if (e0.f == 0. || step <= 1.e-14 * pn || (hi - lo) <= 1.e-14 * hi) break;
+        if (Ar::FLAT && ar.bad()) break;
       }
-      if (iters > MAXIT) fallback = 1;
-      pCand = p;
-      if (lfac_at) *lfac_at = lf;
+      R.st.iters = iters;
+      if (iters > MAXIT) R.st.fallback = 1;
+      R.p = p;
+      R.lfac = e0.inside ? e0.lfac : -1.;
     }
   }
-  if (st) {
-    st->iters = iters;
-    st->fallback = fallback;
-    st->deferred = 0;
-    st->poor = poor;
-  }
-  return pCand;
+  return R;
 }
 
 template <class Cfg>
-GB_HD_OUTLINE double c2p_pressure_outline(const Phys &ph, double D, double S, double S2, double E, double pCand,
-                                          C2PStats *st, double *lfac_at, bool defer) {
-  return c2p_pressure_body<Cfg>(ph, D, S, S2, E, pCand, st, lfac_at, defer);
+GB_HD_OUTLINE C2PRoot c2p_pressure_outline(const Phys &ph, double D, double S, double S2, double E, double pCand,
+                                           bool defer) {
+  PlainOps ar;
+  return c2p_pressure_body<Cfg>(ar, ph, D, S, S2, E, pCand, defer);
 }
 
-// The cartesian step calls the search from one out-of-line copy: inlined at
-// every call site of the fused step kernel it crowds the instruction cache
-// (3% slower).  The spherical kernels, the 2D passes and the batch cons2prim
-// keep it inline, which is as fast or faster there.  OUTLINE forces the
-// out-of-line copy (a second, rarely taken call site).
-template <class Cfg, bool OUTLINE = !Cfg::SPH>
-GB_HD double c2p_pressure(const Phys &ph, double D, double S, double S2, double E, double pCand, C2PStats *st,
-                          double *lfac_at = nullptr, bool defer = false) {
-  if (!OUTLINE) return c2p_pressure_body<Cfg>(ph, D, S, S2, E, pCand, st, lfac_at, defer);
-  return c2p_pressure_outline<Cfg>(ph, D, S, S2, E, pCand, st, lfac_at, defer);
+// The step with the learned guess, and formulas formed again with PlainOps,
+// call the cartesian search from one out-of-line copy: inlined at every call
+// site of the fused step kernel it crowds the instruction cache.  OUTLINE
+// forces the out-of-line copy (a second, rarely taken call site).  FlatOps
+// searches are inline: a call would end their straight-line code.
+template <class Cfg, bool OUTLINE, class Ar>
+GB_HD C2PRoot c2p_pressure(Ar &ar, const Phys &ph, double D, double S, double S2, double E, double pCand,
+                           bool defer = false) {
+  if (Ar::FLAT || !OUTLINE) return c2p_pressure_body<Cfg>(ar, ph, D, S, S2, E, pCand, defer);
+  return c2p_pressure_outline<Cfg>(ph, D, S, S2, E, pCand, defer);
 }
 
 // What cons2prim's root search is given: D, E = D + tau, S and S^2 of the
@@ -525,8 +572,8 @@ struct C2PInput {
   double D, E, ss, S2, S, pCand;
 };
 
-template <class Cfg>
-GB_HD C2PInput c2p_input(const double *cons, const double *prim) {
+template <class Cfg, class Ar>
+GB_HD C2PInput c2p_input(Ar &ar, const double *cons, const double *prim) {
   C2PInput in;
   in.D = cons[DEN];
   const double tau = cons[TAU];
@@ -535,7 +582,7 @@ GB_HD C2PInput c2p_input(const double *cons, const double *prim) {
   double S2 = 0.;
   S2 += in.ss * in.ss;
   in.S2 = S2;
-  in.S = Cfg::FAST_ROOT ? fabs(in.ss) : sqrt(S2);
+  in.S = Cfg::FAST_ROOT ? fabs(in.ss) : ar.root(S2);
   in.pCand = Cfg::SPH ? fmax(1.e-13, prim[PPP]) : prim[PPP];
   return in;
 }
@@ -550,16 +597,17 @@ GB_HD C2PInput c2p_input(const double *cons, const double *prim) {
 // (st->deferred, c2p_pressure_body) and prim and cons are left as they were,
 // for a second call from a better starting pressure.  OUTLINE: the search's
 // out-of-line copy (c2p_pressure).
-template <class Cfg, class Hooks = gamma_problem::Problem, bool OUTLINE = !Cfg::SPH>
-GB_HD void cons2prim(const Phys &ph, double *cons, double *prim, C2PStats *st, const double *par = nullptr,
+template <class Cfg, class Hooks = gamma_problem::Problem, bool OUTLINE = !Cfg::SPH, class Ar>
+GB_HD void cons2prim(Ar &ar, const Phys &ph, double *cons, double *prim, C2PStats *st, const double *par = nullptr,
                      bool defer = false) {
-  const C2PInput in = c2p_input<Cfg>(cons, prim);
+  const C2PInput in = c2p_input<Cfg>(ar, cons, prim);
   const double D = in.D, E = in.E, ss = in.ss, S2 = in.S2, S = in.S;
-  double lf_root = -1.;
-  const double pCand = c2p_pressure<Cfg, OUTLINE>(ph, D, S, S2, E, in.pCand, st, &lf_root, defer);
-  if (defer && st && st->deferred) return;
+  const C2PRoot root = c2p_pressure<Cfg, OUTLINE>(ar, ph, D, S, S2, E, in.pCand, defer);
+  if (st) *st = root.st;
+  if (defer && root.st.deferred) return;
 
-  double p = pCand;
+  const double lf_root = root.lfac;
+  double p = root.p;
   double rho, uu;
   if (Cfg::FAST_ROOT) {  // lfac = W/sqrt(W^2-S^2), rho = D/lfac, u = lfac v S_i/S with v = S/W
     const double rW = 1. / (E + p);
@@ -573,14 +621,14 @@ GB_HD void cons2prim(const Phys &ph, double *cons, double *prim, C2PStats *st, c
     double lfac = lf_root;
     if (!(lfac > 0. && S * S == S2)) {
       double Ep2 = (E + p) * (E + p);
-      double v2 = qdiv(S2, Ep2);
-      lfac = 1. / sqrt(fabs(1. - v2));
+      double v2 = ar.quo0(S2, ar.by(Ep2));
+      lfac = ar.rroot(fabs(1. - v2));
     }
-    rho = D / lfac;
+    rho = ar.quo(D, ar.by(lfac));
     if (Cfg::CYL ? fabs(S) < 1.e-14 : fabs(S) == 0.) {  // rel_cyl.cpp:207
       uu = 0;
     } else {
-      double v = sqrt(1. - 1. / (lfac * lfac));
+      double v = ar.root(1. - ar.inv(lfac * lfac));
       // ss/S is exactly +-1 when S == |ss|
       uu = lfac * v * (fabs(ss) == S ? (ss > 0. ? 1. : -1.) : ss / S);
     }
@@ -592,15 +640,58 @@ GB_HD void cons2prim(const Phys &ph, double *cons, double *prim, C2PStats *st, c
   prim[UU1] = uu;
   prim[UU2] = 0.;
   if (Cfg::FAST) {
-    const double rD = 1. / D;
+    const double rD = ar.inv(D);
 #pragma unroll
     for (int t = TR1; t < Cfg::NQ; ++t) prim[t] = cons[t] * rD;
   } else {
+    const auto byD = ar.by(D);
 #pragma unroll
-    for (int t = TR1; t < Cfg::NQ; ++t) prim[t] = qdiv(cons[t], D);
+    for (int t = TR1; t < Cfg::NQ; ++t) prim[t] = ar.quo0(cons[t], byD);
   }
-  prim2cons<Cfg>(ph, prim, cons);
+  prim2cons<Cfg>(ar, ph, prim, cons);
 }
+template <class Cfg, class Hooks = gamma_problem::Problem, bool OUTLINE = !Cfg::SPH>
+GB_HD void cons2prim(const Phys &ph, double *cons, double *prim, C2PStats *st, const double *par = nullptr,
+                     bool defer = false) {
+  PlainOps ar;
+  cons2prim<Cfg, Hooks, OUTLINE>(ar, ph, cons, prim, st, par, defer);
+}
+
+#ifdef __CUDACC__
+// State k of a batch (cons, prim: [NQ rows][n] in the reference's slot order),
+// from its own pressure or, if positive, from p0.
+template <class Cfg, class Ar>
+GB_HD bool cons2prim_at_ops(const Phys &ph, double *cons, double *prim, int n, int k, int *iters, double p0) {
+  constexpr int NQ = Cfg::NQ;
+  Ar ar;
+  double c[NQ], p[NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
+    c[q] = cons[(long long)q * n + k];
+    p[q] = prim[(long long)q * n + k];
+  }
+  if (p0 > 0.) p[PPP] = p0;
+  C2PStats st;
+  cons2prim<Cfg, gamma_problem::Problem, false>(ar, ph, c, p, &st);
+  if (ar.bad()) return false;  // nothing written yet
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
+    cons[(long long)q * n + k] = c[q];
+    prim[(long long)q * n + k] = p[q];
+  }
+  if (iters) iters[k] = st.iters;
+  return true;
+}
+template <class Cfg>
+GB_HD_OUTLINE void cons2prim_at_plain(const Phys &ph, double *cons, double *prim, int n, int k, int *iters, double p0) {
+  cons2prim_at_ops<Cfg, PlainOps>(ph, cons, prim, n, k, iters, p0);
+}
+template <class Cfg>
+GB_HD void cons2prim_at(const Phys &ph, double *cons, double *prim, int n, int k, int *iters, double p0) {
+  if (!cons2prim_at_ops<Cfg, FlatOps>(ph, cons, prim, n, k, iters, p0))
+    cons2prim_at_plain<Cfg>(ph, cons, prim, n, k, iters, p0);
+}
+#endif  // __CUDACC__
 
 // ---------------------------------------------------------------------------
 // Riemann problem at a moving interface
@@ -611,26 +702,29 @@ struct Waves {
 
 // Interface::wavespeedEstimates + computeLambda (rel_sph.cpp:322-394;
 // rel_cart.cpp:260-302 switches to the linear root when |FhllE| < 1e-15).
-template <class Cfg>
-GB_HD Waves compute_lambda_ref(const Phys &ph, const FState<Cfg> &L, const FState<Cfg> &R) {
+template <class Cfg, class Ar>
+GB_HD Waves compute_lambda_ref(Ar &ar, const Phys &ph, const FState<Cfg> &L, const FState<Cfg> &R) {
   const bool ws = Cfg::SPH && ph.eos_ws;
-  const double GL = ws ? eos_gamma(ph, L.prim[RHO], L.prim[PPP]) : ph.gamma_ad;
-  const double GR = ws ? eos_gamma(ph, R.prim[RHO], R.prim[PPP]) : ph.gamma_ad;
+  const double GL = ws ? eos_gamma(ar, ph, L.prim[RHO], L.prim[PPP]) : ph.gamma_ad;
+  const double GR = ws ? eos_gamma(ar, ph, R.prim[RHO], R.prim[PPP]) : ph.gamma_ad;
   Waves w;
   double lfacL = L.lfac;
   double lfacR = R.lfac;
   double vL = L.v;
   double vR = R.v;
-  double cSL = sqrt(GL * L.prim[PPP] / (L.prim[RHO] + L.prim[PPP] * GL / (GL - 1.)));
-  double cSR = sqrt(GR * R.prim[PPP] / (R.prim[RHO] + R.prim[PPP] * GR / (GR - 1.)));
-  double sgSL = cSL * cSL / (lfacL * lfacL * (1. - cSL * cSL));
-  double sgSR = cSR * cSR / (lfacR * lfacR * (1. - cSR * cSR));
+  const auto gm1L = ws ? ar.by(GL - 1.) : by_gm1(ar, ph), gm1R = ws ? ar.by(GR - 1.) : by_gm1(ar, ph);
+  double cSL = ar.root(ar.quo(GL * L.prim[PPP], ar.by(L.prim[RHO] + ar.quo(L.prim[PPP] * GL, gm1L))));
+  double cSR = ar.root(ar.quo(GR * R.prim[PPP], ar.by(R.prim[RHO] + ar.quo(R.prim[PPP] * GR, gm1R))));
+  double sgSL = ar.quo(cSL * cSL, ar.by(lfacL * lfacL * (1. - cSL * cSL)));
+  double sgSR = ar.quo(cSR * cSR, ar.by(lfacR * lfacR * (1. - cSR * cSR)));
+  const double rtL = ar.root(sgSL * (1. - vL * vL + sgSL)), rtR = ar.root(sgSR * (1. - vR * vR + sgSR));
+  const auto nL = ar.by(1. + sgSL), nR = ar.by(1. + sgSR);
   double l1, l2;
-  l1 = (vR - sqrt(sgSR * (1. - vR * vR + sgSR))) / (1. + sgSR);
-  l2 = (vL - sqrt(sgSL * (1. - vL * vL + sgSL))) / (1. + sgSL);
+  l1 = ar.quo(vR - rtR, nR);
+  l2 = ar.quo(vL - rtL, nL);
   w.lL = fmin(l1, l2);
-  l1 = (vR + sqrt(sgSR * (1. - vR * vR + sgSR))) / (1. + sgSR);
-  l2 = (vL + sqrt(sgSL * (1. - vL * vL + sgSL))) / (1. + sgSL);
+  l1 = ar.quo(vR + rtR, nR);
+  l2 = ar.quo(vL + rtL, nL);
   w.lR = fmax(l1, l2);
 
   const double lL = w.lL, lR = w.lR;
@@ -644,25 +738,26 @@ GB_HD Waves compute_lambda_ref(const Phys &ph, const FState<Cfg> &L, const FStat
   double AR = lR * ER - mmR;
   double BL = mmL * (lL - vL) - pL;
   double BR = mmR * (lR - vR) - pR;
-  double FhllE = qdiv(lL * AR - lR * AL, lR - lL);
-  double Ehll = (AR - AL) / (lR - lL);
-  double Fhllm = (lL * BR - lR * BL) / (lR - lL);
-  double mhll = qdiv(BR - BL, lR - lL);
+  const auto dl = ar.by(lR - lL);
+  double FhllE = ar.quo0(lL * AR - lR * AL, dl);
+  double Ehll = ar.quo(AR - AL, dl);
+  double Fhllm = ar.quo(lL * BR - lR * BL, dl);
+  double mhll = ar.quo0(BR - BL, dl);
   bool linear = Cfg::SPH ? (fabs(FhllE) == 0) : (fabs(FhllE) < 1.e-15);
   if (linear) {
-    w.lS = qdiv(mhll, Ehll + Fhllm);
+    w.lS = ar.quo0(mhll, ar.by(Ehll + Fhllm));
   } else {
     // pow(x, 2.) of the C library is the correctly rounded square: x*x
     const double ef = Ehll + Fhllm;
     double delta = ef * ef - 4. * FhllE * mhll;
-    w.lS = ((Ehll + Fhllm) - sqrt(delta)) / (2. * FhllE);
+    w.lS = ar.quo((Ehll + Fhllm) - ar.root(delta), ar.by(2. * FhllE));
   }
   return w;
 }
 
-template <class Cfg>
-GB_HD Waves compute_lambda(const Phys &ph, const FState<Cfg> &L, const FState<Cfg> &R) {
-  if (!Cfg::FAST_RIEMANN || ph.eos_ws) return compute_lambda_ref<Cfg>(ph, L, R);
+template <class Cfg, class Ar>
+GB_HD Waves compute_lambda(Ar &ar, const Phys &ph, const FState<Cfg> &L, const FState<Cfg> &R) {
+  if (!Cfg::FAST_RIEMANN || ph.eos_ws) return compute_lambda_ref<Cfg>(ar, ph, L, R);
   const double G = ph.gamma_ad;
   const double kg = ph.kgam;
   Waves w;
@@ -706,8 +801,8 @@ GB_HD Waves compute_lambda(const Phys &ph, const FState<Cfg> &L, const FState<Cf
 // HLLC flux F - vU in the frame of an interface moving at v, times dA
 // (hllc.cpp:12-39 with starState rel_sph.cpp:397-450).  The four branch tests
 // are independent ifs in the reference and stay so.
-template <class Cfg>
-GB_HD void hllc_flux(const FState<Cfg> &L, const FState<Cfg> &R, const Waves &w, double v, double dA,
+template <class Cfg, class Ar>
+GB_HD void hllc_flux(Ar &ar, const FState<Cfg> &L, const FState<Cfg> &R, const Waves &w, double v, double dA,
                      double *flux) {
   const double lS = w.lS;
   auto star = [&](const FState<Cfg> &Sin, double lbda, double *out_cons) {
@@ -718,17 +813,18 @@ GB_HD void hllc_flux(const FState<Cfg> &L, const FState<Cfg> &R, const Waves &w,
     const double E = Sin.cons[TAU] + Sin.cons[DEN];
     const double A = lbda * E - m;
     const double B = m * (lbda - vv) - p;
-    const double pS = (A * lS - B) / (1. - lbda * lS);
+    const double pS = ar.quo(A * lS - B, ar.by(1. - lbda * lS));
     double k;
     if (Cfg::FAST) {
-      const double rk = 1. / (lbda - lS);
+      const double rk = ar.inv(lbda - lS);
       k = (lbda - vv) * rk;
       out_cons[SS1] = (m * (lbda - vv) + pS - p) * rk;
       out_cons[TAU] = (E * (lbda - vv) + pS * lS - p * vv) * rk - D * k;
     } else {  // rel_sph.cpp:433-442
-      k = (lbda - vv) / (lbda - lS);
-      out_cons[SS1] = (m * (lbda - vv) + pS - p) / (lbda - lS);
-      out_cons[TAU] = (E * (lbda - vv) + pS * lS - p * vv) / (lbda - lS) - D * k;
+      const auto dl = ar.by(lbda - lS);
+      k = ar.quo(lbda - vv, dl);
+      out_cons[SS1] = ar.quo(m * (lbda - vv) + pS - p, dl);
+      out_cons[TAU] = ar.quo(E * (lbda - vv) + pS * lS - p * vv, dl) - D * k;
     }
     out_cons[DEN] = D * k;
     out_cons[SS2] = 0.;
@@ -762,42 +858,46 @@ GB_HD void hllc_flux(const FState<Cfg> &L, const FState<Cfg> &R, const Waves &w,
 // ---------------------------------------------------------------------------
 // Shock detector (radiation_sph.cpp:41-158), forward direction.  Returns false
 // (and leaves *pspec alone) where the reference returns -1 early.
-template <class Cfg>
-GB_HD bool compute_Sd(const Phys &ph, const FState<Cfg> &S1, const FState<Cfg> &S2, double *Sd,
+template <class Cfg, class Ar>
+GB_HD bool compute_Sd(Ar &ar, const Phys &ph, const FState<Cfg> &S1, const FState<Cfg> &S2, double *Sd,
                       double *pspec) {
   // with eos_ws, the upstream state's Gamma_eff throughout
-  const double G = (Cfg::SPH && ph.eos_ws) ? eos_gamma(ph, S1.prim[RHO], S1.prim[PPP]) : ph.gamma_ad;
+  const double G = (Cfg::SPH && ph.eos_ws) ? eos_gamma(ar, ph, S1.prim[RHO], S1.prim[PPP]) : ph.gamma_ad;
   const int n_evals = 10;
   const double chi = 0.5;
   double p1 = S1.prim[PPP];
   double p2 = S2.prim[PPP];
-  if (fabs(qdiv(p1 - p2, p1)) < 1.e-10 || p1 < p2) {
+  const auto by_p1 = ar.by(p1);
+  if (fabs(ar.quo0(p1 - p2, by_p1)) < 1.e-10 || p1 < p2) {
     *Sd = -1;
     return false;
   }
   double delta_p = p2 - p1;
-  double dp = delta_p / (double)n_evals;
+  double dp = ar.quo(delta_p, ar.by((double)n_evals));
   double rho1 = S1.prim[RHO];
   double rho2 = S2.prim[RHO];
-  double h1 = 1 + p1 * G / (G - 1.) / rho1;
-  double h2 = 1 + p2 * G / (G - 1.) / rho2;
+  const auto bgm1 = Cfg::SPH && ph.eos_ws ? ar.by(G - 1.) : by_gm1(ar, ph);
+  double h1 = 1 + ar.quo(ar.quo(p1 * G, bgm1), ar.by(rho1));
+  const auto by_rho2 = ar.by(rho2);
+  double h2 = 1 + ar.quo(ar.quo(p2 * G, bgm1), by_rho2);
   double lfac2 = S2.lfac;
   double vx1 = S1.v;
   double vx2 = S2.v;
-  double v12 = (vx1 - vx2) / (1 - vx1 * vx2);
+  double v12 = ar.quo(vx1 - vx2, ar.by(1 - vx1 * vx2));
   double A1 = h1 * 0.;
   double I = 0;
-  const double ginv = 1. / G;
+  const double ginv = ar.inv(G);
 #pragma unroll 2
   for (int ip = 0; ip < n_evals; ++ip) {
     double p = p1 + (ip + .5) * dp;
-    double rho = rho1 * isentrope_pow(p / p1, ginv);
-    double h = 1 + p * G / (G - 1.) / rho;
-    double cs = sqrt(G * p / (rho + p * G / (G - 1.)));
+    double rho = rho1 * isentrope_pow(ar, ar.quo(p, by_p1), ginv);
+    const double pg = ar.quo(p * G, bgm1);
+    double h = 1 + ar.quo(pg, ar.by(rho));
+    double cs = ar.root(ar.quo(G * p, ar.by(rho + pg)));
     // with A1 = 0 (1D: no transverse velocity) the root is sqrt(h*h) = h exactly
     // (h >= 1, and sqrt of a rounded square is the number itself)
-    const double num = A1 == 0. ? h : sqrt(h * h + A1 * A1 * (1. - cs * cs));
-    double dI = num / ((h * h + A1 * A1) * rho * cs) * dp;
+    const double num = A1 == 0. ? h : ar.root(h * h + A1 * A1 * (1. - cs * cs));
+    double dI = ar.quo(num, ar.by((h * h + A1 * A1) * rho * cs)) * dp;
     I += dI;
   }
   double vSR = tanh(I);
@@ -807,20 +907,20 @@ GB_HD bool compute_Sd(const Phys &ph, const FState<Cfg> &S1, const FState<Cfg> &
   double g = G;
   double gm1 = (g - 1.);
   double gm12 = gm1 * gm1;
-  double Da = 4. * g * p1 * ((g - 1) * p2 + p1) / (gm12 * (p1 - p2) * (p1 - p2));
-  double Db = h2 * (p2 - p1) / rho2 - h2 * h2;
+  double Da = ar.quo(4. * g * p1 * ((g - 1) * p2 + p1), ar.by(gm12 * (p1 - p2) * (p1 - p2)));
+  double Db = ar.quo(h2 * (p2 - p1), by_rho2) - h2 * h2;
   double Dd = 1. - Da * Db;
-  double h3 = (sqrt(Dd) - 1) * gm1 * (p1 - p2) / (2 * (gm1 * p2 + p1));
-  double J232a = -g / gm1 * (p1 - p2);
-  double J232b = h3 * (h3 - 1) / p1 - h2 * (h2 - 1) / p2;
-  double J232 = J232a / J232b;
-  double J23 = sqrt(J232);
-  double Vsa = rho22 * lfac22 * vx2 + fabs(J23) * sqrt(J232 + rho22 * lfac22 * (1. - vx22));
+  double h3 = ar.quo((ar.root(Dd) - 1) * gm1 * (p1 - p2), ar.by(2 * (gm1 * p2 + p1)));
+  double J232a = ar.quo(-g, bgm1) * (p1 - p2);
+  double J232b = ar.quo(h3 * (h3 - 1), by_p1) - ar.quo(h2 * (h2 - 1), ar.by(p2));
+  double J232 = ar.quo(J232a, ar.by(J232b));
+  double J23 = ar.root(J232);
+  double Vsa = rho22 * lfac22 * vx2 + fabs(J23) * ar.root(J232 + rho22 * lfac22 * (1. - vx22));
   double Vsb = rho22 * lfac22 + J232;
-  double Vs = Vsa / Vsb;
+  double Vs = ar.quo(Vsa, ar.by(Vsb));
   double v2Sa = (p1 - p2) * (1. - vx2 * Vs);
   double v2Sb = (Vs - vx2) * (h2 * rho2 * lfac22 * (1. - vx22) + p1 - p2);
-  double v2S = v2Sa / v2Sb;
+  double v2S = ar.quo(v2Sa, ar.by(v2Sb));
   double vlim = vSR + chi * (v2S - vSR);
   *Sd = v12 - vlim;
   *pspec = P_SPEC;  // spectral_p with VARIABLE_PSPEC_ disabled
@@ -874,16 +974,22 @@ GB_HD void inject_particles(const Phys &ph, const SynchConst &sc, double *prim, 
 }
 
 // Cell::radiativeSourceTerms: returns the increment of cons[GMX] and cons[GMN]
-template <class Cfg>
-GB_HD double radiative_source(const Phys &ph, const SynchConst &sc, const double *prim, double dV, double dt) {
+template <class Cfg, class Ar>
+GB_HD double radiative_source(Ar &ar, const Phys &ph, const SynchConst &sc, const double *prim, double dV,
+                              double dt) {
   double rho = prim[RHO];
   double p = prim[PPP];
-  double gma = state_gamma<Cfg>(ph, prim);
-  double h = 1 + p * gma / (gma - 1.) / rho;
-  double eps = rho * (h - 1.) / gma;
+  double gma = state_gamma<Cfg>(ar, ph, prim);
+  double h = 1 + ar.quo(ar.quo(p * gma, by_state_gm1<Cfg>(ar, ph, gma)), ar.by(rho));
+  double eps = ar.quo(rho * (h - 1.), ar.by(gma));
   double eB = EPS_B * eps;
-  double B = sqrt(8. * PI_ * eB);
+  double B = ar.root(8. * PI_ * eB);
   return sc.Nalpha * pow(rho, 4. / 3.) * B * B * dV * dt;
+}
+template <class Cfg>
+GB_HD double radiative_source(const Phys &ph, const SynchConst &sc, const double *prim, double dV, double dt) {
+  PlainOps ar;
+  return radiative_source<Cfg>(ar, ph, sc, prim, dV, dt);
 }
 
 // ---------------------------------------------------------------------------
@@ -893,8 +999,8 @@ struct Geom {
   double x, dx, dV, dl, cen;
 };
 
-template <class Cfg>
-GB_HD Geom make_geom(double x, double dx) {
+template <class Cfg, class Ar>
+GB_HD Geom make_geom(Ar &ar, double x, double dx) {
   Geom g;
   g.x = x;
   g.dx = dx;
@@ -904,18 +1010,23 @@ GB_HD Geom make_geom(double x, double dx) {
     g.dV = 4. * PI_ * r * r * dr;
     double r2 = r * r;
     double dr2 = dr * dr;
-    g.cen = 3. * r * (r2 + dr2) / (3 * r2 + dr2);
+    g.cen = ar.quo(3. * r * (r2 + dr2), ar.by(3 * r2 + dr2));
   } else {
     g.dV = 1. * dx;
     g.cen = x;
   }
   return g;
 }
+template <class Cfg>
+GB_HD Geom make_geom(double x, double dx) {
+  PlainOps ar;
+  return make_geom<Cfg>(ar, x, dx);
+}
 
 // Cell::move: geometry between two interfaces
-template <class Cfg>
-GB_HD Geom geom_between(double xL, double xR) {
-  return make_geom<Cfg>((xR + xL) / 2., (xR - xL));
+template <class Cfg, class Ar>
+GB_HD Geom geom_between(Ar &ar, double xL, double xR) {
+  return make_geom<Cfg>(ar, (xR + xL) / 2., (xR - xL));
 }
 
 template <class Cfg>

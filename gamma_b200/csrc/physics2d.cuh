@@ -32,61 +32,62 @@ struct Cfg2 {
 };
 
 // FluidState::lfac (fluid.cpp:10-22)
-GB_HD double lfac(const double *prim) {
+template <class Ar>
+GB_HD double lfac(Ar &ar, const double *prim) {
   double u = 0.;
   u += prim[UU1] * prim[UU1];
   u += prim[UU2] * prim[UU2];
-  u = sqrt(u);
-  return sqrt(1 + u * u);
+  u = ar.root(u);
+  return ar.root(1 + u * u);
+}
+GB_HD double lfac(const double *prim) {
+  PlainOps ar;
+  return lfac(ar, prim);
 }
 
-// FluidState::prim2cons (rel_sph.cpp:55-82) at radius r
-GB_HD void prim2cons(const Phys &ph, const double *prim, double *cons, double r) {
+// FluidState::prim2cons (rel_sph.cpp:55-82) at radius r; lf: the state's lfac
+template <class Ar>
+GB_HD void prim2cons(Ar &ar, const Phys &ph, const double *prim, double lf, double *cons, double r) {
   double rho = prim[RHO];
   double p = prim[PPP];
-  double u = 0;
-  double uu[2];
-  for (int i = 0; i < 2; ++i) {
-    uu[i] = prim[UU1 + i];
-    u += uu[i] * uu[i];
-  }
-  u = sqrt(u);
-  double lf = sqrt(1 + u * u);
-  double gma = eos_gamma(ph, rho, p);
-  double h = 1. + p * gma / (gma - 1.) / rho;
+  double gma = eos_gamma(ar, ph, rho, p);
+  double h = 1. + ar.quo(ar.quo(p * gma, by_state_gm1<Cfg2>(ar, ph, gma)), ar.by(rho));
   double D = lf * rho;
   double tau = D * h * lf - p - D;
   cons[DEN] = D;
   cons[TAU] = tau;
-  for (int i = 0; i < 2; ++i) cons[SS1 + i] = D * h * uu[i];
+  for (int i = 0; i < 2; ++i) cons[SS1 + i] = D * h * prim[UU1 + i];
   cons[SS2] *= r;
 #pragma unroll
   for (int t = TR1; t < NQ; ++t) cons[t] = prim[t] * D;
 }
+template <class Ar>
+GB_HD void prim2cons(Ar &ar, const Phys &ph, const double *prim, double *cons, double r) {
+  prim2cons(ar, ph, prim, lfac(ar, prim), cons, r);
+}
+GB_HD void prim2cons(const Phys &ph, const double *prim, double *cons, double r) {
+  PlainOps ar;
+  prim2cons(ar, ph, prim, cons, r);
+}
 
 // FluidState::state2flux (rel_sph.cpp:85-113), the flux along dimension n only
-GB_HD void state2flux(const double *prim, const double *cons, int n, double r, double *flux) {
+template <class Ar>
+GB_HD void state2flux(Ar &ar, const double *prim, const double *cons, double lfac, int n, double r, double *flux) {
   double p = prim[PPP];
-  double u = 0;
-  double uu[2];
-  for (int i = 0; i < 2; ++i) {
-    uu[i] = prim[UU1 + i];
-    u += uu[i] * uu[i];
-  }
-  u = sqrt(u);
-  double lf = sqrt(1 + u * u);
+  const double un = prim[UU1 + n];
+  const auto lf = ar.by(lfac);
   double D = cons[DEN];
   double ss[2] = {cons[SS1], cons[SS2]};
-  ss[1] = qdiv(ss[1], r);
-  flux[DEN] = qdiv(D * uu[n], lf);
+  ss[1] = ar.quo0(ss[1], ar.by(r));
+  flux[DEN] = ar.quo0(D * un, lf);
   for (int i = 0; i < 2; ++i) {
-    if (i == n) flux[SS1 + i] = qdiv(ss[i] * uu[n], lf) + p;
-    else flux[SS1 + i] = qdiv(ss[i] * uu[n], lf);
+    if (i == n) flux[SS1 + i] = ar.quo0(ss[i] * un, lf) + p;
+    else flux[SS1 + i] = ar.quo0(ss[i] * un, lf);
   }
   flux[SS2] *= r;
-  flux[TAU] = ss[n] - qdiv(D * uu[n], lf);
+  flux[TAU] = ss[n] - flux[DEN];
 #pragma unroll
-  for (int t = TR1; t < NQ; ++t) flux[t] = qdiv(cons[t] * uu[n], lf);
+  for (int t = TR1; t < NQ; ++t) flux[t] = ar.quo0(cons[t] * un, lf);
 }
 
 // One side of a Riemann problem: the state, its flux along the interface
@@ -98,10 +99,11 @@ struct St {
 
 // prim2cons + state2flux at radius r (what reconstructStates does for a
 // reconstructed state; a cell state uses its own centre radius)
-GB_HD void fill(const Phys &ph, St &S, int dim, double r) {
-  prim2cons(ph, S.prim, S.cons, r);
-  state2flux(S.prim, S.cons, dim, r, S.flux);
-  S.lfac = lfac(S.prim);
+template <class Ar>
+GB_HD void fill(Ar &ar, const Phys &ph, St &S, int dim, double r) {
+  S.lfac = lfac(ar, S.prim);
+  prim2cons(ar, ph, S.prim, S.lfac, S.cons, r);
+  state2flux(ar, S.prim, S.cons, S.lfac, dim, r, S.flux);
 }
 
 struct Waves {
@@ -110,30 +112,37 @@ struct Waves {
 
 // Interface::wavespeedEstimates + computeLambda (rel_sph.cpp:322-394) along
 // dim; d = r for the theta direction (the momentum is stored times r)
-GB_HD Waves compute_lambda(const Phys &ph, const St &L, const St &R, int dim, double xr) {
-  const double GL = ph.eos_ws ? eos_gamma(ph, L.prim[RHO], L.prim[PPP]) : ph.gamma_ad;
-  const double GR = ph.eos_ws ? eos_gamma(ph, R.prim[RHO], R.prim[PPP]) : ph.gamma_ad;
+template <class Ar>
+GB_HD Waves compute_lambda(Ar &ar, const Phys &ph, const St &L, const St &R, int dim, double xr) {
+  const double GL = ph.eos_ws ? eos_gamma(ar, ph, L.prim[RHO], L.prim[PPP]) : ph.gamma_ad;
+  const double GR = ph.eos_ws ? eos_gamma(ar, ph, R.prim[RHO], R.prim[PPP]) : ph.gamma_ad;
   const int u = UU1 + dim, s = SS1 + dim;
   Waves w;
   double lfacL = L.lfac, lfacR = R.lfac;
-  double vL = qdiv(L.prim[u], lfacL);
-  double vR = qdiv(R.prim[u], lfacR);
-  double cSL = sqrt(GL * L.prim[PPP] / (L.prim[RHO] + L.prim[PPP] * GL / (GL - 1.)));
-  double cSR = sqrt(GR * R.prim[PPP] / (R.prim[RHO] + R.prim[PPP] * GR / (GR - 1.)));
-  double sgSL = cSL * cSL / (lfacL * lfacL * (1. - cSL * cSL));
-  double sgSR = cSR * cSR / (lfacR * lfacR * (1. - cSR * cSR));
+  double vL = ar.quo0(L.prim[u], ar.by(lfacL));
+  double vR = ar.quo0(R.prim[u], ar.by(lfacR));
+  const auto gm1L = ph.eos_ws ? ar.by(GL - 1.) : by_gm1(ar, ph), gm1R = ph.eos_ws ? ar.by(GR - 1.) : by_gm1(ar, ph);
+  double cSL = ar.root(ar.quo(GL * L.prim[PPP], ar.by(L.prim[RHO] + ar.quo(L.prim[PPP] * GL, gm1L))));
+  double cSR = ar.root(ar.quo(GR * R.prim[PPP], ar.by(R.prim[RHO] + ar.quo(R.prim[PPP] * GR, gm1R))));
+  double sgSL = ar.quo(cSL * cSL, ar.by(lfacL * lfacL * (1. - cSL * cSL)));
+  double sgSR = ar.quo(cSR * cSR, ar.by(lfacR * lfacR * (1. - cSR * cSR)));
+  const double rtL = ar.root(sgSL * (1. - vL * vL + sgSL)), rtR = ar.root(sgSR * (1. - vR * vR + sgSR));
+  const auto nL = ar.by(1. + sgSL), nR = ar.by(1. + sgSR);
   double l1, l2;
-  l1 = (vR - sqrt(sgSR * (1. - vR * vR + sgSR))) / (1. + sgSR);
-  l2 = (vL - sqrt(sgSL * (1. - vL * vL + sgSL))) / (1. + sgSL);
+  l1 = ar.quo(vR - rtR, nR);
+  l2 = ar.quo(vL - rtL, nL);
   w.lL = fmin(l1, l2);
-  l1 = (vR + sqrt(sgSR * (1. - vR * vR + sgSR))) / (1. + sgSR);
-  l2 = (vL + sqrt(sgSL * (1. - vL * vL + sgSL))) / (1. + sgSL);
+  l1 = ar.quo(vR + rtR, nR);
+  l2 = ar.quo(vL + rtL, nL);
   w.lR = fmax(l1, l2);
 
-  const double d = dim == F1 ? xr : 1.;
   const double lL = w.lL, lR = w.lR;
-  double mmL = qdiv(L.cons[s], d);
-  double mmR = qdiv(R.cons[s], d);
+  double mmL = L.cons[s], mmR = R.cons[s];
+  if (dim == F1) {  // (the radial momentum is divided by 1)
+    const auto d = ar.by(xr);
+    mmL = ar.quo0(mmL, d);
+    mmR = ar.quo0(mmR, d);
+  }
   double pL = L.prim[PPP];
   double pR = R.prim[PPP];
   double EL = L.cons[TAU] + L.cons[DEN];
@@ -142,48 +151,51 @@ GB_HD Waves compute_lambda(const Phys &ph, const St &L, const St &R, int dim, do
   double AR = lR * ER - mmR;
   double BL = mmL * (lL - vL) - pL;
   double BR = mmR * (lR - vR) - pR;
-  double FhllE = qdiv(lL * AR - lR * AL, lR - lL);
-  double Ehll = (AR - AL) / (lR - lL);
-  double Fhllm = (lL * BR - lR * BL) / (lR - lL);
-  double mhll = qdiv(BR - BL, lR - lL);
+  const auto dl = ar.by(lR - lL);
+  double FhllE = ar.quo0(lL * AR - lR * AL, dl);
+  double Ehll = ar.quo(AR - AL, dl);
+  double Fhllm = ar.quo(lL * BR - lR * BL, dl);
+  double mhll = ar.quo0(BR - BL, dl);
   if (fabs(FhllE) == 0) {
-    w.lS = qdiv(mhll, Ehll + Fhllm);
+    w.lS = ar.quo0(mhll, ar.by(Ehll + Fhllm));
     return w;
   }
   // pow(x, 2.) of the C library is the correctly rounded square: x*x
   const double ef = Ehll + Fhllm;
   double delta = ef * ef - 4. * FhllE * mhll;
-  w.lS = ((Ehll + Fhllm) - sqrt(delta)) / (2. * FhllE);
+  w.lS = ar.quo((Ehll + Fhllm) - ar.root(delta), ar.by(2. * FhllE));
   return w;
 }
 
 // Interface::starState (rel_sph.cpp:397-450) along dim at radius xr
-GB_HD void star_state(const St &Sin, double lbda, double lS, int dim, double xr, double *out) {
+template <class Ar>
+GB_HD void star_state(Ar &ar, const St &Sin, double lbda, double lS, int dim, double xr, double *out) {
   const int u = UU1 + dim, s = SS1 + dim, so = SS1 + (1 - dim);
   double r = xr;
   double mm[2] = {Sin.cons[SS1], Sin.cons[SS2]};
-  mm[1] = qdiv(mm[1], r);
-  double lf = Sin.lfac;
-  double v = qdiv(Sin.prim[u], lf);
+  mm[1] = ar.quo0(mm[1], ar.by(r));
+  double v = ar.quo0(Sin.prim[u], ar.by(Sin.lfac));
   double m = mm[dim];
   double p = Sin.prim[PPP];
   double D = Sin.cons[DEN];
   double E = Sin.cons[TAU] + Sin.cons[DEN];
   double A = lbda * E - m;
   double B = m * (lbda - v) - p;
-  double pS = (A * lS - B) / (1. - lbda * lS);
-  double k = (lbda - v) / (lbda - lS);
+  double pS = ar.quo(A * lS - B, ar.by(1. - lbda * lS));
+  const auto dl = ar.by(lbda - lS);
+  double k = ar.quo(lbda - v, dl);
   out[DEN] = D * k;
-  out[s] = (m * (lbda - v) + pS - p) / (lbda - lS);
+  out[s] = ar.quo(m * (lbda - v) + pS - p, dl);
   out[so] = mm[so - SS1] * k;
   out[SS2] *= r;
-  out[TAU] = (E * (lbda - v) + pS * lS - p * v) / (lbda - lS) - D * k;
+  out[TAU] = ar.quo(E * (lbda - v) + pS * lS - p * v, dl) - D * k;
 #pragma unroll
   for (int t = TR1; t < NQ; ++t) out[t] = Sin.cons[t] * k;
 }
 
 // Interface::computeFlux (hllc.cpp:12-39): F - vU in the interface frame, times dA
-GB_HD void hllc_flux(const St &L, const St &R, const Waves &w, double v, double dA, int dim, double xr,
+template <class Ar>
+GB_HD void hllc_flux(Ar &ar, const St &L, const St &R, const Waves &w, double v, double dA, int dim, double xr,
                      double *flux) {
   if (v < w.lL) {
 #pragma unroll
@@ -191,13 +203,13 @@ GB_HD void hllc_flux(const St &L, const St &R, const Waves &w, double v, double 
   }
   if (w.lL <= v && v < w.lS) {
     double sc[NQ];
-    star_state(L, w.lL, w.lS, dim, xr, sc);
+    star_state(ar, L, w.lL, w.lS, dim, xr, sc);
 #pragma unroll
     for (int q = 0; q < NQ; ++q) flux[q] = L.flux[q] + w.lL * (sc[q] - L.cons[q]) - v * sc[q];
   }
   if (w.lS <= v && v < w.lR) {
     double sc[NQ];
-    star_state(R, w.lR, w.lS, dim, xr, sc);
+    star_state(ar, R, w.lR, w.lS, dim, xr, sc);
 #pragma unroll
     for (int q = 0; q < NQ; ++q) flux[q] = R.flux[q] + w.lR * (sc[q] - R.cons[q]) - v * sc[q];
   }
@@ -221,40 +233,46 @@ GB_HD SdSide sd_side(const St &S, int dim) {
   return SdSide{S.prim[PPP], S.prim[RHO], S.prim[UU1 + dim], S.prim[UU2 - dim], S.lfac};
 }
 
-GB_HD bool compute_Sd(const Phys &ph, const SdSide &S1, const SdSide &S2, bool reverse, double *Sd) {
+template <class Ar>
+GB_HD bool compute_Sd(Ar &ar, const Phys &ph, const SdSide &S1, const SdSide &S2, bool reverse, double *Sd) {
   // with eos_ws, the upstream state's Gamma_eff throughout
-  const double G = ph.eos_ws ? eos_gamma(ph, S1.rho, S1.p) : ph.gamma_ad;
+  const double G = ph.eos_ws ? eos_gamma(ar, ph, S1.rho, S1.p) : ph.gamma_ad;
   const int n_evals = 10;
   const double chi = 0.5;
   double p1 = S1.p;
   double p2 = S2.p;
-  if (fabs(qdiv(p1 - p2, p1)) < 1.e-10 || p1 < p2) {
+  const auto by_p1 = ar.by(p1);
+  if (fabs(ar.quo0(p1 - p2, by_p1)) < 1.e-10 || p1 < p2) {
     *Sd = -1;
     return false;
   }
   double delta_p = p2 - p1;
-  double dp = delta_p / (double)n_evals;
+  double dp = ar.quo(delta_p, ar.by((double)n_evals));
   double rho1 = S1.rho;
   double rho2 = S2.rho;
-  double h1 = 1 + p1 * G / (G - 1.) / rho1;
-  double h2 = 1 + p2 * G / (G - 1.) / rho2;
+  const auto bgm1 = ph.eos_ws ? ar.by(G - 1.) : by_gm1(ar, ph);
+  double h1 = 1 + ar.quo(ar.quo(p1 * G, bgm1), ar.by(rho1));
+  const auto by_rho2 = ar.by(rho2);
+  double h2 = 1 + ar.quo(ar.quo(p2 * G, bgm1), by_rho2);
   double lfac2 = S2.lfac;
-  double vx1 = qdiv(S1.ux, S1.lfac);
-  double vx2 = qdiv(S2.ux, lfac2);
+  double vx1 = ar.quo0(S1.ux, ar.by(S1.lfac));
+  double vx2 = ar.quo0(S2.ux, ar.by(lfac2));
   if (reverse) {
     vx1 *= -1;
     vx2 *= -1;
   }
   double ut1 = S1.ut;
-  double v12 = qdiv(vx1 - vx2, 1 - vx1 * vx2);
+  double v12 = ar.quo0(vx1 - vx2, ar.by(1 - vx1 * vx2));
   double A1 = h1 * ut1;
   double I = 0;
+  const double ginv = ar.inv(G);
   for (int ip = 0; ip < n_evals; ++ip) {
     double p = p1 + (ip + .5) * dp;
-    double rho = rho1 * isentrope_pow(p / p1, 1. / G);
-    double h = 1 + p * G / (G - 1.) / rho;
-    double cs = sqrt(G * p / (rho + p * G / (G - 1.)));
-    double dI = sqrt(h * h + A1 * A1 * (1. - cs * cs)) / ((h * h + A1 * A1) * rho * cs) * dp;
+    double rho = rho1 * isentrope_pow(ar, ar.quo(p, by_p1), ginv);
+    const double pg = ar.quo(p * G, bgm1);
+    double h = 1 + ar.quo(pg, ar.by(rho));
+    double cs = ar.root(ar.quo(G * p, ar.by(rho + pg)));
+    double dI = ar.quo(ar.root(h * h + A1 * A1 * (1. - cs * cs)), ar.by((h * h + A1 * A1) * rho * cs)) * dp;
     I += dI;
   }
   double vSR = tanh(I);
@@ -264,20 +282,20 @@ GB_HD bool compute_Sd(const Phys &ph, const SdSide &S1, const SdSide &S2, bool r
   double g = G;
   double gm1 = (g - 1.);
   double gm12 = gm1 * gm1;
-  double Da = 4. * g * p1 * ((g - 1) * p2 + p1) / (gm12 * (p1 - p2) * (p1 - p2));
-  double Db = h2 * (p2 - p1) / rho2 - h2 * h2;
+  double Da = ar.quo(4. * g * p1 * ((g - 1) * p2 + p1), ar.by(gm12 * (p1 - p2) * (p1 - p2)));
+  double Db = ar.quo(h2 * (p2 - p1), by_rho2) - h2 * h2;
   double Dd = 1. - Da * Db;
-  double h3 = (sqrt(Dd) - 1) * gm1 * (p1 - p2) / (2 * (gm1 * p2 + p1));
-  double J232a = -g / gm1 * (p1 - p2);
-  double J232b = h3 * (h3 - 1) / p1 - h2 * (h2 - 1) / p2;
-  double J232 = J232a / J232b;
-  double J23 = sqrt(J232);
-  double Vsa = rho22 * lfac22 * vx2 + fabs(J23) * sqrt(J232 + rho22 * lfac22 * (1. - vx22));
+  double h3 = ar.quo((ar.root(Dd) - 1) * gm1 * (p1 - p2), ar.by(2 * (gm1 * p2 + p1)));
+  double J232a = ar.quo(-g, bgm1) * (p1 - p2);
+  double J232b = ar.quo(h3 * (h3 - 1), by_p1) - ar.quo(h2 * (h2 - 1), ar.by(p2));
+  double J232 = ar.quo(J232a, ar.by(J232b));
+  double J23 = ar.root(J232);
+  double Vsa = rho22 * lfac22 * vx2 + fabs(J23) * ar.root(J232 + rho22 * lfac22 * (1. - vx22));
   double Vsb = rho22 * lfac22 + J232;
-  double Vs = Vsa / Vsb;
+  double Vs = ar.quo(Vsa, ar.by(Vsb));
   double v2Sa = (p1 - p2) * (1. - vx2 * Vs);
   double v2Sb = (Vs - vx2) * (h2 * rho2 * lfac22 * (1. - vx22) + p1 - p2);
-  double v2S = v2Sa / v2Sb;
+  double v2S = ar.quo(v2Sa, ar.by(v2Sb));
   double vlim = vSR + chi * (v2S - vSR);
   *Sd = v12 - vlim;
   return true;  // spectral index: p_ (VARIABLE_PSPEC_ disabled)
@@ -288,17 +306,18 @@ struct C2PInput2 {
   double D, E, ss[2], S2, S, pCand;
 };
 
-GB_HD C2PInput2 c2p_input(const double *cons, const double *prim, double r) {
+template <class Ar>
+GB_HD C2PInput2 c2p_input(Ar &ar, const double *cons, const double *prim, double r) {
   C2PInput2 in;
   in.D = cons[DEN];
   double tau = cons[TAU];
   in.E = in.D + tau;
   in.ss[0] = cons[SS1];
-  in.ss[1] = qdiv(cons[SS2], r);
+  in.ss[1] = ar.quo0(cons[SS2], ar.by(r));
   double S2 = 0.;
   for (int d = 0; d < 2; ++d) S2 += in.ss[d] * in.ss[d];
   in.S2 = S2;
-  in.S = sqrt(S2);
+  in.S = ar.root(S2);
   in.pCand = fmax(1.e-13, prim[PPP]);
   return in;
 }
@@ -306,35 +325,45 @@ GB_HD C2PInput2 c2p_input(const double *cons, const double *prim, double r) {
 // FluidState::cons2prim (rel_sph.cpp:213-320) at radius r: warm start from
 // prim[PPP]; cons is rewritten by the closing prim2cons(r).  defer, OUTLINE:
 // as in the 1D cons2prim (physics.cuh).
-template <bool OUTLINE = false>
-GB_HD void cons2prim(const Phys &ph, double *cons, double *prim, double r, C2PStats *st, bool defer = false) {
-  const C2PInput2 in = c2p_input(cons, prim, r);
+template <bool OUTLINE = false, class Ar>
+GB_HD void cons2prim(Ar &ar, const Phys &ph, double *cons, double *prim, double r, C2PStats *st,
+                     bool defer = false) {
+  const C2PInput2 in = c2p_input(ar, cons, prim, r);
   double D = in.D;
   double E = in.E;
   double ss[2] = {in.ss[0], in.ss[1]};
   double S2 = in.S2;
   double S = in.S;
-  double p = c2p_pressure<Cfg2, OUTLINE>(ph, D, S, S2, E, in.pCand, st, nullptr, defer);
-  if (defer && st && st->deferred) return;
+  const C2PRoot root = c2p_pressure<Cfg2, OUTLINE>(ar, ph, D, S, S2, E, in.pCand, defer);
+  if (st) *st = root.st;
+  if (defer && root.st.deferred) return;
+  double p = root.p;
   double Ep2 = (E + p) * (E + p);
-  double v2 = qdiv(S2, Ep2);
-  double lf = 1. / sqrt(fabs(1. - v2));
-  double rho = D / lf;
+  double v2 = ar.quo0(S2, ar.by(Ep2));
+  double lf = ar.rroot(fabs(1. - v2));
+  double rho = ar.quo(D, ar.by(lf));
   double uu[2];
   if (fabs(S) == 0.) {
     uu[0] = uu[1] = 0;
   } else {
-    double v = sqrt(1. - 1. / (lf * lf));
-    for (int d = 0; d < 2; ++d) uu[d] = lf * v * qdiv(ss[d], S);
+    double v = ar.root(1. - ar.inv(lf * lf));
+    const auto by_S = ar.by(S);
+    for (int d = 0; d < 2; ++d) uu[d] = lf * v * ar.quo0(ss[d], by_S);
   }
   p = fmax(p, P_FLOOR);
   prim[PPP] = p;
   prim[RHO] = rho;
   prim[UU1] = uu[0];
   prim[UU2] = uu[1];
+  const auto by_D = ar.by(D);
 #pragma unroll
-  for (int t = TR1; t < NQ; ++t) prim[t] = qdiv(cons[t], D);
-  prim2cons(ph, prim, cons, r);
+  for (int t = TR1; t < NQ; ++t) prim[t] = ar.quo0(cons[t], by_D);
+  prim2cons(ar, ph, prim, cons, r);
+}
+template <bool OUTLINE = false>
+GB_HD void cons2prim(const Phys &ph, double *cons, double *prim, double r, C2PStats *st, bool defer = false) {
+  PlainOps ar;
+  cons2prim<OUTLINE>(ar, ph, cons, prim, r, st, defer);
 }
 
 // ---------------------------------------------------------------------------
@@ -387,7 +416,8 @@ struct Geom {
 };
 
 // computeAllGeom (cell.cpp:31-39 -> spherical.cpp: computedl, computedV, computeCentroid)
-GB_HD Geom make_geom(double r, double dr, const TrackGeo &t) {
+template <class Ar>
+GB_HD Geom make_geom(Ar &ar, double r, double dr, const TrackGeo &t) {
   Geom g;
   g.r = r;
   g.dr = dr;
@@ -397,8 +427,12 @@ GB_HD Geom make_geom(double r, double dr, const TrackGeo &t) {
   g.dV = 4. / 3. * PI_ * rsq * dr * t.sfac;
   double rr2 = r * r;
   double dr2 = dr * dr;
-  g.cen_r = 3. * r * (rr2 + dr2) / (3 * rr2 + dr2);
+  g.cen_r = ar.quo(3. * r * (rr2 + dr2), ar.by(3 * rr2 + dr2));
   return g;
+}
+GB_HD Geom make_geom(double r, double dr, const TrackGeo &t) {
+  PlainOps ar;
+  return make_geom(ar, r, dr, t);
 }
 
 // Interface::computedA (spherical.cpp:81-112): a radial-direction interface at
@@ -415,21 +449,22 @@ GB_HD double dA_t(double r, double dr, double s_abs) {
 }
 
 // Cell::sourceTerms, 2D (rel_sph.cpp:469-496)
-GB_HD void source_terms(const Phys &ph, const double *prim, const Geom &G, const TrackGeo &t, double dt,
+template <class Ar>
+GB_HD void source_terms(Ar &ar, const Phys &ph, const double *prim, const Geom &G, const TrackGeo &t, double dt,
                         double *cons) {
   double rho = prim[RHO];
   double ut = prim[UU2];
   double p = prim[PPP];
-  double gma = eos_gamma(ph, rho, p);
-  double h = 1. + p * gma / (gma - 1.) / rho;
+  double gma = eos_gamma(ar, ph, rho, p);
+  double h = 1. + ar.quo(ar.quo(p * gma, by_state_gm1<Cfg2>(ar, ph, gma)), ar.by(rho));
   double r = G.r;
   double dr = G.dr;
   double dV = G.dV;
   double r1 = r - dr / 2.;
   double r2 = r + dr / 2.;
-  double rsq = (r2 * r2 + r1 * r1 + r2 * r1) / 3.;
-  cons[SS1] += (rho * h * ut * ut + 2. * p) * (r / rsq) * dV * dt;
-  cons[SS2] += p * t.cos_th / t.s_mid * dV * dt;
+  double rsq = ar.quo(r2 * r2 + r1 * r1 + r2 * r1, ar.by(3.));
+  cons[SS1] += (rho * h * ut * ut + 2. * p) * ar.quo(r, ar.by(rsq)) * dV * dt;
+  cons[SS2] += ar.quo0(p * t.cos_th, ar.by(t.s_mid)) * dV * dt;
 }
 
 // ---------------------------------------------------------------------------

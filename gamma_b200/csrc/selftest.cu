@@ -21,9 +21,45 @@ __global__ void qdiv_kernel(const double *a, const double *b, double *mine, doub
   }
 }
 
+// one FlatOps result each, and whether its operands were in range
+__global__ void flat_ops_kernel(const double *a, const double *b, double *quo, double *inv, double *root,
+                                double *rroot, int *bad, int n) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    gb::FlatOps q, v, r, s;
+    quo[i] = q.quo(a[i], q.by(b[i]));
+    inv[i] = v.inv(b[i]);
+    root[i] = r.root(a[i]);
+    rroot[i] = s.rroot(a[i]);
+    bad[i] = (q.bad() ? 1 : 0) | (v.bad() ? 2 : 0) | (r.bad() ? 4 : 0) | (s.bad() ? 8 : 0);
+  }
+}
+
 }  // namespace
 
 extern "C" {
+
+// gb::FlatOps on n host pairs, on the current device: out [4][n] takes a/b,
+// 1/b, sqrt(a) and 1/sqrt(a), bad [n] the out-of-range bits (1, 2, 4, 8).
+// Returns 0 or the CUDA error code.
+__attribute__((visibility("default"))) int gb_selftest_flat_ops(const double *a, const double *b, double *out,
+                                                                int *bad, int n) {
+  if (n <= 0) return 0;
+  double *d = nullptr;
+  const size_t s = (size_t)n * sizeof(double), m = (size_t)n;
+  cudaError_t e = cudaMalloc(&d, 7 * s);
+  if (e != cudaSuccess) return (int)e;
+  int *db = reinterpret_cast<int *>(d + 6 * m);
+  e = cudaMemcpy(d, a, s, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(d + m, b, s, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    flat_ops_kernel<<<(n + 255) / 256, 256>>>(d, d + m, d + 2 * m, d + 3 * m, d + 4 * m, d + 5 * m, db, n);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(out, d + 2 * m, 4 * s, cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess) e = cudaMemcpy(bad, db, m * sizeof(int), cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  return (int)e;
+}
 
 // gb::qdiv(a, b) and the plain IEEE quotient a / b of n host pairs, on the
 // current device.  Returns 0 or the CUDA error code.

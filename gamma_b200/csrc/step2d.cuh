@@ -107,15 +107,23 @@ GB_HD int iL_of(const Grid2 &G) { return G.ngst - 1; }
 GB_HD int jL_of(const Grid2 &G) { return G.ngst - 1; }
 GB_HD int jR_of(const Grid2 &G) { return G.NJ - G.ngst; }
 
-GB_HD double cen_r(double r, double dr) {
+template <class Ar>
+GB_HD double cen_r(Ar &ar, double r, double dr) {
   double r2 = r * r;
   double dr2 = dr * dr;
-  return 3. * r * (r2 + dr2) / (3 * r2 + dr2);
+  return ar.quo(3. * r * (r2 + dr2), ar.by(3 * r2 + dr2));
+}
+GB_HD double cen_r(double r, double dr) {
+  PlainOps ar;
+  return cen_r(ar, r, dr);
 }
 
 GB_HD TrackGeo tgeo(const Grid2 &G, int j) { return track_geo(G.tg + (long long)j * TG_WORDS); }
 
-GB_HD Geom cell_geom(const Grid2 &G, int j, long long g) { return make_geom(G.x[g], G.dx[g], tgeo(G, j)); }
+template <class Ar>
+GB_HD Geom cell_geom(Ar &ar, const Grid2 &G, int j, long long g) {
+  return make_geom(ar, G.x[g], G.dx[g], tgeo(G, j));
+}
 
 GB_HD void load_prim(const Grid2 &G, long long g, double *p) {
 #pragma unroll
@@ -217,30 +225,35 @@ GB_HD double outer_velocity(const Grid2 &G, const Params2 &P, long long it) {
 }
 
 // cell state as prepForUpdate leaves it: prim2cons and state2flux at the cell's r
-GB_HD void cell_state(const Phys &ph, const Grid2 &G, long long g, int dim, St &S) {
+template <class Ar>
+GB_HD void cell_state(Ar &ar, const Phys &ph, const Grid2 &G, long long g, int dim, St &S) {
   load_prim(G, g, S.prim);
-  fill(ph, S, dim, G.x[g]);
+  fill(ar, ph, S, dim, G.x[g]);
 }
 
-GB_HD void mv_interface(const Phys &ph, const Params2 &P, const Grid2 &G, int j, int i, long long it) {
+// The interface with the operators Ar.  False (the interface's own outputs not
+// written) where an operand left their range.
+template <class Ar>
+GB_HD bool mv_interface_ops(const Phys &ph, const Params2 &P, const Grid2 &G, int j, int i, long long it) {
+  Ar ar;
   const int n = G.ntrack[j];
-  if (i > n - 2) return;
   const long long o = (long long)j * G.cap, g = o + i;
   const double xI = G.xI[g];
   St L, R;
   if (i == 0 || i == n - 2) {
-    cell_state(ph, G, g, MV, L);
-    cell_state(ph, G, g + 1, MV, R);
+    cell_state(ar, ph, G, g, MV, L);
+    cell_state(ar, ph, G, g + 1, MV, R);
   } else {
-    const double cLL = cen_r(G.x[g - 1], G.dx[g - 1]), cL = cen_r(G.x[g], G.dx[g]);
-    const double cR = cen_r(G.x[g + 1], G.dx[g + 1]), cRR = cen_r(G.x[g + 2], G.dx[g + 2]);
+    const double cLL = cen_r(ar, G.x[g - 1], G.dx[g - 1]), cL = cen_r(ar, G.x[g], G.dx[g]);
+    const double cR = cen_r(ar, G.x[g + 1], G.dx[g + 1]), cRR = cen_r(ar, G.x[g + 2], G.dx[g + 2]);
+    const auto dL = ar.by(cL - cLL), dN = ar.by(cR - cL), dR = ar.by(cRR - cR);
 #pragma unroll
     for (int q = 0; q < NQ; ++q) {
       const double qLL = G.prim[q * G.NC + g - 1], qL = G.prim[q * G.NC + g];
       const double qR = G.prim[q * G.NC + g + 1], qRR = G.prim[q * G.NC + g + 2];
-      double gL = qdiv(qL - qLL, cL - cLL);
-      const double gN = qdiv(qR - qL, cR - cL);
-      double gR = qdiv(qRR - qR, cRR - cR);
+      double gL = ar.quo0(qL - qLL, dL);
+      const double gN = ar.quo0(qR - qL, dN);
+      double gR = ar.quo0(qRR - qR, dR);
       gL = minmod(gL, gN);
       gR = minmod(gR, gN);
       // grad_mv stored in the cells; cell i from its right interface, except
@@ -250,25 +263,35 @@ GB_HD void mv_interface(const Phys &ph, const Params2 &P, const Grid2 &G, int j,
       L.prim[q] = qL + gL * (xI - cL);
       R.prim[q] = qR + gR * (xI - cR);
     }
-    fill(ph, L, MV, xI);
-    fill(ph, R, MV, xI);
+    fill(ar, ph, L, MV, xI);
+    fill(ar, ph, R, MV, xI);
   }
-  const Waves w = compute_lambda(ph, L, R, MV, xI);
+  const Waves w = compute_lambda(ar, ph, L, R, MV, xI);
   double v = ph.vi * w.lS;
   if (i >= n - 1 - G.ngst) v = outer_velocity(G, P, it);
+  double fl[NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) fl[q] = 0.;
+  hllc_flux(ar, L, R, w, v, dA_r(xI, tgeo(G, j)), MV, xI, fl);
+  double Sd;
+  const bool have = compute_Sd(ar, ph, sd_side(L, MV), sd_side(R, MV), false, &Sd);
+  if (ar.bad()) return false;
   G.lL[g] = w.lL;
   G.lR[g] = w.lR;
   G.v[g] = v;
-  double fl[NQ];
-  hllc_flux(L, R, w, v, dA_r(xI, tgeo(G, j)), MV, xI, fl);
 #pragma unroll
   for (int q = 0; q < NQ; ++q) G.flx[q * G.NC + g] = fl[q];
   // measureShock, moving direction: forward shocks only, into the left cell
-  double Sd;
-  if (compute_Sd(ph, sd_side(L, MV), sd_side(R, MV), false, &Sd)) {
-    if (P_SPEC > G.pspec[g]) G.pspec[g] = P_SPEC;
-  }
+  if (have && P_SPEC > G.pspec[g]) G.pspec[g] = P_SPEC;
   G.sd[g] = fmax(G.sd[g], Sd);
+  return true;
+}
+GB_HD_OUTLINE void mv_interface_plain(const Phys &ph, const Params2 &P, const Grid2 &G, int j, int i, long long it) {
+  mv_interface_ops<PlainOps>(ph, P, G, j, i, it);
+}
+GB_HD void mv_interface(const Phys &ph, const Params2 &P, const Grid2 &G, int j, int i, long long it) {
+  if (i > G.ntrack[j] - 2) return;
+  if (!mv_interface_ops<FlatOps>(ph, P, G, j, i, it)) mv_interface_plain(ph, P, G, j, i, it);
 }
 
 // ---------------------------------------------------------------------------
@@ -317,8 +340,16 @@ GB_HD void cell_mv(const Grid2 &G, int j, int i) {
   const long long g = (long long)j * G.cap + i;
   // Cell::update_dt, moving direction
   const double a = G.dx[g];
-  double dL = (G.lR[g - 1] > G.v[g]) ? a / (G.lR[g - 1] - G.v[g]) : DT_INF;
-  double dR = (G.lL[g] < G.v[g - 1]) ? a / (G.v[g - 1] - G.lL[g]) : DT_INF;
+  const double rL = G.lR[g - 1] - G.v[g], rR = G.v[g - 1] - G.lL[g];
+  const bool onL = G.lR[g - 1] > G.v[g], onR = G.lL[g] < G.v[g - 1];
+  FlatOps ar;
+  double dL = ar.quo(a, ar.by(onL ? rL : 1.)), dR = ar.quo(a, ar.by(onR ? rR : 1.));
+  if (ar.bad()) {
+    dL = a / rL;
+    dR = a / rR;
+  }
+  if (!onL) dL = DT_INF;
+  if (!onR) dR = DT_INF;
   const double cand = fmin(dL, dR);
   if (cand < 0) *G.status = 30;
   else G.dtl[g] = fmin(G.dtl[g], cand);
@@ -345,28 +376,31 @@ GB_HD void overlap(const Grid2 &G, long long g0, long long gn, double *xm, doubl
 }
 
 // Geometry of the gradient towards neighbour gn, the same for every slot:
-// the offsets of the overlap's centre from both cell centres, the theta
-// distance, and the overlap's area.
+// the offsets of the overlap's centre from both cell centres and the
+// overlap's area.  (The theta distance is the list's: its cells are
+// consecutive cells of one track.)
 struct NbrGeo {
-  double dxmL, dxmR, dcen, dA;
+  double dxmL, dxmR, dA;
 };
 
-GB_HD NbrGeo neighbour_geo(const Grid2 &G, long long g0, long long gn, double cr0, double ct0, double s) {
+template <class Ar>
+GB_HD NbrGeo neighbour_geo(Ar &ar, const Grid2 &G, long long g0, long long gn, double cr0, double s) {
   double xm, w;
   overlap(G, g0, gn, &xm, &w);
   NbrGeo n;
   n.dxmL = xm - cr0;
-  n.dxmR = xm - cen_r(G.x[gn], G.dx[gn]);
-  n.dcen = tgeo(G, track_of(G, gn)).cen_t - ct0;
+  n.dxmR = xm - cen_r(ar, G.x[gn], G.dx[gn]);
   n.dA = dA_t(xm, w, s);
   return n;
 }
 
 // The gradient of slot q towards neighbour gn, (qR - qL) / dcen.
-GB_HD double neighbour_grad(const Grid2 &G, int q, long long gn, const NbrGeo &n, double p0, double m0) {
+template <class Ar>
+GB_HD double neighbour_grad(Ar &ar, const Grid2 &G, int q, long long gn, const NbrGeo &n, typename Ar::By dcen,
+                            double p0, double m0) {
   const double qL = p0 + m0 * n.dxmL;
   const double qR = G.prim[q * G.NC + gn] + G.gmv[q * G.NC + gn] * n.dxmR;
-  return qdiv(qR - qL, n.dcen);
+  return ar.quo0(qR - qL, dcen);
 }
 
 // Pass 1 forms the dA-weighted average; pass 2 folds in minmod with each
@@ -378,16 +412,13 @@ GB_HD double neighbour_grad(const Grid2 &G, int q, long long gn, const NbrGeo &n
 // operations and their order are those of the reference's loops.
 constexpr int KGEO = 4;
 
-GB_HD void trans_grad(const Grid2 &G, int j, int i) {
-  const int n = G.ntrack[j];
-  if (i >= n) return;
+// False where an operand left the range of Ar (grad_f1 of the cell is then to
+// be formed again).
+template <class Ar>
+GB_HD bool trans_grad_ops(const Grid2 &G, int j, int i) {
+  Ar ar;
   const long long g0 = (long long)j * G.cap + i;
-  if (j == G.NJ - 1) {  // never recomputed: keeps its copied value
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) G.gf1n[q * G.NC + g0] = G.gf1[q * G.NC + g0];
-    return;
-  }
-  const double cr0 = cen_r(G.x[g0], G.dx[g0]);
+  const double cr0 = cen_r(ar, G.x[g0], G.dx[g0]);
   const TrackGeo t0 = tgeo(G, j);
   const double ct0 = t0.cen_t;
   const int f0 = G.nbr[0 * G.NC + g0], c0 = G.nbr[1 * G.NC + g0];
@@ -397,15 +428,25 @@ GB_HD void trans_grad(const Grid2 &G, int j, int i) {
   // the interface is th - dth/2 below and th (unmoved) above
 #define TG_NBR(kn) ((kn) < c0 ? (long long)f0 + (kn) : (long long)f1 + ((kn) - c0))
 #define TG_S(kn) ((kn) < c0 ? t0.s_lo : t0.s_mid)
+#define TG_D(kn) ((kn) < c0 ? d0 : d1)
+  // theta distances to the two lists' tracks (1 where a list is empty)
+  const auto d0 = ar.by(c0 > 0 ? tgeo(G, track_of(G, f0)).cen_t - ct0 : 1.);
+  const auto d1 = ar.by(c1 > 0 ? tgeo(G, track_of(G, f1)).cen_t - ct0 : 1.);
   NbrGeo geo[KGEO];
   double dAtot = 0.;
 #pragma unroll
   for (int kn = 0; kn < KGEO; ++kn)
     if (kn < nn) {
-      geo[kn] = neighbour_geo(G, g0, TG_NBR(kn), cr0, ct0, TG_S(kn));
+      geo[kn] = neighbour_geo(ar, G, g0, TG_NBR(kn), cr0, TG_S(kn));
       dAtot += geo[kn].dA;
     }
-  for (int kn = KGEO; kn < nn; ++kn) dAtot += neighbour_geo(G, g0, TG_NBR(kn), cr0, ct0, TG_S(kn)).dA;
+  for (int kn = KGEO; kn < nn; ++kn) dAtot += neighbour_geo(ar, G, g0, TG_NBR(kn), cr0, TG_S(kn)).dA;
+  if (nn == 0) {  // no neighbours: the reference's 0 / 0
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) G.gf1n[q * G.NC + g0] = nan("");
+    return true;
+  }
+  const auto by_tot = ar.by(dAtot);
 #pragma unroll 1
   for (int q = 0; q < NQ; ++q) {
     const double p0 = G.prim[q * G.NC + g0], m0 = G.gmv[q * G.NC + g0];
@@ -413,25 +454,38 @@ GB_HD void trans_grad(const Grid2 &G, int j, int i) {
 #pragma unroll
     for (int kn = 0; kn < KGEO; ++kn)
       if (kn < nn) {
-        kept[kn] = neighbour_grad(G, q, TG_NBR(kn), geo[kn], p0, m0);
+        kept[kn] = neighbour_grad(ar, G, q, TG_NBR(kn), geo[kn], TG_D(kn), p0, m0);
         avg += kept[kn] * geo[kn].dA;
       }
     for (int kn = KGEO; kn < nn; ++kn) {
-      const NbrGeo e = neighbour_geo(G, g0, TG_NBR(kn), cr0, ct0, TG_S(kn));
-      avg += neighbour_grad(G, q, TG_NBR(kn), e, p0, m0) * e.dA;
+      const NbrGeo e = neighbour_geo(ar, G, g0, TG_NBR(kn), cr0, TG_S(kn));
+      avg += neighbour_grad(ar, G, q, TG_NBR(kn), e, TG_D(kn), p0, m0) * e.dA;
     }
-    avg = qdiv(avg, dAtot);
+    avg = ar.quo0(avg, by_tot);
 #pragma unroll
     for (int kn = 0; kn < KGEO; ++kn)
       if (kn < nn) avg = minmod(avg, kept[kn]);
     for (int kn = KGEO; kn < nn; ++kn) {
-      const NbrGeo e = neighbour_geo(G, g0, TG_NBR(kn), cr0, ct0, TG_S(kn));
-      avg = minmod(avg, neighbour_grad(G, q, TG_NBR(kn), e, p0, m0));
+      const NbrGeo e = neighbour_geo(ar, G, g0, TG_NBR(kn), cr0, TG_S(kn));
+      avg = minmod(avg, neighbour_grad(ar, G, q, TG_NBR(kn), e, TG_D(kn), p0, m0));
     }
     G.gf1n[q * G.NC + g0] = avg;
   }
 #undef TG_NBR
 #undef TG_S
+#undef TG_D
+  return !ar.bad();
+}
+GB_HD_OUTLINE void trans_grad_plain(const Grid2 &G, int j, int i) { trans_grad_ops<PlainOps>(G, j, i); }
+GB_HD void trans_grad(const Grid2 &G, int j, int i) {
+  if (i >= G.ntrack[j]) return;
+  if (j == G.NJ - 1) {  // never recomputed: keeps its copied value
+    const long long g0 = (long long)j * G.cap + i;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) G.gf1n[q * G.NC + g0] = G.gf1[q * G.NC + g0];
+    return;
+  }
+  if (!trans_grad_ops<FlatOps>(G, j, i)) trans_grad_plain(G, j, i);
 }
 
 // ---------------------------------------------------------------------------
@@ -444,7 +498,9 @@ struct F1Result {
   bool have_fwd, have_rev;
 };
 
-GB_HD void f1_interface(const Phys &ph, const Grid2 &G, int j, long long g0, long long gn, F1Result &out) {
+template <class Ar>
+GB_HD bool f1_interface(const Phys &ph, const Grid2 &G, int j, long long g0, long long gn, F1Result &out) {
+  Ar ar;
   const int jn = track_of(G, gn);
   const TrackGeo t0 = tgeo(G, j);
   const double jpos = t0.th + t0.dth / 2.;
@@ -454,14 +510,14 @@ GB_HD void f1_interface(const Phys &ph, const Grid2 &G, int j, long long g0, lon
   St L, R;
   const bool pc = j == 0 || j == G.NJ - 2 || G.nbr[1 * G.NC + g0] == 0 || G.nbr[3 * G.NC + gn] == 0;
   if (pc) {
-    cell_state(ph, G, g0, F1, L);
-    cell_state(ph, G, gn, F1, R);
+    cell_state(ar, ph, G, g0, F1, L);
+    cell_state(ar, ph, G, gn, F1, R);
   } else {
     // the upper cell's transverse gradient: this stage's if the reference's
     // track-by-track loop has reached it already, else the previous stage's
     const double *gR = (jn < j || (jn == j && gn < g0)) ? G.gf1n : G.gf1;
-    const double dxmL = xm - cen_r(G.x[g0], G.dx[g0]);
-    const double dxmR = xm - cen_r(G.x[gn], G.dx[gn]);
+    const double dxmL = xm - cen_r(ar, G.x[g0], G.dx[g0]);
+    const double dxmR = xm - cen_r(ar, G.x[gn], G.dx[gn]);
     const double dxfL = jpos - t0.cen_t;
     const double dxfR = jpos - tgeo(G, jn).cen_t;
 #pragma unroll
@@ -471,11 +527,13 @@ GB_HD void f1_interface(const Phys &ph, const Grid2 &G, int j, long long g0, lon
       L.prim[q] = qL + G.gf1n[q * G.NC + g0] * dxfL;  // this stage's (computed first)
       R.prim[q] = qR + gR[q * G.NC + gn] * dxfR;
     }
-    fill(ph, L, F1, xm);
-    fill(ph, R, F1, xm);
+    fill(ar, ph, L, F1, xm);
+    fill(ar, ph, R, F1, xm);
   }
-  const Waves wv = compute_lambda(ph, L, R, F1, xm);
-  hllc_flux(L, R, wv, 0., dA, F1, xm, out.flux);
+  const Waves wv = compute_lambda(ar, ph, L, R, F1, xm);
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) out.flux[q] = 0.;
+  hllc_flux(ar, L, R, wv, 0., dA, F1, xm, out.flux);
   // measureShock across the tracks (radiation_sph.cpp:160-175): the forward
   // test (L upstream) and the reverse one (R upstream).  compute_Sd passes its
   // pressure test only where the upstream pressure is the larger, so at most
@@ -487,11 +545,18 @@ GB_HD void f1_interface(const Phys &ph, const Grid2 &G, int j, long long g0, lon
   const bool fw = sL.p > sR.p;
   const bool nan_p = isnan(sL.p) || isnan(sR.p);
   double sd;
-  const bool have = compute_Sd(ph, fw ? sL : sR, fw ? sR : sL, !fw, &sd);
+  const bool have = compute_Sd(ar, ph, fw ? sL : sR, fw ? sR : sL, !fw, &sd);
   out.have_fwd = (fw || nan_p) && have;
   out.sd_fwd = (fw || nan_p) ? sd : -1.;
   out.have_rev = !fw && have;
   out.sd_rev = fw ? -1. : sd;
+  return !ar.bad();
+}
+
+GB_HD_OUTLINE F1Result f1_interface_plain(const Phys &ph, const Grid2 &G, int j, long long g0, long long gn) {
+  F1Result r;
+  f1_interface<PlainOps>(ph, G, j, g0, gn, r);
+  return r;
 }
 
 // Interface s of track j's list: upper neighbour k of its owning cell.  Its
@@ -503,7 +568,8 @@ GB_HD void f1_if(const Phys &ph, const Grid2 &G, int j, int s) {
   const long long g0 = (long long)j * G.cap + G.if_own[sl];
   const int k = s - G.if_off[g0];
   F1Result r;
-  f1_interface(ph, G, j, g0, G.nbr[2 * G.NC + g0] + k, r);
+  if (!f1_interface<FlatOps>(ph, G, j, g0, G.nbr[2 * G.NC + g0] + k, r))
+    r = f1_interface_plain(ph, G, j, g0, G.nbr[2 * G.NC + g0] + k);
   const long long IS = (long long)G.NJ * if_cap(G);
 #pragma unroll
   for (int q = 0; q < NQ; ++q) G.ifs[q * IS + sl] = r.flux[q];
@@ -726,6 +792,106 @@ GB_HD void cell_cons2prim(const Phys &ph, double *cons, double *prim, double r, 
   }
 }
 
+// The update of one active cell in pieces.  What stays between them:
+struct CellStep {
+  double prim[NQ], cons[NQ];
+  double dt, r1, r2, xn, dxn, dV1;
+  TrackGeo tj;
+};
+
+// Cell::update up to cons2prim (at radius r1)
+template <class Ar>
+GB_HD void cell_advance(Ar &ar, const Phys &ph, const Params2 &P, const Grid2 &G, int j, long long g, int stage,
+                        CellStep &c) {
+  c.dt = *G.dt;
+  const Geom G0 = cell_geom(ar, G, j, g);
+  prim2cons(ar, ph, c.prim, c.cons, G0.r);
+  if (stage == 1) {
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) G.cons0[q * G.NC + g] = c.cons[q];
+    G.dV0[g] = G0.dV;
+  }
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) c.cons[q] *= G0.dV;
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) c.cons[q] += (G.flx[q * G.NC + g - 1] - G.flx[q * G.NC + g]) * c.dt;
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) c.cons[q] += (G.f1lo[q * G.NC + g] - G.f1hi[q * G.NC + g]) * c.dt;
+  c.tj = tgeo(G, j);
+  source_terms(ar, ph, c.prim, G0, c.tj, c.dt, c.cons);
+  {  // Cell::radiativeSourceTerms
+    const SynchConst sc{P.Nalpha, P.Nmp, P.Nme};
+    const double dg = radiative_source<Cfg2>(ar, ph, sc, c.prim, G0.dV, c.dt);
+    c.cons[GMX] += dg;
+    c.cons[GMN] += dg;
+  }
+  const double xL = G.xIm[g - 1], xR = G.xIm[g];
+  const Geom G1 = make_geom(ar, (xR + xL) / 2., (xR - xL), c.tj);
+  const auto by = ar.by(G1.dV);
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) c.cons[q] = q <= TAU ? ar.quo(c.cons[q], by) : ar.quo0(c.cons[q], by);
+  c.r1 = G1.cen_r;
+  c.dV1 = G1.dV;
+  c.xn = G1.r;
+  c.dxn = G1.dr;
+}
+
+// the stage's combine, up to its cons2prim (at radius r2)
+template <class Ar>
+GB_HD void cell_combine(Ar &ar, const Grid2 &G, long long g, int stage, CellStep &c) {
+  const double w0 = stage == 2 ? 3. / 4. : 1. / 3.;
+  const double w1 = stage == 2 ? 1. / 4. : 2. / 3.;
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) c.cons[q] = w0 * G.cons0[q * G.NC + g] * G.dV0[g] + w1 * c.cons[q] * c.dV1;
+  const double cL = G.xI[g - 1], cR = G.xI[g];  // combined positions
+  const Geom G2 = make_geom(ar, (cR + cL) / 2., (cR - cL), c.tj);
+  const auto by = ar.by(G2.dV);
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) c.cons[q] = q <= TAU ? ar.quo(c.cons[q], by) : ar.quo0(c.cons[q], by);
+  c.r2 = G2.r;
+  c.xn = G2.r;
+  c.dxn = G2.dr;
+}
+
+// the whole update, with the reference's warm starts
+struct CellUpdate {
+  double prim[NQ], xn, dxn;
+  C2PStats c1, c2;
+  bool ok;
+};
+template <class Ar>
+GB_HD CellUpdate cell_update_ops(const Phys &ph, const Params2 &P, const Grid2 &G, int j, long long g, int stage) {
+  Ar ar;
+  CellStep c;
+  CellUpdate u;
+  load_prim(G, g, c.prim);
+  cell_advance(ar, ph, P, G, j, g, stage, c);
+  cons2prim(ar, ph, c.cons, c.prim, c.r1, &u.c1);
+  u.c2 = C2PStats{0, 0, 0, 0};
+  if (stage > 1) {
+    cell_combine(ar, G, g, stage, c);
+    cons2prim(ar, ph, c.cons, c.prim, c.r2, &u.c2);
+  }
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) u.prim[q] = c.prim[q];
+  u.xn = c.xn;
+  u.dxn = c.dxn;
+  u.ok = !ar.bad();
+  return u;
+}
+GB_HD_OUTLINE CellUpdate cell_update_plain(const Phys &ph, const Params2 &P, const Grid2 &G, int j, long long g,
+                                           int stage) {
+  return cell_update_ops<PlainOps>(ph, P, G, j, g, stage);
+}
+
+GB_HD void count_c2p(unsigned long long *c2p, const C2PStats &cs) {
+  c2p[0] += 1;
+  c2p[1] += cs.iters;
+  c2p[2] += cs.fallback;
+  if ((unsigned long long)cs.iters > c2p[3]) c2p[3] = cs.iters;
+  c2p[5] += cs.poor;
+}
+
 // `live` = false: a lane without a cell (the learned guess' warp-uniform loop).
 template <class Guess>
 GB_HD void update_cell(const Phys &ph, const Params2 &P, const Grid2 &G, int j, int i, int stage,
@@ -737,62 +903,39 @@ GB_HD void update_cell(const Phys &ph, const Params2 &P, const Grid2 &G, int j, 
   const int iL = iL_of(G), iR = n - G.ngst;
   const bool active_track = j > jL && j < jR;
   const bool upd = live && active_track && i >= iL + 1 && i <= iR - 1;
-  double prim[NQ], cons[NQ];
-#pragma unroll
-  for (int q = 0; q < NQ; ++q) prim[q] = cons[q] = 0.;
-  if (live) load_prim(G, g, prim);
-  double dt = 0., r1 = 1., r2 = 1., xn = 0., dxn = 0., dV1 = 0.;
-  TrackGeo tj{};
-  if (upd) {
-    dt = *G.dt;
-    const Geom G0 = cell_geom(G, j, g);
-    prim2cons(ph, prim, cons, G0.r);
-    if (stage == 1) {
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) G.cons0[q * G.NC + g] = cons[q];
-      G.dV0[g] = G0.dV;
+  double prim[NQ], xn = 0., dxn = 0.;
+  if (Guess::ON) {
+    // blocks under `upd`, so that the whole warp meets at each inference
+    PlainOps ar;
+    CellStep c{};
+    c.r1 = c.r2 = 1.;
+    if (live) load_prim(G, g, c.prim);
+    if (upd) cell_advance(ar, ph, P, G, j, g, stage, c);
+    cell_cons2prim(ph, c.cons, c.prim, c.r1, upd, c2p, guess);
+    if (stage > 1) {
+      if (upd) cell_combine(ar, G, g, stage, c);
+      cell_cons2prim(ph, c.cons, c.prim, c.r2, upd, c2p, guess);
     }
+    if (!live) return;
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) cons[q] *= G0.dV;
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) cons[q] += (G.flx[q * G.NC + g - 1] - G.flx[q * G.NC + g]) * dt;
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) cons[q] += (G.f1lo[q * G.NC + g] - G.f1hi[q * G.NC + g]) * dt;
-    tj = tgeo(G, j);
-    source_terms(ph, prim, G0, tj, dt, cons);
-    {  // Cell::radiativeSourceTerms
-      const SynchConst sc{P.Nalpha, P.Nmp, P.Nme};
-      const double dg = radiative_source<Cfg2>(ph, sc, prim, G0.dV, dt);
-      cons[GMX] += dg;
-      cons[GMN] += dg;
-    }
-    const double xL = G.xIm[g - 1], xR = G.xIm[g];
-    const Geom G1 = make_geom((xR + xL) / 2., (xR - xL), tj);
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) cons[q] = q <= TAU ? cons[q] / G1.dV : qdiv(cons[q], G1.dV);
-    r1 = G1.cen_r;
-    dV1 = G1.dV;
-    xn = G1.r;
-    dxn = G1.dr;
-  }
-  cell_cons2prim(ph, cons, prim, r1, upd, c2p, guess);
-  if (stage > 1) {
+    for (int q = 0; q < NQ; ++q) prim[q] = c.prim[q];
+    xn = c.xn;
+    dxn = c.dxn;
+  } else {
+    if (!live) return;
     if (upd) {
-      const double w0 = stage == 2 ? 3. / 4. : 1. / 3.;
-      const double w1 = stage == 2 ? 1. / 4. : 2. / 3.;
+      CellUpdate u = cell_update_ops<FlatOps>(ph, P, G, j, g, stage);
+      if (!u.ok) u = cell_update_plain(ph, P, G, j, g, stage);
+      count_c2p(c2p, u.c1);
+      if (stage > 1) count_c2p(c2p, u.c2);
 #pragma unroll
-      for (int q = 0; q < NQ; ++q) cons[q] = w0 * G.cons0[q * G.NC + g] * G.dV0[g] + w1 * cons[q] * dV1;
-      const double cL = G.xI[g - 1], cR = G.xI[g];  // combined positions
-      const Geom G2 = make_geom((cR + cL) / 2., (cR - cL), tj);
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) cons[q] = q <= TAU ? cons[q] / G2.dV : qdiv(cons[q], G2.dV);
-      r2 = G2.r;
-      xn = G2.r;
-      dxn = G2.dr;
+      for (int q = 0; q < NQ; ++q) prim[q] = u.prim[q];
+      xn = u.xn;
+      dxn = u.dxn;
+    } else {
+      load_prim(G, g, prim);
     }
-    cell_cons2prim(ph, cons, prim, r2, upd, c2p, guess);
   }
-  if (!live) return;
   if (upd) {
     G.x[g] = xn;
     G.dx[g] = dxn;

@@ -22,6 +22,8 @@
 #include "physics.cuh"
 #include "regrid.cuh"
 
+#include <type_traits>
+
 #ifdef GB_SWEEP_NOINLINE
 #define GB_SWEEP_ATTR __noinline__
 #else
@@ -182,8 +184,9 @@ struct TrackStep {
 
   // Reconstructed left/right states at interface i from staged cells
   // (Grid::reconstructStates, 1d.cpp:370-461).  c = slot of cell i.
-  __device__ static void reconstruct(const Smem &sm, const Phys &ph, int i, int n, int c, double xI,
-                                     FState<Cfg> &L, FState<Cfg> &R) {
+  template <class Ar>
+  __device__ __forceinline__ static void reconstruct(Ar &ar, const Smem &sm, const Phys &ph, int i, int n, int c,
+                                                     double xI, FState<Cfg> &L, FState<Cfg> &R) {
     if (i == 0 || i == n - 2) {
 #pragma unroll
       for (int s = 0; s < NQS; ++s) {
@@ -209,8 +212,173 @@ struct TrackStep {
     }
     L.prim[UU2] = 0.;
     R.prim[UU2] = 0.;
-    fill_state<Cfg>(ph, L);
-    fill_state<Cfg>(ph, R);
+    fill_state<Cfg>(ar, ph, L);
+    fill_state<Cfg>(ar, ph, R);
+  }
+
+  // What the solution of one interface gives: fluxes in the interface's frame
+  // times its area, the outer wave speeds, its velocity, and the shock
+  // detector's result into the cell on its left (pspec < 0: none).
+  struct IfaceSol {
+    double flux[NQ], lL, lR, v, Sd, pspec;
+  };
+
+  template <class Ar>
+  __device__ __forceinline__ static void solve_interface(Ar &ar, const Smem &sm, const Phys &ph,
+                                                         const gamma_problem::HookArgs &A, int i, int n, int c,
+                                                         double xI, IfaceSol &s) {
+    FState<Cfg> L, R;
+    reconstruct(ar, sm, ph, i, n, c, xI, L, R);
+    const Waves w = compute_lambda<Cfg>(ar, ph, L, R);
+    s.v = ph.vi * w.lS;
+    Hooks::user_kinematics(A, i, &s.v);  // Grid::userKinematics (1d.cpp:749)
+    s.lL = w.lL;
+    s.lR = w.lR;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) s.flux[q] = 0.;
+    hllc_flux<Cfg>(ar, L, R, w, s.v, iface_area<Cfg>(xI), s.flux);
+    s.Sd = -1.;
+    s.pspec = -1.;
+    if (Cfg::SHOCK) {
+      double ps = 0.;
+      if (compute_Sd<Cfg>(ar, ph, L, R, &s.Sd, &ps)) s.pspec = ps;
+    }
+  }
+
+  // The hooks' arguments of run r, as step() forms them.
+  __device__ __forceinline__ static gamma_problem::HookArgs hook_args(const Tracks &T, const Phys &ph, int r, int n) {
+    const RunState &R = T.run[r];
+    return gamma_problem::HookArgs{T.par + (size_t)r * gamma_problem::PARAM_WORDS, ph.gamma_ad, R.t, R.it, n,
+                                   ph.ngst - 1, n - ph.ngst};
+  }
+
+  // Formulas formed again with the plain operators, where an operand left the
+  // range of FlatOps: rare, hence out of line.  The interface's solution goes
+  // through its shared slots (written by this thread only, before the chunk's
+  // next barrier).
+  __device__ __noinline__ static void solve_interface_plain(Smem &sm, const Tracks &T, const Phys &ph, int r, int n,
+                                                            int i, int c, double xI) {
+    PlainOps ar;
+    IfaceSol s;
+    solve_interface(ar, sm, ph, hook_args(T, ph, r, n), i, n, c, xI, s);
+#pragma unroll
+    for (int k = 0; k < NQS; ++k) sm.fl[k][c] = s.flux[Slots<Cfg>::q_of(k)];
+    sm.lL[c] = s.lL;
+    sm.lR[c] = s.lR;
+    sm.v[c] = s.v;
+    sm.xold[c] = s.Sd;
+    sm.xnew[c] = s.pspec;
+  }
+  __device__ __noinline__ static void pair_gradient_plain(Smem &sm, int k) {
+    const double d = sm.cen[k + 1] - sm.cen[k];
+    for (int s = 0; s < NQS; ++s) sm.gp[s][k] = qdiv(sm.cp[s][k + 1] - sm.cp[s][k], d);
+  }
+  __device__ __noinline__ static double centroid_plain(double x, double dx) { return make_geom<Cfg>(x, dx).cen; }
+
+  // Cell::update (cell.cpp:102-127) up to cons2prim: cons per volume after the
+  // stage, the primitives before it (the warm start) and the new geometry.
+  template <class Ar>
+  __device__ __forceinline__ static void advance_cell(Ar &ar, const Tracks &T, const Phys &ph,
+                                                      const gamma_problem::HookArgs &A, const SynchConst &sc,
+                                                      const Smem &sm, long long g, int tt, int stage, double dt,
+                                                      double *cons, double *prim, Geom &G1) {
+    const int c = tt + 1;
+#pragma unroll
+    for (int s = 0; s < NQS; ++s) prim[Slots<Cfg>::q_of(s)] = sm.cp[s][c];
+    prim[UU2] = 0.;
+    const Geom G0 = make_geom<Cfg>(ar, sm.cx[c], sm.cdx[c]);
+    prim2cons<Cfg>(ar, ph, prim, cons);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) cons[q] *= G0.dV;
+    if (stage == 1) {
+#pragma unroll
+      for (int s = 0; s < NQS; ++s) T.u0[s * T.N + g] = cons[Slots<Cfg>::q_of(s)];
+    }
+#pragma unroll
+    for (int s = 0; s < NQS; ++s) {
+      const int q = Slots<Cfg>::q_of(s);
+      cons[q] += (sm.fl[s][tt] - sm.fl[s][tt + 1]) * dt;
+    }
+    if (Cfg::SPH) {  // Cell::sourceTerms, 1D (rel_sph.cpp:452-466)
+      double p = prim[PPP];
+      double r = G0.x, dr = G0.dx, dV = G0.dV;
+      double r1 = r - dr / 2., r2 = r + dr / 2.;
+      double rsq = ar.quo(r2 * r2 + r1 * r1 + r2 * r1, ar.by(3.));
+      cons[SS1] += (2. * p) * ar.quo(r, ar.by(rsq)) * dV * dt;
+    }
+    if (Cfg::CYL) {  // Cell::sourceTerms of rel_cyl.cpp:358-364, r = G.x[r_]
+      cons[SS1] += ar.quo(prim[PPP], ar.by(G0.x)) * G0.dV * dt;
+    }
+    Hooks::user_source_terms(A, G0.x, G0.dx, G0.dV, prim, cons, dt);  // Cell::userSourceTerms
+    if (Cfg::SYNCH) {
+      const double dg = radiative_source<Cfg>(ar, ph, sc, prim, G0.dV, dt);
+      cons[GMX] += dg;
+      cons[GMN] += dg;
+    }
+    G1 = geom_between<Cfg>(ar, sm.xnew[tt], sm.xnew[tt + 1]);
+    per_volume(ar, cons, G1.dV);
+  }
+
+  // cons / dV
+  template <class Ar>
+  __device__ __forceinline__ static void per_volume(Ar &ar, double *cons, double dV) {
+    if (Cfg::FAST) {
+      const double rdV = ar.inv(dV);
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) cons[q] *= rdV;
+    } else {
+      const auto by = ar.by(dV);
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) cons[q] = q <= TAU ? ar.quo(cons[q], by) : ar.quo0(cons[q], by);
+    }
+  }
+
+  // RK3 combine (rk3.cpp:27-55, 63-92)
+  template <class Ar>
+  __device__ __forceinline__ static void combine_cell(Ar &ar, const Tracks &T, const Smem &sm, long long g, int tt,
+                                                      int stage, double dV1, double *cons) {
+    const double w0 = stage == 2 ? 3. / 4. : 1. / 3.;
+    const double w1 = stage == 2 ? 1. / 4. : 2. / 3.;
+#pragma unroll
+    for (int s = 0; s < NQS; ++s) {
+      const int q = Slots<Cfg>::q_of(s);
+      cons[q] = w0 * T.u0[s * T.N + g] + w1 * cons[q] * dV1;
+    }
+    per_volume(ar, cons, geom_between<Cfg>(ar, sm.xcmb[tt], sm.xcmb[tt + 1]).dV);
+  }
+
+  // The whole update of one cell, with the reference's warm starts; its
+  // cons2prim statistics.
+  template <class Ar>
+  __device__ __forceinline__ static void update_cell(Ar &ar, const Tracks &T, const Phys &ph,
+                                                     const gamma_problem::HookArgs &A, const SynchConst &sc,
+                                                     const Smem &sm, long long g, int tt, int stage, double dt,
+                                                     double *prim, C2PStats &c1, C2PStats &c2) {
+    double cons[NQ];
+    Geom G1;
+    advance_cell(ar, T, ph, A, sc, sm, g, tt, stage, dt, cons, prim, G1);
+    cons2prim<Cfg, Hooks>(ar, ph, cons, prim, &c1, A.par);
+    if (stage > 1) {
+      combine_cell(ar, T, sm, g, tt, stage, G1.dV, cons);
+      cons2prim<Cfg, Hooks>(ar, ph, cons, prim, &c2, A.par);
+    }
+  }
+  struct CellResult {
+    double prim[NQS];
+    C2PStats c1, c2;
+  };
+  __device__ __noinline__ static CellResult update_cell_plain(const Smem &sm, const Tracks &T, const Phys &ph, int r,
+                                                              int n, long long g, int tt, int stage, double dt) {
+    PlainOps ar;
+    const gamma_problem::HookArgs A = hook_args(T, ph, r, n);
+    SynchConst sc;
+    Hooks::synchrotron_norm(A.par, &sc.Nalpha, &sc.Nmp, &sc.Nme);
+    double prim[NQ];
+    CellResult R{};
+    update_cell(ar, T, ph, A, sc, sm, g, tt, stage, dt, prim, R.c1, R.c2);
+#pragma unroll
+    for (int s = 0; s < NQS; ++s) R.prim[s] = prim[Slots<Cfg>::q_of(s)];
+    return R;
   }
 
   // Cell::update_dt, moving direction (cell.cpp:47-74).  Returns false on a
@@ -263,13 +431,16 @@ struct TrackStep {
   // whose call frame costs local-memory traffic).
   __device__ GB_SWEEP_ATTR static double sweep(const Tracks &T, const Phys &ph, const gamma_problem::HookArgs &A,
                                               const SynchConst &sc,
-                                 Smem &sm, long long off, int n, int stage, int mode, double dt, double t,
+                                 Smem &sm, int r, long long off, int n, int stage, int mode, double dt,
                                  StepStats &st, const mlp::InferSmem *inf) {
     const int tid = threadIdx.x;
     const int ng = ph.ngst, iL = ng - 1, iR = n - ng;
+    // RK3 weights of the interface positions
     const double w0 = stage == 2 ? 3. / 4. : 1. / 3.;
     const double w1 = stage == 2 ? 1. / 4. : 2. / 3.;
     double run_min = DT_INF;
+    // the step with the learned guess keeps the plain operators
+    using Ops = typename std::conditional<GUESS, PlainOps, FlatOps>::type;
 
     for (int a = 0; a < n; a += CH) {
       // ---- stage cells a-1 .. a+CH+1 (slot k <-> cell a-1+k); slot 0 is carried
@@ -284,7 +455,10 @@ struct TrackStep {
           cell_geom(T, sm, off, n, ng, stage, i, (k == 1 && a > 0) ? &sm.xold[0] : nullptr, &gx, &gdx);
           sm.cx[k] = gx;
           sm.cdx[k] = gdx;
-          sm.cen[k] = make_geom<Cfg>(gx, gdx).cen;
+          Ops ar;
+          double cen = make_geom<Cfg>(ar, gx, gdx).cen;
+          if (ar.bad()) cen = centroid_plain(gx, gdx);
+          sm.cen[k] = cen;
         }
       }
       __syncthreads();
@@ -302,8 +476,11 @@ struct TrackStep {
 #pragma unroll
               for (int s = 0; s < NQS; ++s) sm.gp[s][k] = (sm.cp[s][k + 1] - sm.cp[s][k]) * rd;
             } else {
+              Ops ar;
+              const auto by = ar.by(d);
 #pragma unroll
-              for (int s = 0; s < NQS; ++s) sm.gp[s][k] = qdiv(sm.cp[s][k + 1] - sm.cp[s][k], d);
+              for (int s = 0; s < NQS; ++s) sm.gp[s][k] = ar.quo0(sm.cp[s][k + 1] - sm.cp[s][k], by);
+              if (ar.bad()) pair_gradient_plain(sm, k);
             }
           }
         }
@@ -331,25 +508,32 @@ struct TrackStep {
 #pragma unroll
           for (int s = 0; s < NQS; ++s) myflux[Slots<Cfg>::q_of(s)] = T.fl1[s * T.N + gi];
         } else {
-          FState<Cfg> L, R;
-          reconstruct(sm, ph, i, n, c, xI, L, R);
-          const Waves w = compute_lambda<Cfg>(ph, L, R);
-          double v = ph.vi * w.lS;
-          Hooks::user_kinematics(A, i, &v);  // Grid::userKinematics (1d.cpp:749)
-          my_lL = w.lL;
-          my_lR = w.lR;
-          my_v = v;
-          hllc_flux<Cfg>(L, R, w, v, iface_area<Cfg>(xI), myflux);
+          Ops ar;
+          IfaceSol sol;
+          solve_interface(ar, sm, ph, A, i, n, c, xI, sol);
+          if (ar.bad()) {
+            solve_interface_plain(sm, T, ph, r, n, i, c, xI);
+#pragma unroll
+            for (int k = 0; k < NQS; ++k) sol.flux[Slots<Cfg>::q_of(k)] = sm.fl[k][c];
+            sol.lL = sm.lL[c];
+            sol.lR = sm.lR[c];
+            sol.v = sm.v[c];
+            sol.Sd = sm.xold[c];
+            sol.pspec = sm.xnew[c];
+          }
+          my_lL = sol.lL;
+          my_lR = sol.lR;
+          my_v = sol.v;
+#pragma unroll
+          for (int q = 0; q < NQ; ++q) myflux[q] = sol.flux[q];
           if (Cfg::SHOCK) {  // measureShock into cell i (radiation_sph.cpp:160-175)
-            double Sd, ps;
-            const bool have = compute_Sd<Cfg>(ph, L, R, &Sd, &ps);
-            const double sd0 = fmax(T.sd[gi], Sd);
+            const double sd0 = fmax(T.sd[gi], sol.Sd);
             T.sd[gi] = sd0;
-            if (have && ps > T.pspec[gi]) T.pspec[gi] = ps;
+            if (sol.pspec > T.pspec[gi]) T.pspec[gi] = sol.pspec;
             if (stage == 1) T.shocked[gi] = sd0 > DETECT_SHOCK_THRESHOLD ? 1 : 0;  // detectShock
           }
           if (mode == 0) {  // keep the stage-1 solution for the update pass
-            T.v1[gi] = v;
+            T.v1[gi] = my_v;
 #pragma unroll
             for (int s = 0; s < NQS; ++s) T.fl1[s * T.N + gi] = myflux[Slots<Cfg>::q_of(s)];
           }
@@ -411,76 +595,33 @@ struct TrackStep {
       }
 
       if (mode == 1) {
-        // Cell::update (cell.cpp:102-127).  Written as straight-line blocks
-        // under `upd` so that, with the learned guess, the whole warp meets at
-        // each inference.
         const bool upd = i >= iL + 1 && i <= iR - 1;
         const long long g = off + i;
-        double prim[NQ], cons[NQ];
-        Geom G1;
-        if (upd) {
-#pragma unroll
-          for (int s = 0; s < NQS; ++s) prim[Slots<Cfg>::q_of(s)] = sm.cp[s][c];
-          prim[UU2] = 0.;
-          const Geom G0 = make_geom<Cfg>(sm.cx[c], sm.cdx[c]);
-          prim2cons<Cfg>(ph, prim, cons);
-#pragma unroll
-          for (int q = 0; q < NQ; ++q) cons[q] *= G0.dV;
-          if (stage == 1) {
-#pragma unroll
-            for (int s = 0; s < NQS; ++s) T.u0[s * T.N + g] = cons[Slots<Cfg>::q_of(s)];
-          }
-#pragma unroll
-          for (int s = 0; s < NQS; ++s) {
-            const int q = Slots<Cfg>::q_of(s);
-            cons[q] += (sm.fl[s][tt] - sm.fl[s][tt + 1]) * dt;
-          }
-          if (Cfg::SPH) {  // Cell::sourceTerms, 1D (rel_sph.cpp:452-466)
-            double p = prim[PPP];
-            double r = G0.x, dr = G0.dx, dV = G0.dV;
-            double r1 = r - dr / 2., r2 = r + dr / 2.;
-            double rsq = (r2 * r2 + r1 * r1 + r2 * r1) / 3.;
-            cons[SS1] += (2. * p) * (r / rsq) * dV * dt;
-          }
-          if (Cfg::CYL) {  // Cell::sourceTerms of rel_cyl.cpp:358-364, r = G.x[r_]
-            cons[SS1] += prim[PPP] / G0.x * G0.dV * dt;
-          }
-          Hooks::user_source_terms(A, G0.x, G0.dx, G0.dV, prim, cons, dt);  // Cell::userSourceTerms
-          if (Cfg::SYNCH) {
-            const double dg = radiative_source<Cfg>(ph, sc, prim, G0.dV, dt);
-            cons[GMX] += dg;
-            cons[GMN] += dg;
-          }
-          G1 = geom_between<Cfg>(sm.xnew[tt], sm.xnew[tt + 1]);
-          if (Cfg::FAST) {
-            const double rdV1 = 1. / G1.dV;
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) cons[q] *= rdV1;
-          } else {
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) cons[q] = q <= TAU ? cons[q] / G1.dV : qdiv(cons[q], G1.dV);
-          }
-        }
-        // every lane of the warp meets here (the network works across it)
-        cell_cons2prim(inf, ph, cons, prim, upd, st, A.par);
-        if (stage > 1) {
-          if (upd) {  // RK3 combine (rk3.cpp:27-55, 63-92)
-#pragma unroll
-            for (int s = 0; s < NQS; ++s) {
-              const int q = Slots<Cfg>::q_of(s);
-              cons[q] = w0 * T.u0[s * T.N + g] + w1 * cons[q] * G1.dV;
-            }
-            const Geom G2 = geom_between<Cfg>(sm.xcmb[tt], sm.xcmb[tt + 1]);
-            if (Cfg::FAST) {
-              const double rdV2 = 1. / G2.dV;
-#pragma unroll
-              for (int q = 0; q < NQ; ++q) cons[q] *= rdV2;
-            } else {
-#pragma unroll
-              for (int q = 0; q < NQ; ++q) cons[q] = q <= TAU ? cons[q] / G2.dV : qdiv(cons[q], G2.dV);
-            }
-          }
+        double prim[NQ];
+        if (GUESS) {
+          // blocks under `upd`, so that the whole warp meets at each inference
+          double cons[NQ];
+          Geom G1;
+          PlainOps ar;
+          if (upd) advance_cell(ar, T, ph, A, sc, sm, g, tt, stage, dt, cons, prim, G1);
           cell_cons2prim(inf, ph, cons, prim, upd, st, A.par);
+          if (stage > 1) {
+            if (upd) combine_cell(ar, T, sm, g, tt, stage, G1.dV, cons);
+            cell_cons2prim(inf, ph, cons, prim, upd, st, A.par);
+          }
+        } else if (upd) {
+          Ops ar;
+          C2PStats c1, c2;
+          update_cell(ar, T, ph, A, sc, sm, g, tt, stage, dt, prim, c1, c2);
+          if (ar.bad()) {
+            const CellResult R = update_cell_plain(sm, T, ph, r, n, g, tt, stage, dt);
+#pragma unroll
+            for (int s = 0; s < NQS; ++s) prim[Slots<Cfg>::q_of(s)] = R.prim[s];
+            c1 = R.c1;
+            c2 = R.c2;
+          }
+          count_c2p(st, c1, c1.poor);
+          if (stage > 1) count_c2p(st, c2, c2.poor);
         }
         if (upd) {
           if (Cfg::SYNCH && stage == (ph.euler ? 1 : 3)) {  // radiation_injectParticles, active cells
@@ -566,28 +707,22 @@ struct TrackStep {
     }
     __syncthreads();
 
-    // stage 1: ghosts, CFL candidates, dt
-    edge_geom(T, sm, off, n, ng, 1);
-    ghosts(T, ph, A, off, n, sm.edge);
-    __syncthreads();
-    double m = sweep(T, ph, A, sc, sm, off, n, 1, 0, 0., t, st, inf);
-    m = block_min(sm, m);
-    const double dt = ph.cfl * m;
-    // stage 1 update (the whole Grid::evolve of Timestep/euler.cpp)
-    sweep(T, ph, A, sc, sm, off, n, 1, 1, dt, t, st, inf);
-    __syncthreads();
-    if (!ph.euler) {
-      // stage 2
-      edge_geom(T, sm, off, n, ng, 2);
-      ghosts(T, ph, A, off, n, sm.edge);
-      __syncthreads();
-      sweep(T, ph, A, sc, sm, off, n, 2, 1, dt, t, st, inf);
-      __syncthreads();
-      // stage 3
-      edge_geom(T, sm, off, n, ng, 3);
-      ghosts(T, ph, A, off, n, sm.edge);
-      __syncthreads();
-      sweep(T, ph, A, sc, sm, off, n, 3, 1, dt, t, st, inf);
+    // The sweeps of the step: the stage-1 CFL pass, which gives dt, the stage-1
+    // update (the whole Grid::evolve of Timestep/euler.cpp), stage 2, stage 3.
+    // One loop, so that the kernel holds one copy of the sweep's code: four
+    // inlined copies overflow the instruction cache.
+    double dt = 0.;
+    const int npass = ph.euler ? 2 : 4;
+#pragma unroll 1
+    for (int pass = 0; pass < npass; ++pass) {
+      const int stage = pass < 2 ? 1 : pass;
+      if (pass != 1) {
+        edge_geom(T, sm, off, n, ng, stage);
+        ghosts(T, ph, A, off, n, sm.edge);
+        __syncthreads();
+      }
+      const double m = sweep(T, ph, A, sc, sm, r, off, n, stage, pass > 0 ? 1 : 0, dt, st, inf);
+      if (pass == 0) dt = ph.cfl * block_min(sm, m);
       __syncthreads();
     }
 
@@ -639,7 +774,7 @@ struct TrackStep {
 // chose this kernel, the one with (nonzero) or without (0) the learned guess.
 template <class Cfg, class Hooks, int BS, bool GUESS = false, int CPT = 1, int MINB = Cfg::MIN_BLOCKS>
 __global__ void __launch_bounds__(BS, MINB)
-    track_step_kernel(Tracks T, Phys ph, int nsteps, const int *order, int nruns, int *queue, StepStats *stats,
+    track_step_kernel(const __grid_constant__ Tracks T, const __grid_constant__ Phys ph, int nsteps, const int *order, int nruns, int *queue, StepStats *stats,
                       int regrid_only, unsigned words_bytes, const int *gate) {
   if (gate && ((*gate != 0) != GUESS)) return;
   using TS = TrackStep<Cfg, Hooks, BS, GUESS, CPT>;
