@@ -155,11 +155,10 @@ struct FState {
 
 template <class Ar>
 GB_HD double lfac_of(Ar &ar, double uu) {
-  // fluid.cpp:10-22 (u = sqrt(sum uu^2) then sqrt(1+u^2))
-  double u = 0.;
-  u += uu * uu;
-  u = ar.root(u);
-  return ar.root(1 + u * u);
+  // fluid.cpp:10-22 takes u = sqrt(uu^2) and then sqrt(1 + u^2): the root of a
+  // rounded square is the number itself, and where the square underflows
+  // 1 + u^2 is 1
+  return ar.root(1 + uu * uu);
 }
 GB_HD double lfac_of(double uu) {
   PlainOps ar;
@@ -405,45 +404,46 @@ GB_HD double c2p_f(const Phys &ph, double p, double D, double S2, double E, doub
   return f;
 }
 
-// f(p) and, on request, its slope; lfac and lfac^2 at p, and whether
-// 1 - S^2/W^2 was not negative there (else lfac is that of its magnitude).
+// f(p) with x = S^2/W^2, lfac and lfac^2 at p, and whether 1 - x was not
+// negative there (else lfac is that of its magnitude).
 struct C2PEval {
-  double f, df, lfac, l2;
+  double f, x, lfac, l2;
   bool inside;
 };
 
 // f in the reference's operation order (rel_sph.cpp:198-207, rel_cart.cpp:118-120).
 template <class Cfg, class Ar>
-GB_HD C2PEval c2p_f_ref(Ar &ar, const Phys &ph, double p, double D, double S, double E, bool slope,
-                        bool p_may_be_zero = false) {
+GB_HD C2PEval c2p_f_ref(Ar &ar, const Phys &ph, double p, double D, double S, double E, bool p_may_be_zero = false) {
   C2PEval e;
   const double W = E + p;
-  const double x = ar.quo0(S * S, ar.by(W * W));
-  const double arg = Cfg::SPH ? fabs(1. - x) : (1. - x);
+  e.x = ar.quo0(S * S, ar.by(W * W));
+  const double arg = Cfg::SPH ? fabs(1. - e.x) : (1. - e.x);
   const double lfac = ar.rroot(arg);
   const bool ideal = !Cfg::SPH || ph.eos == 0;
   const double gma = ideal ? ph.gamma_ad : eos_gamma(ar, ph, ar.quo(D, ar.by(lfac)), p);
   const auto gm1 = ideal ? by_gm1(ar, ph) : ar.by(gma - 1.);
-  // p = 0 at the bracket's lower end p_lo, which every search evaluates
+  // p = 0 at the bracket's lower end p_lo
   const double kp = gma * p * lfac * lfac;
   e.f = (E + p - D * lfac - (p_may_be_zero ? ar.quo0(kp, gm1) : ar.quo(kp, gm1)));
   e.l2 = lfac * lfac;
   e.lfac = lfac;
   e.inside = arg >= 0.;
-  e.df = 0.;
-  if (slope) {
-    if (!ideal) {  // Gamma_eff(p) terms: take them from the derivative form
-      double dfast;
-      c2p_f<Cfg>(ph, p, D, S * S, E, &dfast);
-      e.df = dfast;
-    } else {  // d lfac/dp = -lfac^3 x / W with the same lfac and x as f
-      const double sgn = (1. - x) >= 0. ? 1. : -1.;
-      const double dl = ar.quo0(-sgn * lfac * e.l2 * x, ar.by(W));
-      // kgam is GAMMA_/(GAMMA_-1) rounded once on the host: gma/(gma-1) exactly
-      e.df = 1. - D * dl - ph.kgam * (e.l2 + 2. * p * lfac * dl);
-    }
-  }
   return e;
+}
+
+// df/dp at p, after c2p_f_ref there
+template <class Cfg, class Ar>
+GB_HD double c2p_slope_ref(Ar &ar, const Phys &ph, double p, double D, double S, double E, const C2PEval &e) {
+  if (Cfg::SPH && ph.eos != 0) {  // Gamma_eff(p) terms: take them from the derivative form
+    double dfast;
+    c2p_f<Cfg>(ph, p, D, S * S, E, &dfast);
+    return dfast;
+  }
+  // d lfac/dp = -lfac^3 x / W with the same lfac and x as f
+  const double sgn = (1. - e.x) >= 0. ? 1. : -1.;
+  const double dl = ar.quo0(-sgn * e.lfac * e.l2 * e.x, ar.by(E + p));
+  // kgam is GAMMA_/(GAMMA_-1) rounded once on the host: gma/(gma-1) exactly
+  return 1. - D * dl - ph.kgam * (e.l2 + 2. * p * e.lfac * dl);
 }
 
 // What the root search returns: the pressure the reference would go on with
@@ -468,31 +468,44 @@ struct C2PRoot {
 template <class Cfg, class Ar>
 GB_HD C2PRoot c2p_pressure_body(Ar &ar, const Phys &ph, double D, double S, double S2, double E, double pCand,
                                 bool defer) {
-  auto feval = [&](double p, bool slope, bool p_may_be_zero = false) -> C2PEval {
-    if (!Cfg::FAST_ROOT) return c2p_f_ref<Cfg>(ar, ph, p, D, S, E, slope, p_may_be_zero);
+  auto feval = [&](double p, bool p_may_be_zero = false) -> C2PEval {
+    if (!Cfg::FAST_ROOT) return c2p_f_ref<Cfg>(ar, ph, p, D, S, E, p_may_be_zero);
     C2PEval e;
-    e.f = c2p_f<Cfg>(ph, p, D, S2, E, slope ? &e.df : nullptr, &e.l2);
+    e.f = c2p_f<Cfg>(ph, p, D, S2, E, nullptr, &e.l2);
+    e.x = 0.;
     e.lfac = sqrt(e.l2);
     e.inside = false;
     return e;
   };
+  auto slope = [&](double p, const C2PEval &e) -> double {
+    if (!Cfg::FAST_ROOT) return c2p_slope_ref<Cfg>(ar, ph, p, D, S, E, e);
+    double df;
+    c2p_f<Cfg>(ph, p, D, S2, E, &df);
+    return df;
+  };
   C2PRoot R;
   R.st = C2PStats{0, 0, 0, 0};
-  // f at the warm start, with its slope: the search starts there when the
-  // warm start lies in the bracket (f does not depend on whether df is asked for)
-  C2PEval e0 = feval(pCand, true);
+  // f at the warm start: the search starts there when it lies in the bracket
+  C2PEval e0 = feval(pCand);
   R.p = pCand;
   R.lfac = e0.inside ? e0.lfac : -1.;
   // rel_cyl.cpp:161 searches only where |f| exceeds 1e-13 (rel_sph, rel_cart: 0)
   if (fabs(e0.f) > (Cfg::CYL ? 1.e-13 : 0.)) {
-    R.st.poor = c2p_warm_start_poor(e0.f, e0.df, pCand);
+    double df = slope(pCand, e0);
+    R.st.poor = c2p_warm_start_poor(e0.f, df, pCand);
     if (defer && R.st.poor) {
       R.st.deferred = 1;
       return R;
     }
     double p_lo = fmax(0., (1. + 1e-13) * S - E);
+    // No solution where f(p_lo) < 0.  At p_lo = 0, f = E - D lfac with
+    // lfac^2 = E^2 / (E^2 - S^2): certainly not negative, whatever its rounding
+    // (lfac carries eps E^2 / (E^2 - S^2)), where D^2 stays that much below
+    // E^2 - S^2, as it does unless the gas is colder than p/rho ~ 1e-14 lfac^2;
+    // then f need not be formed (2 quotients and 2 roots of every search).
     bool find_p = true;
-    if (feval(p_lo, false, true).f < 0) find_p = false;
+    const bool surely = p_lo == 0. && D * D <= (E - S) * (E + S) - 0x1p-47 * (E * E);
+    if (!surely && feval(p_lo, true).f < 0) find_p = false;
     double p_hi;
     if (e0.f < 0) {
       p_hi = 1. * pCand;
@@ -501,7 +514,7 @@ GB_HD C2PRoot c2p_pressure_body(Ar &ar, const Phys &ph, double D, double S, doub
       // the reference grows p_hi without bound (a zero guess would never end);
       // 400 decades reach infinity, where f is NaN and the loop stops anyway.
       // Its first test re-evaluates f(pCand), which is e0.f.
-      for (int g = 0; g < 400 && (g == 0 ? e0.f : feval(p_hi, false).f) > 0; ++g) {
+      for (int g = 0; g < 400 && (g == 0 ? e0.f : feval(p_hi).f) > 0; ++g) {
         p_hi *= 10;
         if (Ar::FLAT && ar.bad()) break;
       }
@@ -512,7 +525,10 @@ GB_HD C2PRoot c2p_pressure_body(Ar &ar, const Phys &ph, double D, double S, doub
       double lo = p_lo, hi = p_hi;
       if (e0.f > 0.) lo = fmax(lo, pCand);
       double p = fmin(fmax(pCand, lo), hi);
-      if (!(p == pCand)) e0 = feval(p, true);
+      if (!(p == pCand)) {
+        e0 = feval(p);
+        df = slope(p, e0);
+      }
       const int MAXIT = 100;
       const double eps = 2.220446049250313e-16;
       int iters;
@@ -524,13 +540,14 @@ GB_HD C2PRoot c2p_pressure_body(Ar &ar, const Phys &ph, double D, double S, doub
         const double noise =
             eps * (E + p + D * e0.lfac * (1. + e0.l2) + 4. * p * e0.l2 * (1. + 2. * e0.l2));
         if (e0.f == 0. || fabs(e0.f) <= noise) break;
-        double pn = p - ar.quo(e0.f, ar.by(e0.df));
+        if (iters > 1) df = slope(p, e0);
+        double pn = p - ar.quo(e0.f, ar.by(df));
         if (!(pn > lo && pn < hi)) {
           // Newton left the bracket: bisect, geometrically once lo > 0
           pn = lo > 0. ? sqrt(lo) * sqrt(hi) : 0.5 * (lo + hi);
           if (!(pn > lo && pn < hi)) pn = 0.5 * (lo + hi);
         }
-        e0 = feval(pn, true);
+        e0 = feval(pn);
         if (e0.f > 0.) lo = pn;
         else if (e0.f < 0.) hi = pn;
         const double step = fabs(pn - p);
@@ -582,7 +599,7 @@ GB_HD C2PInput c2p_input(Ar &ar, const double *cons, const double *prim) {
   double S2 = 0.;
   S2 += in.ss * in.ss;
   in.S2 = S2;
-  in.S = Cfg::FAST_ROOT ? fabs(in.ss) : ar.root(S2);
+  in.S = Cfg::FAST_ROOT ? fabs(in.ss) : ar.root_of_square(in.ss, S2);  // sqrt(S2)
   in.pCand = Cfg::SPH ? fmax(1.e-13, prim[PPP]) : prim[PPP];
   return in;
 }
