@@ -99,10 +99,8 @@ struct gamma_ctx {
   cudaGraphExec_t gexec = nullptr;
   long long gkey[4] = {-1, -1, -1, -1};  // nsteps, variant, guess pointer, regrid_only of the graph
   int variant = 0;     // step-kernel launch shape (tune.h); 0 = the default kernel
-  // grid and shared memory of each launch shape, without [0] and with [1] the
-  // learned guess (grid 0: not configured yet)
-  int vgrid[2][gb::tune::kVariants] = {};
-  size_t vsmem[2][gb::tune::kVariants] = {};
+  // each launch shape, without [0] and with [1] the learned guess
+  gb::LaunchShape vshape[2][gb::tune::kVariants];
   std::string err;
 };
 
@@ -174,8 +172,8 @@ __global__ void k_guess_policy(const gb::StepStats *prev, int *use_guess) {
 }
 
 // Launch shape v of the context's step kernel, without or with the learned guess.
-int configure_launch(gamma_ctx *c, int v, bool guess, int *grid, size_t *smem) {
-  GB_CUDA(c, c->prob->configure(v, guess, c->nruns, c->max_cap, grid, smem));
+int configure_launch(gamma_ctx *c, int v, bool guess) {
+  GB_CUDA(c, c->prob->configure(v, guess, c->nruns, (int)(c->N / c->nruns), c->max_cap, &c->vshape[guess ? 1 : 0][v]));
   return GAMMA_OK;
 }
 
@@ -329,7 +327,7 @@ GAMMA_API int gamma_gpu_create(const gamma_config_t *cfg, int nruns, const int *
       cudaSuccess)
     return fail(e, "copy capacities");
   if ((e = cudaStreamSynchronize(c->stream)) != cudaSuccess) return fail(e, "sync");
-  int rc = configure_launch(c, 0, false, &c->vgrid[0][0], &c->vsmem[0][0]);
+  int rc = configure_launch(c, 0, false);
   if (rc != GAMMA_OK) {
     gamma_gpu_destroy(c);
     return rc;
@@ -446,7 +444,7 @@ int enqueue_steps(gamma_ctx_t *ctx, int nsteps, int regrid_only) {
   GB_CUDA(ctx, cudaMemsetAsync(ctx->d_stats, 0, sizeof(gb::StepStats), ctx->stream));
   const int v = ctx->variant;
   for (int k = 0; k <= (guess ? 1 : 0); ++k) {
-    const cudaError_t e = ctx->prob->launch(v, k == 1, ctx->vgrid[k][v], ctx->vsmem[k][v], ctx->stream, ctx->T,
+    const cudaError_t e = ctx->prob->launch(k == 1, ctx->vshape[k][v], ctx->stream, ctx->T,
                                             phys_of(ctx->cfg), nsteps, ctx->d_order, ctx->nruns, ctx->d_queue,
                                             ctx->d_stats, regrid_only, ctx->max_cap,
                                             guess ? ctx->d_use_guess : nullptr);
@@ -512,8 +510,8 @@ GAMMA_API int gamma_gpu_step(gamma_ctx_t *ctx, int nsteps, gamma_step_stats_t *s
 
 GAMMA_API int gamma_gpu_set_guess(gamma_ctx_t *ctx, const float *params) {
   if (!ctx) return GAMMA_ERR_INVALID;
-  if (params && !ctx->vgrid[1][ctx->variant]) {
-    int rc = configure_launch(ctx, ctx->variant, true, &ctx->vgrid[1][ctx->variant], &ctx->vsmem[1][ctx->variant]);
+  if (params && !ctx->vshape[1][ctx->variant].grid) {
+    int rc = configure_launch(ctx, ctx->variant, true);
     if (rc != GAMMA_OK) return rc;
   }
   if (params && !ctx->T.mlp) {  // the next step starts with the guess (k_guess_policy)
@@ -709,8 +707,8 @@ GAMMA_API int gamma_gpu_variant_info(int variant, int *threads, int *cells_per_t
 GAMMA_API int gamma_gpu_set_variant(gamma_ctx_t *ctx, int variant) {
   if (!ctx || variant < 0 || variant >= gb::tune::kVariants) return GAMMA_ERR_INVALID;
   for (int guess = 0; guess < 2; ++guess) {
-    if (ctx->vgrid[guess][variant] != 0 || (guess && !ctx->T.mlp)) continue;
-    const int rc = configure_launch(ctx, variant, guess != 0, &ctx->vgrid[guess][variant], &ctx->vsmem[guess][variant]);
+    if (ctx->vshape[guess][variant].grid != 0 || (guess && !ctx->T.mlp)) continue;
+    const int rc = configure_launch(ctx, variant, guess != 0);
     if (rc != GAMMA_OK) return rc;
   }
   ctx->variant = variant;

@@ -140,12 +140,11 @@ extern "C" GAMMA_API int gamma_gpu_step_tubes_noalloc(const gamma_config_t *cfg,
   // no refinement criterion, so the capacity does not size any shared memory)
   const gb::ProblemEntry *tube = gb::find_problem(GAMMA_PROBLEM_TUBE);
   if (!tube) return GAMMA_ERR_INVALID;
-  int grid = 0;
-  size_t smem = 0;
-  if (tube->configure(0, false, nruns, 0, &grid, &smem) != cudaSuccess) return GAMMA_ERR_CUDA;
+  gb::LaunchShape shape;
+  if (tube->configure(0, false, nruns, (int)(total / nruns), 0, &shape) != cudaSuccess) return GAMMA_ERR_CUDA;
   auto *qs = reinterpret_cast<int *>(ws + off_queue);
   auto *st = reinterpret_cast<gb::StepStats *>(ws + off_stats);
-  if (tube->launch(0, false, grid, smem, s, T, ph, nsteps, reinterpret_cast<const int *>(ws + off_order), nruns, qs,
+  if (tube->launch(false, shape, s, T, ph, nsteps, reinterpret_cast<const int *>(ws + off_order), nruns, qs,
                    st, 0, 0, nullptr) != cudaSuccess)
     return GAMMA_ERR_CUDA;
 

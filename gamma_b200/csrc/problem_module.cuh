@@ -18,15 +18,58 @@
 
 namespace gb {
 
+// One launch: the kernel (its shape in tune.h), grid, shared memory and CTAs per
+// run (a cluster).
+struct LaunchShape {
+  int kernel = 0;
+  int grid = 0;  // 0: not configured yet
+  size_t smem = 0;
+  int cluster = 1;
+};
+
+// CTAs per run for a CTA of `threads`: runs that leave SMs idle are spread over
+// clusters of up to 8 CTAs (the portable size), as many as there are SMs for
+// and cells to work on.
+inline int team_size(int nsm, int nruns, int cells, int threads) {
+  int c = 1;
+  while (c < 8 && 2LL * c * nruns <= nsm && c * threads < cells) c *= 2;
+  return c;
+}
+
+// The shape behind variant 0 on nsm SMs.  The runs of a batch differ in length
+// and each runs at its CTA's pace, so a batch that does not fill the GPU wants
+// more threads per run, and one that does wants small CTAs (their chunk barriers
+// stall fewer warps).  Measured us per step with 128, 256, 512 threads per run
+// (tubes of 1,001 to 8,191 cells; settled BM1D runs of 1,000 to 8,000 initial
+// cells), clusters by team_size:
+//   runs   tubes                 BM1D
+//     20    341   206   137      201   177   160
+//     72    646   392   256      302   236   256
+//    200   1302   770   494      511   398   429
+//    440   1606   927   684      728   696   718
+//    900   1881  1105  1403     1516  1283  1348
+//   4096 (256 to 8,192 cells)  3507  3618  4720
+inline int default_shape(int nsm, int nruns, int cells) {
+  const int most = nruns <= 3LL * nsm ? 512 : (nruns <= 16LL * nsm ? 256 : 128);
+  int c = 1;
+  while (c < 8 && 2LL * c * nruns <= nsm) c *= 2;
+  int threads = 128;
+  while (threads < most && c * threads < cells) threads *= 2;  // no more than the cells of a run
+  for (int v = 0; v < tune::kVariants; ++v)
+    if (tune::kShapes[v].threads == threads && tune::kShapes[v].cells_per_thread == 1) return v;
+  return 0;
+}
+
 struct ProblemEntry {
   const char *name;
   int id;       // a fixed id (the built-in GAMMA_PROBLEM_* values), or -1
   int modules;  // gamma_problem::MODULES_*
   bool regrid;  // Hooks::REGRID
-  // launch shape v of the step kernel, without or with the learned guess
-  cudaError_t (*configure)(int v, bool guess, int nruns, int max_cap, int *grid, size_t *smem);
+  // launch shape v of the step kernel, without or with the learned guess, for
+  // nruns runs of about `cells` cells (max_cap sizes the regrid's bit words)
+  cudaError_t (*configure)(int v, bool guess, int nruns, int cells, int max_cap, LaunchShape *shape);
   // gate: nullptr, or the step kernels' choice (track_step_kernel)
-  cudaError_t (*launch)(int v, bool guess, int grid, size_t smem, cudaStream_t s, const Tracks &T, const Phys &ph,
+  cudaError_t (*launch)(bool guess, const LaunchShape &shape, cudaStream_t s, const Tracks &T, const Phys &ph,
                         int nsteps, const int *order, int nruns, int *queue, StepStats *stats, int regrid_only,
                         int max_cap, const int *gate);
   // Simu::initialise of one run on the host (prim [NQ][cap])
@@ -72,24 +115,49 @@ struct ModuleKernel {
     if (GUESS) b = ((b + 15u) & ~size_t(15)) + sizeof(mlp::InferSmem);
     return b;
   }
-  static cudaError_t configure(int nruns, int max_cap, int *grid, size_t *sm) {
-    *sm = smem(max_cap);
-    cudaError_t e = raise_smem_limit((const void *)fn, *sm);
+  static cudaError_t configure(int nruns, int cells, int max_cap, LaunchShape *L) {
+    L->smem = smem(max_cap);
+    cudaError_t e = raise_smem_limit((const void *)fn, L->smem);
     if (e != cudaSuccess) return e;
     int dev = 0, nsm = 0, occ = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, BS, *sm)) != cudaSuccess) return e;
+    L->kernel = V;
+    L->cluster = team_size(nsm, nruns, cells, BS * CPT);
+    for (; L->cluster > 1; L->cluster /= 2) {
+      cudaLaunchAttribute at;
+      cudaLaunchConfig_t c = config(*L, &at, L->cluster, nullptr);
+      int nc = 0;
+      if ((e = cudaOccupancyMaxActiveClusters(&nc, fn, &c)) != cudaSuccess) return e;
+      if (nc < 1) continue;
+      L->grid = L->cluster * (nruns < nc ? nruns : nc);
+      return cudaSuccess;
+    }
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, BS, L->smem)) != cudaSuccess) return e;
     if (occ < 1) occ = 1;
-    *grid = nruns < nsm * occ ? nruns : nsm * occ;
+    L->grid = nruns < nsm * occ ? nruns : nsm * occ;
     return cudaSuccess;
   }
-  static cudaError_t launch(int grid, size_t sm, cudaStream_t s, const Tracks &T, const Phys &ph, int nsteps,
+  static cudaLaunchConfig_t config(const LaunchShape &L, cudaLaunchAttribute *at, int grid, cudaStream_t s) {
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = L.cluster;
+    at->val.clusterDim.y = at->val.clusterDim.z = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(BS);
+    c.dynamicSmemBytes = L.smem;
+    c.stream = s;
+    c.attrs = at;
+    c.numAttrs = L.cluster > 1 ? 1 : 0;
+    return c;
+  }
+  static cudaError_t launch(const LaunchShape &L, cudaStream_t s, const Tracks &T, const Phys &ph, int nsteps,
                             const int *order, int nruns, int *queue, StepStats *stats, int regrid_only, int max_cap,
                             const int *gate) {
-    fn<<<grid, BS, sm, s>>>(T, ph, nsteps, order, nruns, queue, stats, regrid_only,
-                            module_words_bytes<Hooks>(max_cap), gate);
-    return cudaGetLastError();
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t c = config(L, &at, L.grid, s);
+    return cudaLaunchKernelEx(&c, fn, T, ph, nsteps, order, nruns, queue, stats, regrid_only,
+                              module_words_bytes<Hooks>(max_cap), gate);
   }
 };
 
@@ -97,12 +165,19 @@ struct ModuleKernel {
 static_assert(tune::kVariants == 8, "GB_MODULE_SHAPES lists every launch shape");
 
 template <class C, class Hooks>
-cudaError_t module_configure(int v, bool guess, int nruns, int max_cap, int *grid, size_t *smem) {
+cudaError_t module_configure(int v, bool guess, int nruns, int cells, int max_cap, LaunchShape *L) {
+  if (v == 0) {
+    int dev = 0, nsm = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    v = default_shape(nsm, nruns, cells);
+  }
   switch (v) {
 #define GB_CASE(k)                                                                       \
   case k:                                                                                \
-    return guess ? ModuleKernel<C, Hooks, k, true>::configure(nruns, max_cap, grid, smem) \
-                 : ModuleKernel<C, Hooks, k, false>::configure(nruns, max_cap, grid, smem);
+    return guess ? ModuleKernel<C, Hooks, k, true>::configure(nruns, cells, max_cap, L)      \
+                 : ModuleKernel<C, Hooks, k, false>::configure(nruns, cells, max_cap, L);
     GB_MODULE_SHAPES(GB_CASE)
 #undef GB_CASE
   }
@@ -110,16 +185,16 @@ cudaError_t module_configure(int v, bool guess, int nruns, int max_cap, int *gri
 }
 
 template <class C, class Hooks>
-cudaError_t module_launch(int v, bool guess, int grid, size_t smem, cudaStream_t s, const Tracks &T, const Phys &ph,
+cudaError_t module_launch(bool guess, const LaunchShape &L, cudaStream_t s, const Tracks &T, const Phys &ph,
                           int nsteps, const int *order, int nruns, int *queue, StepStats *stats, int regrid_only,
                           int max_cap, const int *gate) {
-  switch (v) {
-#define GB_CASE(k)                                                                                             \
-  case k:                                                                                                      \
-    return guess ? ModuleKernel<C, Hooks, k, true>::launch(grid, smem, s, T, ph, nsteps, order, nruns, queue,  \
-                                                           stats, regrid_only, max_cap, gate)                  \
-                 : ModuleKernel<C, Hooks, k, false>::launch(grid, smem, s, T, ph, nsteps, order, nruns, queue, \
-                                                            stats, regrid_only, max_cap, gate);
+  switch (L.kernel) {
+#define GB_CASE(k)                                                                                              \
+  case k:                                                                                                       \
+    return guess ? ModuleKernel<C, Hooks, k, true>::launch(L, s, T, ph, nsteps, order, nruns, queue, stats,     \
+                                                           regrid_only, max_cap, gate)                          \
+                 : ModuleKernel<C, Hooks, k, false>::launch(L, s, T, ph, nsteps, order, nruns, queue, stats,    \
+                                                            regrid_only, max_cap, gate);
     GB_MODULE_SHAPES(GB_CASE)
 #undef GB_CASE
   }

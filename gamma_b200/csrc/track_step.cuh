@@ -1,20 +1,34 @@
-// One CTA advances one run (one 1D track of cells) through whole RK3 steps.
+// One team advances one run (one 1D track of cells) through whole RK3 steps: one
+// CTA, or a cluster of CTAs where there are fewer runs than the GPU has room for.
 //
 // Per step (src/simu.cpp:79-105): [regrid] -> reset shocks -> ghosts ->
-// stage-1 CFL candidates -> per-run dt (block min) -> stage-1 update ->
+// stage-1 CFL candidates -> per-run dt (team min) -> stage-1 update ->
 // ghosts -> stage-2 fluxes+update+RK combine -> ghosts -> stage-3 -> inject.
 // With the Euler module (Timestep/euler.cpp:12-19) the step ends after the
 // stage-1 update: inject, and no RK combine.
 //
-// Each stage is one left-to-right sweep over the track in chunks of BS cells
-// (one interface and one cell per thread).  A chunk stages the stencil
-// (cells a-1 .. a+BS+1) in shared memory, computes the BS interfaces
-// a .. a+BS-1 (PLM + HLLC at the contact-speed interface), then updates cells
-// a .. a+BS-1 in place.  The old state of cell a+BS-1 and the results of
-// interface a+BS-1 are carried to the next chunk, so the in-place update never
-// feeds a neighbour's stencil.  Runs are independent (own dt, own regrid), so
-// a CTA takes runs from a work queue and can advance each by many steps
-// without any grid-wide synchronisation.
+// Each CTA owns a segment of consecutive cells (alone, the whole track).  Each
+// stage is one left-to-right sweep over the segment in chunks of CH = BS CPT
+// cells (one interface and one cell per thread at a time).  A chunk stages the
+// stencil (cells a-1 .. a+CH+1) in shared memory, computes the interfaces
+// a .. a+CH-1 (PLM + HLLC at the contact-speed interface), then updates cells
+// a .. a+CH-1 in place.  The old state of cell a+CH-1 and the results of
+// interface a+CH-1 are carried to the next chunk, so the in-place update never
+// feeds a neighbour's stencil.  The last three staged cells and the gradients
+// between them move to the next chunk's first slots, so that staging and
+// gradients take one pass of the threads each.  In a team, a segment's first
+// chunk starts at the interface on its left, which its neighbour computes too
+// (the same bits); the two cells beyond either end are read before any CTA
+// updates (halo), and the CTAs wait for one another twice per stage.
+// Measured at 20 steps a call, one B200: 12 tubes of 1,001 to 8,191 cells take
+// 1,951 us per step with a CTA each and 102 us with 8, one tube of 500 cells 131
+// and 48 us, one BM1D run of 2,000 initial cells 560 and 107 us.
+// (A segment per warp, whose warps wait only twice per stage, is slower: 4,096
+// tubes 3.97 against 3.58 ms per step, the BM1D sweep 1.82 against 1.38 ms.  The
+// warps drift apart and no longer share the instruction cache.)
+// Runs are independent (own dt, own regrid), so a team takes runs from a work
+// queue and can advance each by many steps without any grid-wide
+// synchronisation.
 #pragma once
 
 #include "gamma_problem.h"
@@ -75,8 +89,23 @@ struct StepStats {
 };
 
 
-// BS threads advance one run; each sweep chunk holds CPT cells per thread
-// (CH = BS * CPT), which a thread takes in turn.  Hooks: the problem module
+// The CTAs that advance one run (a cluster), and this one's rank.
+struct Team {
+  int ncta, rank;
+
+  // every thread of the team: what any wrote before is seen by all after
+  __device__ __forceinline__ void sync() const {
+    if (ncta == 1) {
+      __syncthreads();
+    } else {
+      asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+      asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    }
+  }
+};
+
+// BS threads of each CTA of the team; each sweep chunk holds CPT cells per
+// thread (CH = BS CPT), which a thread takes in turn.  Hooks: the problem module
 // (include/gamma_problem.h), whose hooks run where the reference calls its
 // own: userBoundaries in ghosts, userKinematics and userSourceTerms in the
 // sweep, cons2prim_user in cons2prim, checkCellForRegrid in regrid_track.
@@ -88,31 +117,60 @@ struct TrackStep {
   static constexpr int NC = CH + 3;    // staged cells per chunk: a-1 .. a+CH+1
 
   struct Smem {
+    // by cell (rows of NC; the carry between chunks treats them as one array)
     double cp[NQS][NC];  // staged primitives
     double cx[NC], cdx[NC], cen[NC];
-    double fl[NQS][CH + 1];  // interface fluxes; slot 0 = carry (interface a-1)
-    double lL[CH + 1], lR[CH + 1], v[CH + 1];
-    double xold[CH + 1], xnew[CH + 1], xcmb[CH + 1];
     double gp[NQS][NC];  // gradient between slots k and k+1 (grad())
-    double red[BS / 32];
-    double edge[4];  // x, dx of the left and right edge cells this stage
-    int ints[4];
+    // by interface (rows of CH+1; slot 0 = interface a-1)
+    double fl[NQS][CH + 1];  // interface fluxes
+    double lL[CH + 1], lR[CH + 1], v[CH + 1];
+    double xnew[CH + 1], xcmb[CH + 1];
+    // the segment's surroundings as the stage finds them: cells s-2, s-1, e,
+    // e+1 and the interface on its left
+    double hp[NQS][4], hx[4], hdx[4], hxI;
+    double edge[4];  // x, dx of the track's left and right edge cells this stage
+    double red[BS / 32], cta_min;
   };
 
   // --- helpers ------------------------------------------------------------
 
-  __device__ static double block_min(Smem &sm, double v) {
+  __device__ __forceinline__ static double warp_min(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    return v;
+  }
+  // min over the team (order-free); every thread gets it
+  __device__ static double team_min(Smem &sm, const Team &tm, double v) {
+    v = warp_min(v);
+    if ((threadIdx.x & 31) == 0) sm.red[threadIdx.x >> 5] = v;
     __syncthreads();
-    if (l == 0) sm.red[w] = v;
-    __syncthreads();
-    double r = sm.red[0];
+    double m = sm.red[0];
 #pragma unroll
-    for (int k = 1; k < BS / 32; ++k) r = fmin(r, sm.red[k]);
-    __syncthreads();
-    return r;
+    for (int k = 1; k < BS / 32; ++k) m = fmin(m, sm.red[k]);
+    if (tm.ncta > 1) {
+      if (threadIdx.x == 0) sm.cta_min = m;
+      tm.sync();
+      const unsigned mine = (unsigned)__cvta_generic_to_shared(&sm.cta_min);
+      for (int c = 0; c < tm.ncta; ++c) {
+        unsigned theirs;
+        double x;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(theirs) : "r"(mine), "r"(c));
+        asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(x) : "r"(theirs) : "memory");
+        m = fmin(m, x);
+      }
+    } else {
+      __syncthreads();
+    }
+    return m;
+  }
+
+  // The segment [s, e) of the team's CTA c of nc: whole chunks as far as they
+  // go.  A first chunk that starts at the interface on its left holds one cell
+  // less.
+  __device__ __forceinline__ static void segment(int n, int nc, int c, int &s, int &e) {
+    const int k = (n + nc - 1 + nc * CH - 1) / (nc * CH);  // chunks per CTA
+    s = min(n, c == 0 ? 0 : CH * k + (c - 1) * (CH * k - 1));
+    e = min(n, CH * k + c * (CH * k - 1));
   }
 
   __device__ static void load_prim(const Tracks &T, long long g, double *p) {
@@ -160,25 +218,52 @@ struct TrackStep {
 
   // Geometry of cell i during the current stage.  Active cells: the step-start
   // arrays (stage 1) or the span of their interfaces (stages 2, 3: set by
-  // Cell::move and CellGeomFromInterfacePos).  Ghosts: shifted copies of the
-  // edge cells (updateGhosts).
-  __device__ static void cell_geom(const Tracks &T, const Smem &sm, long long off, int n, int ng, int stage,
-                                   int i, const double *xIold_prev, double *gx, double *gdx) {
+  // Cell::move and CellGeomFromInterfacePos; xL: the left one's position where
+  // it may no longer be read).  Ghosts: shifted copies of the edge cells
+  // (updateGhosts).
+  __device__ __forceinline__ static void cell_geom(const Tracks &T, const double *edge, long long off, int n, int ng,
+                                                   int stage, int i, const double *xLp, double *gx, double *gdx) {
     const int iL = ng - 1, iR = n - ng;
     if (i <= iL) {
-      *gx = sm.edge[0] - (iL - i + 1) * sm.edge[1];
-      *gdx = sm.edge[1];
+      *gx = edge[0] - (iL - i + 1) * edge[1];
+      *gdx = edge[1];
     } else if (i >= iR) {
-      *gx = sm.edge[2] + (i - iR + 1) * sm.edge[3];
-      *gdx = sm.edge[3];
+      *gx = edge[2] + (i - iR + 1) * edge[3];
+      *gdx = edge[3];
     } else if (stage == 1) {
       *gx = T.x[off + i];
       *gdx = T.dx[off + i];
     } else {
-      const double xL = xIold_prev ? *xIold_prev : T.xI[off + i - 1];
+      const double xL = xLp ? *xLp : T.xI[off + i - 1];
       const double xR = T.xI[off + i];
       *gx = (xR + xL) / 2.;
       *gdx = (xR - xL);
+    }
+  }
+
+  // The surroundings of the CTA's segment, before any CTA updates.  Ghost
+  // cells and interfaces are formed here as ghosts() forms them: they are being
+  // written meanwhile.
+  __device__ static void load_halo(const Tracks &T, const Phys &ph, const gamma_problem::HookArgs &A, Smem &sm,
+                                   long long off, int n, int stage, int s, int e) {
+    const int ng = ph.ngst, iL = ng - 1, iR = n - ng;
+    const int k = threadIdx.x;
+    if (k < 4 && s < e) {
+      const int i = k < 2 ? s - 2 + k : e + k - 2;
+      if (i >= 0 && i < n) {
+        double gx, gdx, p[NQ];
+        cell_geom(T, sm.edge, off, n, ng, stage, i, nullptr, &gx, &gdx);
+        load_prim(T, off + min(max(i, iL + 1), iR - 1), p);
+        if (i <= iL || i >= iR) Hooks::user_boundaries(A, i, gx, p);
+#pragma unroll
+        for (int q = 0; q < NQS; ++q) sm.hp[q][k] = p[Slots<Cfg>::q_of(q)];
+        sm.hx[k] = gx;
+        sm.hdx[k] = gdx;
+      }
+    }
+    if (k == 4 && s > 0 && s < e) {
+      const int i = s - 1;
+      sm.hxI = i >= iR ? T.xI[off + iR - 1] + (i - iR) * sm.edge[3] : T.xI[off + i];
     }
   }
 
@@ -254,8 +339,8 @@ struct TrackStep {
 
   // Formulas formed again with the plain operators, where an operand left the
   // range of FlatOps: rare, hence out of line.  The interface's solution goes
-  // through its shared slots (written by this thread only, before the chunk's
-  // next barrier).
+  // through its shared slots (written by this lane only, before the warp's next
+  // synchronisation).
   __device__ __noinline__ static void solve_interface_plain(Smem &sm, const Tracks &T, const Phys &ph, int r, int n,
                                                             int i, int c, double xI) {
     PlainOps ar;
@@ -266,8 +351,8 @@ struct TrackStep {
     sm.lL[c] = s.lL;
     sm.lR[c] = s.lR;
     sm.v[c] = s.v;
-    sm.xold[c] = s.Sd;
-    sm.xnew[c] = s.pspec;
+    sm.xnew[c] = s.Sd;
+    sm.xcmb[c] = s.pspec;
   }
   __device__ __noinline__ static void pair_gradient_plain(Smem &sm, int k) {
     const double d = sm.cen[k + 1] - sm.cen[k];
@@ -383,11 +468,17 @@ struct TrackStep {
 
   // Cell::update_dt, moving direction (cell.cpp:47-74).  Returns false on a
   // negative candidate (the reference's exit(30)).
-  __device__ static bool dt_candidate(double a, double lR_left, double v_right, double lL_right, double v_left,
-                                      double *cand) {
-    double dL = (lR_left > v_right) ? a / (lR_left - v_right) : DT_INF;
-    double dR = (lL_right < v_left) ? a / (v_left - lL_right) : DT_INF;
-    *cand = fmin(dL, dR);
+  __device__ __forceinline__ static bool dt_candidate(double a, double lR_left, double v_right, double lL_right,
+                                                      double v_left, double *cand) {
+    const bool onL = lR_left > v_right, onR = lL_right < v_left;
+    FlatOps ar;
+    double dL = ar.quo(a, ar.by(onL ? lR_left - v_right : 1.));
+    double dR = ar.quo(a, ar.by(onR ? v_left - lL_right : 1.));
+    if (ar.bad()) {
+      dL = a / (lR_left - v_right);
+      dR = a / (v_left - lL_right);
+    }
+    *cand = fmin(onL ? dL : DT_INF, onR ? dR : DT_INF);
     return !(*cand < 0);
   }
 
@@ -424,15 +515,13 @@ struct TrackStep {
     if (upd) count_c2p(st, cs, poor);
   }
 
-  // --- one stage sweep ------------------------------------------------------
-  // mode 0: stage-1 CFL candidates only (returns the run's min dt_loc and
+  // --- one stage sweep of the CTA's segment [s, e) ----------------------------
+  // mode 0: stage-1 CFL candidates only (returns the thread's min dt_loc and
   //         resets dt_loc); mode 1: fluxes + update (+ RK combine for stage>1).
-  // Inlined into the step (measured faster than one shared out-of-line copy,
-  // whose call frame costs local-memory traffic).
   __device__ GB_SWEEP_ATTR static double sweep(const Tracks &T, const Phys &ph, const gamma_problem::HookArgs &A,
-                                              const SynchConst &sc,
-                                 Smem &sm, int r, long long off, int n, int stage, int mode, double dt,
-                                 StepStats &st, const mlp::InferSmem *inf) {
+                                               const SynchConst &sc, Smem &sm, int r, long long off, int n, int s,
+                                               int e, int stage, int mode, double dt, StepStats &st,
+                                               const mlp::InferSmem *inf) {
     const int tid = threadIdx.x;
     const int ng = ph.ngst, iL = ng - 1, iR = n - ng;
     // RK3 weights of the interface positions
@@ -441,18 +530,30 @@ struct TrackStep {
     double run_min = DT_INF;
     // the step with the learned guess keeps the plain operators
     using Ops = typename std::conditional<GUESS, PlainOps, FlatOps>::type;
+    const int a0 = s > 0 ? s - 1 : 0;
+    const int last = min(n - 1, e + 1);  // last staged cell
+    if (s >= e) return run_min;  // a short track leaves the last CTAs without cells
 
-    for (int a = 0; a < n; a += CH) {
-      // ---- stage cells a-1 .. a+CH+1 (slot k <-> cell a-1+k); slot 0 is carried
-      for (int k = tid + 1; k < NC; k += BS) {
+    for (int a = a0; a < e; a += CH) {
+      // ---- stage cells a-1 .. a+CH+1 (slot k <-> cell a-1+k); slots 0..2 are
+      // carried from the previous chunk
+      for (int k = tid + (a > a0 ? 3 : 0); k < NC; k += BS) {
         const int i = a - 1 + k;
-        if (i < n) {
-          const long long g = off + i;
-#pragma unroll
-          for (int s = 0; s < NQS; ++s) sm.cp[s][k] = T.prim[s * T.N + g];
+        if (i >= 0 && i <= last) {
           double gx, gdx;
-          // cell a's left interface was rewritten by the previous chunk: use its carried old position
-          cell_geom(T, sm, off, n, ng, stage, i, (k == 1 && a > 0) ? &sm.xold[0] : nullptr, &gx, &gdx);
+          if (i < s || i >= e) {
+            const int h = i < s ? i - s + 2 : i - e + 2;
+#pragma unroll
+            for (int q = 0; q < NQS; ++q) sm.cp[q][k] = sm.hp[q][h];
+            gx = sm.hx[h];
+            gdx = sm.hdx[h];
+          } else {
+            const long long g = off + i;
+#pragma unroll
+            for (int q = 0; q < NQS; ++q) sm.cp[q][k] = T.prim[q * T.N + g];
+            // (the left interface of the segment's first cell is another CTA's)
+            cell_geom(T, sm.edge, off, n, ng, stage, i, i == s && s > 0 ? &sm.hxI : nullptr, &gx, &gdx);
+          }
           sm.cx[k] = gx;
           sm.cdx[k] = gdx;
           Ops ar;
@@ -464,9 +565,9 @@ struct TrackStep {
       __syncthreads();
       if (!(mode == 1 && stage == 1)) {
         // grad() between staged cells k and k+1: (q[k+1] - q[k]) / (cen[k+1] - cen[k]),
-        // each used by the three interfaces around it (slots past the track end unused)
-        for (int k = tid; k < NC - 1; k += BS) {
-          if ((a > 0 || k > 0) && a + k < n) {  // slots k and k+1 both hold cells
+        // each used by the three interfaces around it
+        for (int k = tid + (a > a0 ? 2 : 0); k < NC - 1; k += BS) {
+          if (a - 1 + k >= 0 && a + k <= last) {  // slots k and k+1 both hold cells
             const double d = sm.cen[k + 1] - sm.cen[k];
             // in the reference's order unless every formula may move (FAST_RIEMANN):
             // minmod of two equal slopes is 0 (1d.cpp:250-260), and a split's two
@@ -474,12 +575,12 @@ struct TrackStep {
             if (Cfg::FAST_RIEMANN) {
               const double rd = 1. / d;
 #pragma unroll
-              for (int s = 0; s < NQS; ++s) sm.gp[s][k] = (sm.cp[s][k + 1] - sm.cp[s][k]) * rd;
+              for (int q = 0; q < NQS; ++q) sm.gp[q][k] = (sm.cp[q][k + 1] - sm.cp[q][k]) * rd;
             } else {
               Ops ar;
               const auto by = ar.by(d);
 #pragma unroll
-              for (int s = 0; s < NQS; ++s) sm.gp[s][k] = ar.quo0(sm.cp[s][k + 1] - sm.cp[s][k], by);
+              for (int q = 0; q < NQS; ++q) sm.gp[q][k] = ar.quo0(sm.cp[q][k + 1] - sm.cp[q][k], by);
               if (ar.bad()) pair_gradient_plain(sm, k);
             }
           }
@@ -492,16 +593,16 @@ struct TrackStep {
       for (int u = 0; u < CPT; ++u) {
       const int tt = tid + u * BS;
       const int i = a + tt;
-      const bool has_if = i <= n - 2;
+      const bool has_if = i <= n - 2 && i < e;
+      const bool own = i >= s;  // else the left neighbour keeps its results
       const int c = tt + 1;  // slot of cell i
       double myflux[NQ];
 #pragma unroll
       for (int q = 0; q < NQ; ++q) myflux[q] = 0.;
-      double my_lL = 0, my_lR = 0, my_v = 0, my_xold = 0, my_xnew = 0, my_xcmb = 0;
+      double my_lL = 0, my_lR = 0, my_v = 0, my_xnew = 0, my_xcmb = 0;
       if (has_if) {
         const long long gi = off + i;
-        const double xI = T.xI[gi];
-        my_xold = xI;
+        const double xI = own ? T.xI[gi] : sm.hxI;
         if (mode == 1 && stage == 1) {
           // stage-1 fluxes and velocities were solved by the CFL pass
           my_v = T.v1[gi];
@@ -518,21 +619,21 @@ struct TrackStep {
             sol.lL = sm.lL[c];
             sol.lR = sm.lR[c];
             sol.v = sm.v[c];
-            sol.Sd = sm.xold[c];
-            sol.pspec = sm.xnew[c];
+            sol.Sd = sm.xnew[c];
+            sol.pspec = sm.xcmb[c];
           }
           my_lL = sol.lL;
           my_lR = sol.lR;
           my_v = sol.v;
 #pragma unroll
           for (int q = 0; q < NQ; ++q) myflux[q] = sol.flux[q];
-          if (Cfg::SHOCK) {  // measureShock into cell i (radiation_sph.cpp:160-175)
+          if (Cfg::SHOCK && own) {  // measureShock into cell i (radiation_sph.cpp:160-175)
             const double sd0 = fmax(T.sd[gi], sol.Sd);
             T.sd[gi] = sd0;
             if (sol.pspec > T.pspec[gi]) T.pspec[gi] = sol.pspec;
             if (stage == 1) T.shocked[gi] = sd0 > DETECT_SHOCK_THRESHOLD ? 1 : 0;  // detectShock
           }
-          if (mode == 0) {  // keep the stage-1 solution for the update pass
+          if (mode == 0 && own) {  // keep the stage-1 solution for the update pass
             T.v1[gi] = my_v;
 #pragma unroll
             for (int s = 0; s < NQS; ++s) T.fl1[s * T.N + gi] = myflux[Slots<Cfg>::q_of(s)];
@@ -542,14 +643,14 @@ struct TrackStep {
           // Interface::move, then the RK combine of interface positions
           my_xnew = xI + dt * my_v;
           if (stage == 1) {
-            T.xI0[gi] = xI;
+            if (own) T.xI0[gi] = xI;
             my_xcmb = my_xnew;
           } else if (i >= iL && i <= iR - 1) {
             my_xcmb = w0 * T.xI0[gi] + w1 * my_xnew;
           } else {
             my_xcmb = my_xnew;
           }
-          T.xI[gi] = my_xcmb;
+          if (own) T.xI[gi] = my_xcmb;
         }
       }
       // cell n-1 has no interface of its own; as for every cell, the shock
@@ -558,7 +659,6 @@ struct TrackStep {
       sm.lR[tt + 1] = my_lR;
       sm.v[tt + 1] = my_v;
       if (mode == 1) {
-        sm.xold[tt + 1] = my_xold;
         sm.xnew[tt + 1] = my_xnew;
         sm.xcmb[tt + 1] = my_xcmb;
 #pragma unroll
@@ -573,7 +673,8 @@ struct TrackStep {
       const int tt = tid + u * BS;
       const int i = a + tt;
       const int c = tt + 1;
-      if (i < n) {
+      const bool mine = i >= s && i < e;
+      if (mine) {
         const long long g = off + i;
         if (i >= 1 && i <= n - 2 && (mode == 0 || stage > 1)) {
           double cand;
@@ -595,7 +696,7 @@ struct TrackStep {
       }
 
       if (mode == 1) {
-        const bool upd = i >= iL + 1 && i <= iR - 1;
+        const bool upd = mine && i >= iL + 1 && i <= iR - 1;
         const long long g = off + i;
         double prim[NQ];
         if (GUESS) {
@@ -632,85 +733,96 @@ struct TrackStep {
       }
       }
       __syncthreads();
-      // ---- carry cell a+CH-1 and interface a+CH-1 to the next chunk
-      if (tid == 0) {
-        sm.lL[0] = sm.lL[CH];
-        sm.lR[0] = sm.lR[CH];
-        sm.v[0] = sm.v[CH];
-        sm.xold[0] = sm.xold[CH];
-        sm.xnew[0] = sm.xnew[CH];
-        sm.xcmb[0] = sm.xcmb[CH];
-        sm.cx[0] = sm.cx[CH];
-        sm.cdx[0] = sm.cdx[CH];
-        sm.cen[0] = sm.cen[CH];
-      }
-      if (tid < NQS) {
-        sm.fl[tid][0] = sm.fl[tid][CH];
-        sm.cp[tid][0] = sm.cp[tid][CH];
+      // ---- cells a+CH-1 .. a+CH+1, their gradients and interface a+CH-1 to
+      // the next chunk's first slots
+      if (a + CH < e) {
+        constexpr int CELLS = 3 * (2 * NQS + 3), IFACES = NQS + 5;
+        double *cell = &sm.cp[0][0], *iface = &sm.fl[0][0];
+#pragma unroll
+        for (int k = tid; k < CELLS + IFACES; k += BS) {
+          if (k < CELLS) {
+            double *row = cell + (k / 3) * NC + k % 3;
+            row[0] = row[CH];
+          } else {
+            double *row = iface + (k - CELLS) * (CH + 1);
+            row[0] = row[CH];
+          }
+        }
       }
       __syncthreads();
     }
     return run_min;
   }
 
-  // Edge-cell geometry for the current stage (written to sm.edge)
+  // Edge-cell geometry for the current stage
   __device__ static void edge_geom(const Tracks &T, Smem &sm, long long off, int n, int ng, int stage) {
-    if (threadIdx.x == 0) {
-      const int e[2] = {ng, n - ng - 1};
-      for (int k = 0; k < 2; ++k) {
-        const long long g = off + e[k];
-        double gx, gdx;
-        if (stage == 1) {
-          gx = T.x[g];
-          gdx = T.dx[g];
-        } else {
-          const double xL = T.xI[g - 1], xR = T.xI[g];
-          gx = (xR + xL) / 2.;
-          gdx = (xR - xL);
-        }
-        sm.edge[2 * k] = gx;
-        sm.edge[2 * k + 1] = gdx;
+    if (threadIdx.x < 2) {
+      const long long g = off + (threadIdx.x == 0 ? ng : n - ng - 1);
+      double gx, gdx;
+      if (stage == 1) {
+        gx = T.x[g];
+        gdx = T.dx[g];
+      } else {
+        const double xL = T.xI[g - 1], xR = T.xI[g];
+        gx = (xR + xL) / 2.;
+        gdx = (xR - xL);
       }
+      sm.edge[2 * threadIdx.x] = gx;
+      sm.edge[2 * threadIdx.x + 1] = gdx;
     }
     __syncthreads();
   }
 
   // --- one full step of run r ---------------------------------------------
-  __device__ static void step(const Tracks &T, const Phys &ph, Smem &sm, uint32_t *words, int r, StepStats &st,
-                              bool regrid_only, const mlp::InferSmem *inf) {
+  // Starts and ends with the team in step (what one wrote, all see).
+  __device__ static void step(const Tracks &T, const Phys &ph, Smem &sm, const Team &tm, uint32_t *words, int r,
+                              StepStats &st, bool regrid_only, const mlp::InferSmem *inf) {
     const long long off = T.off[r];
     const double *par = T.par + (size_t)r * gamma_problem::PARAM_WORDS;
     SynchConst sc;
     Hooks::synchrotron_norm(par, &sc.Nalpha, &sc.Nmp, &sc.Nme);
     RunState &R = T.run[r];
     int n = R.ntrack;
-    const double t = R.t;
     const int ng = ph.ngst;
+    const int tid = tm.rank * BS + threadIdx.x, nth = tm.ncta * BS;  // place in the team
+    const bool first = tm.rank == 0 && threadIdx.x == 0;
 
-    if (Hooks::REGRID) {
-      n = regrid_track<Cfg, Hooks, BS>(T.prim, T.N, T.x, T.dx, T.dtl, T.xI, off, n, T.cap[r], ph, par, T.rg,
-                                       words, st.splits, st.merges);
-      __syncthreads();
+    if (Hooks::REGRID) {  // one CTA's work; its result reaches the others through R
+      if (tm.rank == 0)
+        n = regrid_track<Cfg, Hooks, BS>(T.prim, T.N, T.x, T.dx, T.dtl, T.xI, off, n, T.cap[r], ph, par, T.rg,
+                                         words, st.splits, st.merges);
+      if (tm.ncta > 1) {
+        tm.sync();  // every CTA has read the old count
+        if (first) R.ntrack = n;
+        tm.sync();
+        n = R.ntrack;
+      } else {
+        __syncthreads();
+      }
     }
-    const gamma_problem::HookArgs A{par, ph.gamma_ad, t, R.it, n, ng - 1, n - ng};
+    const gamma_problem::HookArgs A{par, ph.gamma_ad, R.t, R.it, n, ng - 1, n - ng};
     if (regrid_only) {
-      if (threadIdx.x == 0) R.ntrack = n;
-      __syncthreads();
+      if (first) R.ntrack = n;
+      tm.sync();
       return;
     }
     if (Cfg::SHOCK) {  // Cell::resetShock
-      for (int i = threadIdx.x; i < n; i += BS) {
+      for (int i = tid; i < n; i += nth) {
         T.sd[off + i] = -1.;
         T.pspec[off + i] = 0.;
         T.shocked[off + i] = 0;
       }
+      tm.sync();
     }
-    __syncthreads();
 
     // The sweeps of the step: the stage-1 CFL pass, which gives dt, the stage-1
     // update (the whole Grid::evolve of Timestep/euler.cpp), stage 2, stage 3.
     // One loop, so that the kernel holds one copy of the sweep's code: four
-    // inlined copies overflow the instruction cache.
+    // inlined copies overflow the instruction cache.  Before a stage's first
+    // sweep every CTA reads its surroundings and one of them writes the ghosts;
+    // nobody updates until all have.
+    int s, e;
+    segment(n, tm.ncta, tm.rank, s, e);
     double dt = 0.;
     const int npass = ph.euler ? 2 : 4;
 #pragma unroll 1
@@ -718,12 +830,13 @@ struct TrackStep {
       const int stage = pass < 2 ? 1 : pass;
       if (pass != 1) {
         edge_geom(T, sm, off, n, ng, stage);
-        ghosts(T, ph, A, off, n, sm.edge);
-        __syncthreads();
+        if (tm.rank == 0) ghosts(T, ph, A, off, n, sm.edge);
+        if (tm.ncta > 1) load_halo(T, ph, A, sm, off, n, stage, s, e);
+        tm.sync();
       }
-      const double m = sweep(T, ph, A, sc, sm, r, off, n, stage, pass > 0 ? 1 : 0, dt, st, inf);
-      if (pass == 0) dt = ph.cfl * block_min(sm, m);
-      __syncthreads();
+      const double m = sweep(T, ph, A, sc, sm, r, off, n, s, e, stage, pass > 0 ? 1 : 0, dt, st, inf);
+      if (pass == 0) dt = ph.cfl * team_min(sm, tm, m);
+      else tm.sync();
     }
 
     // step-end cell geometry.  RK3: ghosts 0 and n-1 keep the stage-3 ghost
@@ -731,7 +844,7 @@ struct TrackStep {
     // Euler: only Cell::update moves cells (iL+1..iR-1); every ghost keeps
     // its stage-1 copy.
     const int iL = ng - 1, iR = n - ng;
-    for (int i = threadIdx.x; i < n; i += BS) {
+    for (int i = tid; i < n; i += nth) {
       double gx, gdx;
       if (ph.euler ? (i <= iL || i >= iR) : (i == 0 || i == n - 1)) {
         if (i <= iL) {
@@ -757,14 +870,14 @@ struct TrackStep {
       }
     }
     if (st.status) R.status = st.status;  // any thread; every writer stores the same code
-    if (threadIdx.x == 0) {
+    if (first) {
       R.ntrack = n;
       R.dt = dt;
-      R.t = t + dt;
+      R.t = R.t + dt;
       R.it = R.it + 1;
     }
-    st.zone_updates += (unsigned long long)(n - 2 * ng);
-    __syncthreads();
+    if (tm.rank == 0) st.zone_updates += (unsigned long long)(n - 2 * ng);
+    tm.sync();
   }
 };
 
@@ -788,22 +901,26 @@ __global__ void __launch_bounds__(BS, MINB)
     __syncthreads();
   }
   StepStats st{};
-  __shared__ int s_item, s_status;
-  for (;;) {
-    if (threadIdx.x == 0) s_item = atomicAdd(queue, 1);
-    __syncthreads();
-    const int item = s_item;
-    __syncthreads();
+  Team tm;
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(tm.ncta));
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(tm.rank));
+  __shared__ int s_item;
+  // one CTA per run: a queue; a cluster per run: every nteams-th run
+  const int nteams = gridDim.x / tm.ncta;
+  for (int item = blockIdx.x / tm.ncta;; item += nteams) {
+    if (tm.ncta == 1) {
+      if (threadIdx.x == 0) s_item = atomicAdd(queue, 1);
+      __syncthreads();
+      item = s_item;
+      __syncthreads();
+    }
     if (item >= nruns) break;
     const int r = order[item];
     for (int k = 0; k < nsteps; ++k) {
-      // a run whose step failed stops (block-uniform test)
-      if (threadIdx.x == 0) s_status = T.run[r].status;
-      __syncthreads();
-      const int bad = s_status;
-      __syncthreads();
-      if (bad != 0) break;
-      TS::step(T, ph, sm, words, r, st, regrid_only != 0, inf);
+      // a run whose step failed stops (its status is the same to all: the step
+      // before ended with the team in step)
+      if (T.run[r].status != 0) break;
+      TS::step(T, ph, sm, tm, words, r, st, regrid_only != 0, inf);
     }
   }
   // fold the per-thread statistics into the launch totals

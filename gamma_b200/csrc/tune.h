@@ -1,10 +1,12 @@
 // Launch-shape variants of the 1D step kernel for the autotuner
-// (gamma_gpu_autotune).  Variant 0 is the default (128 threads per run, one
-// cell per thread per sweep chunk); variants 1.. change the threads per run
-// (the CTA size) and the cells each thread takes per chunk.  Every problem
-// module instantiates all of them (problem_module.cuh).  The arithmetic of
-// every cell is the same in all of them, so they give identical results; only
-// the speed differs.
+// (gamma_gpu_autotune).  Variant 0 is the default: 128 threads per run, one
+// cell per thread per sweep chunk, or, in a batch that does not fill the GPU
+// that way, one of the larger CTAs (default_shape in problem_module.cuh).
+// Variants 1.. fix the threads per CTA and the cells each thread takes per
+// chunk.  In any of them a run may be spread over a cluster of CTAs (team_size
+// there).  Every problem module instantiates all of them
+// (problem_module.cuh).  The arithmetic of every cell is the same in all of
+// them, so they give identical results; only the speed differs.
 #pragma once
 
 namespace gb {
