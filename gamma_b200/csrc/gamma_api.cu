@@ -295,6 +295,9 @@ GAMMA_API int gamma_gpu_create(const gamma_config_t *cfg, int nruns, const int *
     GB_ALLOC(S.ndtl, 2 * N * d);
     GB_ALLOC(S.nrifx, 2 * N * d);
     GB_ALLOC(S.nrif, 2 * N * sizeof(int));
+    GB_ALLOC(S.ncur, 2 * N * sizeof(int));
+    GB_ALLOC(S.nvic, 2 * N * sizeof(int));
+    GB_ALLOC(S.nstate, 2 * N * sizeof(int));
     GB_ALLOC(S.seg_start, 4 * N * sizeof(int));
     GB_ALLOC(S.seg_src, 4 * N * sizeof(int));
     GB_ALLOC(S.tprim, nqs * N * d);

@@ -9,15 +9,25 @@
 // therefore inherently sequential, but almost every cell is a no-op whose
 // decision does not depend on earlier actions.  So:
 //   A. all threads evaluate the criterion for every original cell in the
-//      original context (bitmasks of split / merge / high-pressure cells);
+//      original context (bitmasks of split / merge / high-pressure cells); a
+//      track where none acts is left as it is;
 //   B. one thread replays the loop exactly.  For an untouched original cell the
 //      precomputed decision is valid whenever its distance to the shock is the
 //      same as in the original context (checked per cell); runs of valid no-op
 //      cells are skipped a bitmask word at a time, so the replay costs
 //      O(actions + cells/32).  New cells and cells near a moved shock are
 //      evaluated in place.  The replay emits the new track as segments
-//      (a run of original cells, or one new cell);
-//   C. all threads expand the segments into the new track.
+//      (a run of original cells, or one new cell).  A merged cell is never
+//      examined itself, so the replay only notes its two cells, and takes its
+//      high-pressure mark to be theirs (where they differ, it is formed at
+//      once);
+//   C. all threads form the merged cells (a merged cell's victim may be a merged
+//      cell: rounds) and compare their marks with the assumed ones; if one
+//      differs, the replay runs again and forms each merged cell as it goes;
+//   D. all threads expand the segments into the new track.
+// Merged one by one inside the replay, the first regrids of a sweep took 10 of
+// its 11 ms per step (thousands of merges per run, each a chain of loads, two
+// state conversions and a pressure root on one thread).
 #pragma once
 
 #include "physics.cuh"
@@ -29,13 +39,17 @@ struct RegridScratch {
   double *nprim;                    // [NQS][2N] new cells of run r at 2*off[r] + id
   double *nx, *ndx, *ndtl, *nrifx;  // [2N]
   int *nrif;                        // [2N] right interface: original index, or -1 (then nrifx)
+  int *ncur, *nvic;                 // [2N] a merged cell's two cells: original index, or -(id+1)
+  int *nstate;                      // [2N] the round that formed the cell, or kMergeLeft / kMergeRight
   int *seg_start, *seg_src;         // [4N] at 4*off[r]: output position; src >= 0 original, else -(id+1)
   double *tprim;                    // [NQS][N] compaction target
   double *tx, *tdx, *tdtl, *txI;    // [N]
   long long N;
 };
 
-// One cell as seen by the replay: an original (data fetched lazily) or new.
+constexpr int kMergeLeft = -1, kMergeRight = -2;  // merged cells still to be formed
+
+// One cell's record: an original (data fetched lazily) or new.
 template <class Cfg>
 struct RCell {
   double prim[Cfg::NQ];
@@ -156,23 +170,28 @@ __device__ void split_cells(const RCell<Cfg> &cL, const RCell<Cfg> &c, const RCe
 }
 
 // Merge cell c with victim v (Grid::merge, 1d.cpp:665-728).
+// (With the plain operators: a few lanes merge, and FlatOps' longer code costs
+// more instruction fetches than its overlap gains, 1.91 against 1.79 ms per step
+// of a sweep's first steps.)
 template <class Cfg, class Hooks>
-__device__ void merge_cells(const Phys &ph, const RCell<Cfg> &c, const RCell<Cfg> &v, bool left, RCell<Cfg> &M,
-                            C2PStats *cs, const double *par) {
+__device__ __forceinline__ void merge_cells(const Phys &ph, const RCell<Cfg> &c, const RCell<Cfg> &v, bool left,
+                                            RCell<Cfg> &M, const double *par) {
   constexpr int NQ = Cfg::NQ;
+  PlainOps ar;
   double cc[NQ], cv[NQ], cons[NQ];
-  prim2cons<Cfg>(ph, c.prim, cc);
-  prim2cons<Cfg>(ph, v.prim, cv);
-  const double dV_loc = make_geom<Cfg>(c.x, c.dx).dV;
-  const double dV_vic = make_geom<Cfg>(v.x, v.dx).dV;
+  prim2cons<Cfg>(ar, ph, c.prim, cc);
+  prim2cons<Cfg>(ar, ph, v.prim, cv);
+  const double dV_loc = make_geom<Cfg>(ar, c.x, c.dx).dV;
+  const double dV_vic = make_geom<Cfg>(ar, v.x, v.dx).dV;
+  const auto by = ar.by(dV_loc + dV_vic);
 #pragma unroll
-  for (int q = 0; q < NQ; ++q) cons[q] = (cc[q] * dV_loc + cv[q] * dV_vic) / (dV_loc + dV_vic);
+  for (int q = 0; q < NQ; ++q) cons[q] = ar.quo0(cc[q] * dV_loc + cv[q] * dV_vic, by);
   if (left) M.x = ((v.x - v.dx / 2.) + (c.x + c.dx / 2.)) / 2.;
   else M.x = ((v.x + v.dx / 2.) + (c.x - c.dx / 2.)) / 2.;
   M.dx = c.dx + v.dx;
 #pragma unroll
   for (int q = 0; q < NQ; ++q) M.prim[q] = c.prim[q];
-  cons2prim<Cfg, Hooks>(ph, cons, M.prim, cs, par);
+  cons2prim<Cfg, Hooks>(ar, ph, cons, M.prim, nullptr, par);
   M.dtl = c.dtl;
   if (left) {
     M.rif = c.rif;
@@ -184,6 +203,62 @@ __device__ void merge_cells(const Phys &ph, const RCell<Cfg> &c, const RCell<Cfg
   M.orig = -1;
   M.loaded = true;
 }
+
+// The scratch records of run r's new cells (from 2*off).
+template <class Cfg>
+__device__ __forceinline__ void store_new_cell(const RegridScratch &S, long long gid, const RCell<Cfg> &c) {
+#pragma unroll
+  for (int s = 0; s < Cfg::NQ - 1; ++s) S.nprim[s * 2 * S.N + gid] = c.prim[s < 3 ? s : s + 1];
+  S.nx[gid] = c.x;
+  S.ndx[gid] = c.dx;
+  S.ndtl[gid] = c.dtl;
+  S.nrif[gid] = c.rif;
+  S.nrifx[gid] = c.rifx;
+}
+
+// The whole record of cell d (an original, or formed new cell -(id+1)).
+template <class Cfg>
+__device__ __forceinline__ RCell<Cfg> whole_cell(const RegridView<Cfg> &V, const RegridScratch &S, long long noff,
+                                                 int d) {
+  RCell<Cfg> c;
+  if (d >= 0) {
+    c = V.orig_cell(d);
+    V.fetch(c);
+  } else {
+    const long long gid = noff + (-d - 1);
+#pragma unroll
+    for (int s = 0; s < Cfg::NQ - 1; ++s) c.prim[s < 3 ? s : s + 1] = S.nprim[s * 2 * S.N + gid];
+    c.prim[UU2] = 0.;
+    c.x = S.nx[gid];
+    c.dx = S.ndx[gid];
+    c.dtl = S.ndtl[gid];
+    c.rif = S.nrif[gid];
+    c.rifx = S.nrifx[gid];
+    c.orig = -1;
+    c.loaded = true;
+  }
+  return c;
+}
+
+// Forms merged cell id from its two cells, the examined one and its victim (the
+// cell on its left or right), and stores its record; returns its
+// high-pressure mark.  Out of line: it is the regrid's, not the step's.
+template <class Cfg, class Hooks>
+__device__ __noinline__ bool form_merged(const Phys &ph, const RegridView<Cfg> &V, const RegridScratch &S,
+                                         long long noff, int id, int cur, int vic, bool left, const double *par) {
+  const RCell<Cfg> c = whole_cell(V, S, noff, cur), v = whole_cell(V, S, noff, vic);
+  RCell<Cfg> M;
+  merge_cells<Cfg, Hooks>(ph, c, v, left, M, par);
+  store_new_cell(S, noff + id, M);
+  return Hooks::regrid_marker(par, M.prim);
+}
+
+// A cell of the walk: what the decisions need of it.
+struct WalkCell {
+  int d;      // original index, or -(id+1)
+  double dx;  // (of an original: once loaded)
+  bool has_dx, hp;
+};
 
 // Shared-memory words needed by regrid_track for a track of capacity cap.
 __host__ __device__ constexpr int regrid_words(int cap) { return (cap + 31) / 32; }
@@ -207,8 +282,8 @@ __device__ int regrid_track(double *prim, long long N, double *x, double *dx, do
   constexpr int NQS = NQ - 1;
   const int ng = ph.ngst, iL = ng - 1, iR0 = n - ng;
   const int nw = regrid_words(cap);
-  uint32_t *hpw = words, *spw = words + nw, *mgw = words + 2 * nw, *outhp = words + 3 * nw;
-  __shared__ int s_hpmax, s_nnew, s_nseg, s_first;
+  uint32_t *hpw = words, *spw = words + nw, *mgw = words + 2 * nw;
+  __shared__ int s_hpmax, s_nnew, s_nseg, s_first, s_nid;
   const double rOut0 = x[off + iR0 - 1];
   auto load = [&](long long g, double *p) {
 #pragma unroll
@@ -252,18 +327,23 @@ __device__ int regrid_track(double *prim, long long N, double *x, double *dx, do
     }
   }
   __syncthreads();
-  // interesting = split | merge (reuse spw|mgw on the fly)
+  bool acts = false;
+  for (int w = threadIdx.x; w < nw; w += BS) acts = acts || (spw[w] | mgw[w]) != 0u;
+  if (!__syncthreads_or(acts)) return n;  // no cell acts, so none moves, so each decision stands
 
-  // ---- B. sequential replay (thread 0)
-  if (threadIdx.x == 0) {
-    RegridView<Cfg> V{prim, N, x, dx, dtl, xI, off};
+  const RegridView<Cfg> V{prim, N, x, dx, dtl, xI, off};
+  const long long noff = 2 * off;
+  unsigned long long walk_splits = 0, walk_merges = 0;
+
+  // ---- B. sequential replay (thread 0); eager: each merged cell formed at once
+  auto walk = [&](bool eager) {
     int *seg_start = S.seg_start + 4 * off;
     int *seg_src = S.seg_src + 4 * off;
-    const long long noff = 2 * off;
     int nseg = 0, out = 0, nid = 0;
     int seg_next_orig = -2;  // original index that would extend the open segment
     int hp_final = -1;       // rightmost final position (> iL) holding a high-pressure cell
     int first_change = n;    // first output position that differs from the input
+    walk_splits = walk_merges = 0;
 
     auto emit_orig_range = [&](int k0, int k1) {  // originals [k0, k1) at positions out..
       if (k1 <= k0) return;
@@ -278,39 +358,49 @@ __device__ int regrid_track(double *prim, long long N, double *x, double *dx, do
       out += k1 - k0;
       seg_next_orig = k1;
     };
-    auto emit = [&](RCell<Cfg> &c) {
-      if (c.orig >= 0) {
-        emit_orig_range(c.orig, c.orig + 1);
+    auto emit = [&](const WalkCell &c) {
+      if (c.d >= 0) {
+        emit_orig_range(c.d, c.d + 1);
         return;
       }
-      const int id = nid++;
-      const long long gid = noff + id;
-#pragma unroll
-      for (int s = 0; s < NQS; ++s) S.nprim[s * 2 * S.N + gid] = c.prim[s < 3 ? s : s + 1];
-      S.nx[gid] = c.x;
-      S.ndx[gid] = c.dx;
-      S.ndtl[gid] = c.dtl;
-      S.nrif[gid] = c.rif;
-      S.nrifx[gid] = c.rifx;
       seg_start[nseg] = out;
-      seg_src[nseg] = -(id + 1);
+      seg_src[nseg] = c.d;
       ++nseg;
       seg_next_orig = -2;
       if (first_change > out) first_change = out;
-      if (out > iL && Hooks::regrid_marker(par, c.prim)) hp_final = max(hp_final, out);
+      if (out > iL && c.hp) hp_final = max(hp_final, out);
       ++out;
     };
-    auto is_hp = [&](const RCell<Cfg> &c) -> bool {
-      if (c.orig >= 0) return bit_of(hpw, c.orig);
-      return Hooks::regrid_marker(par, c.prim);
+    auto orig = [&](int k) { return WalkCell{k, 0., false, bit_of(hpw, k)}; };
+    auto width = [&](WalkCell &c) {
+      if (!c.has_dx) {
+        c.dx = dx[off + c.d];
+        c.has_dx = true;
+      }
+      return c.dx;
+    };
+    // form new cell d if it waits (its victim first, and so on down)
+    auto form = [&](int d) {
+      while (d < 0 && S.nstate[noff + (-d - 1)] < 0) {
+        int t = d;
+        for (int v; (v = S.nvic[noff + (-t - 1)]) < 0 && S.nstate[noff + (-v - 1)] < 0;) t = v;
+        const long long gid = noff + (-t - 1);
+        form_merged<Cfg, Hooks>(ph, V, S, noff, -t - 1, S.ncur[gid], S.nvic[gid], S.nstate[gid] == kMergeLeft, par);
+        S.nstate[gid] = 0;
+      }
+    };
+    auto add_new = [&](const RCell<Cfg> &c) {  // a half of a split cell
+      const int id = nid++;
+      store_new_cell(S, noff + id, c);
+      S.nstate[noff + id] = 0;
+      return WalkCell{-(id + 1), c.dx, true, Hooks::regrid_marker(par, c.prim)};
     };
 
     int ntrack = n, iR = iR0;
     emit_orig_range(0, iL);
-    RCell<Cfg> prev = V.orig_cell(iL), curc = V.orig_cell(iL + 1);
+    WalkCell prev = orig(iL), curc = orig(iL + 1);
     int k = iL + 2;
     int i = iL + 1;
-    C2PStats cs;
     while (i <= iR - 1) {
       // current shock index (rightmost high-pressure cell among positions iL+1..iR-1)
       int iS;
@@ -318,30 +408,30 @@ __device__ int regrid_track(double *prim, long long N, double *x, double *dx, do
         iS = i + 1 + (hpMax - k);
       } else {
         iS = hp_final;
-        if (i - 1 > iL && is_hp(prev)) iS = max(iS, i - 1);
-        if (is_hp(curc)) iS = max(iS, i);
+        if (i - 1 > iL && prev.hp) iS = max(iS, i - 1);
+        if (curc.hp) iS = max(iS, i);
         if (iS < 0) iS = iL + 1;
       }
       int action;
       bool valid = false;
-      if (curc.orig >= 0) {
-        const int dc = i - iS, d0 = curc.orig - (int)iS0;
+      if (curc.d >= 0) {
+        const int dc = i - iS, d0 = curc.d - (int)iS0;
         const bool mc = 0 < dc && dc < Hooks::REGRID_WINDOW, m0 = 0 < d0 && d0 < Hooks::REGRID_WINDOW;
         if (mc == m0) {
           valid = true;
-          action = bit_of(spw, curc.orig) ? SPLIT : (bit_of(mgw, curc.orig) ? MERGE : SKIP);
+          action = bit_of(spw, curc.d) ? SPLIT : (bit_of(mgw, curc.d) ? MERGE : SKIP);
         }
       }
       if (!valid) {
-        V.fetch(curc);
+        const RCell<Cfg> c = whole_cell(V, S, noff, curc.d);  // an original, or a split's half
         double rOut;
-        if (iR - 1 == i) rOut = curc.x;
+        if (iR - 1 == i) rOut = c.x;
         else rOut = x[off + k + (iR - 1 - (i + 1))];
-        action = Hooks::check_cell_for_regrid(par, curc.dx, curc.prim, i, iS, rOut);
+        action = Hooks::check_cell_for_regrid(par, c.dx, c.prim, i, iS, rOut);
       } else if (action == SKIP) {
         // skip a run of original no-op cells whose distance to the shock
         // matches the original context (no action moves anything meanwhile)
-        const int kc = curc.orig;
+        const int kc = curc.d;
         const int delta = i - kc;
         int lim = kc + (iR - i);  // positions i .. iR-1 can be examined
         const bool aligned = (hpMax >= k) || (iS - delta == (int)iS0);
@@ -356,18 +446,14 @@ __device__ int regrid_track(double *prim, long long N, double *x, double *dx, do
         }
         // first original > kc whose precomputed action is not a no-op
         int m = kc + 1;
-        while (m < lim) {
-          const int ms = next_set(spw, m, lim), mm = next_set(mgw, m, lim);
-          m = min(ms, mm);
-          break;
-        }
+        if (m < lim) m = min(next_set(spw, m, lim), next_set(mgw, m, lim));
         if (m > lim) m = lim;
         const int J = m - kc;  // examined no-op positions i .. i+J-1
         if (J >= 2) {
           emit(prev);
           emit_orig_range(kc, m - 1);
-          prev = V.orig_cell(m - 1);
-          curc = V.orig_cell(m);
+          prev = orig(m - 1);
+          curc = orig(m);
           k = m + 1;
           i += J;
           continue;
@@ -375,50 +461,53 @@ __device__ int regrid_track(double *prim, long long N, double *x, double *dx, do
       }
 
       if (action == SPLIT && ntrack < cap - 1) {
-        V.fetch(prev);
-        V.fetch(curc);
-        RCell<Cfg> nxt = V.orig_cell(k);
-        V.fetch(nxt);
+        form(prev.d);
         RCell<Cfg> A, B;
-        split_cells<Cfg>(prev, curc, nxt, A, B);
+        split_cells<Cfg>(whole_cell(V, S, noff, prev.d), whole_cell(V, S, noff, curc.d), whole_cell(V, S, noff, k), A,
+                         B);
         emit(prev);
-        prev = A;
-        curc = B;
+        prev = add_new(A);
+        curc = add_new(B);
         ++ntrack;
         ++iR;
-        ++nsplit;
+        ++walk_splits;
         ++i;
         continue;
       }
       if (action == MERGE && ntrack > 2 * ng + 2) {
-        V.fetch(prev);
-        V.fetch(curc);
-        RCell<Cfg> nxt = V.orig_cell(k);
-        V.fetch(nxt);
-        const bool left = (prev.dx < nxt.dx && i != ng) || i == iR - 1;
-        RCell<Cfg> M;
+        WalkCell nxt = orig(k);
+        const bool left = (width(prev) < width(nxt) && i != ng) || i == iR - 1;
+        WalkCell &vic = left ? prev : nxt;
+        const int id = nid++;
+        const long long gid = noff + id;
+        S.ncur[gid] = curc.d;
+        S.nvic[gid] = vic.d;
+        S.nstate[gid] = left ? kMergeLeft : kMergeRight;
+        WalkCell M{-(id + 1), width(curc) + width(vic), true, curc.hp};
+        if (eager || curc.hp != vic.hp) {
+          form(vic.d);
+          M.hp = form_merged<Cfg, Hooks>(ph, V, S, noff, id, curc.d, vic.d, left, par);
+          S.nstate[gid] = 0;
+        }
         if (left) {
-          merge_cells<Cfg, Hooks>(ph, curc, prev, true, M, &cs, par);
           emit(M);
           prev = nxt;
-          curc = V.orig_cell(k + 1);
         } else {
-          merge_cells<Cfg, Hooks>(ph, curc, nxt, false, M, &cs, par);
           emit(prev);
           prev = M;
-          curc = V.orig_cell(k + 1);
         }
+        curc = orig(k + 1);
         k += 2;
         --ntrack;
         --iR;
-        ++nmerge;
+        ++walk_merges;
         ++i;
         continue;
       }
       // no action
       emit(prev);
       prev = curc;
-      curc = V.orig_cell(k);
+      curc = orig(k);
       ++k;
       ++i;
     }
@@ -428,15 +517,52 @@ __device__ int regrid_track(double *prim, long long N, double *x, double *dx, do
     s_nnew = out;
     s_nseg = nseg;
     s_first = first_change;
+    s_nid = nid;
+  };
+  // the mark assumed of a merged cell: that of its two cells
+  auto mark_of = [&](int d) {
+    if (d >= 0) return bit_of(hpw, d);
+    double p[NQ];
+#pragma unroll
+    for (int s = 0; s < NQS; ++s) p[s < 3 ? s : s + 1] = S.nprim[s * 2 * S.N + noff + (-d - 1)];
+    p[UU2] = 0.;
+    return Hooks::regrid_marker(par, p);
+  };
+  for (bool eager = false;; eager = true) {
+    if (threadIdx.x == 0) walk(eager);
+    __syncthreads();
+    if (eager) break;
+    // ---- C. the merged cells, and whether their marks are as assumed
+    const int nid = s_nid;
+    bool differs = false;
+    for (int round = 1;; ++round) {
+      bool waits = false;
+      for (int id = threadIdx.x; id < nid; id += BS) {
+        const long long gid = noff + id;
+        if (S.nstate[gid] >= 0) continue;
+        const int v = S.nvic[gid];
+        const int vs = v < 0 ? S.nstate[noff + (-v - 1)] : 0;
+        if (vs < 0 || vs >= round) {  // its victim is formed in this round or later
+          waits = true;
+          continue;
+        }
+        const int c = S.ncur[gid];
+        if (form_merged<Cfg, Hooks>(ph, V, S, noff, id, c, v, S.nstate[gid] == kMergeLeft, par) != mark_of(c))
+          differs = true;
+        S.nstate[gid] = round;
+      }
+      if (!__syncthreads_or(waits)) break;
+    }
+    if (!__syncthreads_or(differs)) break;
   }
-  __syncthreads();
+  nsplit += walk_splits;
+  nmerge += walk_merges;
   const int nnew = s_nnew, nseg = s_nseg, first = s_first;
   if (first >= nnew && nnew == n) return n;  // nothing moved
 
-  // ---- C. expand the segments into the new track (positions >= first)
+  // ---- D. expand the segments into the new track (positions >= first)
   const int *seg_start = S.seg_start + 4 * off;
   const int *seg_src = S.seg_src + 4 * off;
-  const long long noff = 2 * off;
   for (int p = first + threadIdx.x; p < nnew; p += BS) {
     int lo = 0, hi = nseg - 1;  // last segment with start <= p
     while (lo < hi) {
@@ -478,7 +604,6 @@ __device__ int regrid_track(double *prim, long long N, double *x, double *dx, do
     dtl[gp] = S.tdtl[gp];
     if (p <= nnew - 2) xI[gp] = S.txI[gp];
   }
-  (void)outhp;
   __syncthreads();
   return nnew;
 }
