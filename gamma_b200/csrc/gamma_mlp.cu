@@ -97,6 +97,23 @@ __global__ void cons2prim_guess_kernel(const __grid_constant__ gb::Phys ph, cons
   }
 }
 
+// A launch that may start while the kernel before it in the stream still runs
+// (its wait_previous() holds it back).
+template <class... P, class... A>
+cudaError_t launch_chained(int grid, int threads, size_t smem, cudaStream_t s, void (*kernel)(P...), A... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
 long long gcd64(long long a, long long b) {
   while (b) {
     const long long t = a % b;
@@ -148,10 +165,13 @@ GAMMA_API int gamma_mlp_train(float *params, const float *x, const float *y, lon
   if (!params || !x || !y || !tc || n <= 0 || tc->epochs < 0 || tc->batch <= 0 || !(tc->lr > 0.f))
     return GAMMA_ERR_INVALID;
   cudaStream_t s = (cudaStream_t)stream;
-  float *ws = nullptr;  // grad, m, v, per-epoch loss
-  const size_t words = 3 * (size_t)NPARAM + (size_t)std::max(tc->epochs, 1);
-  if (cudaMalloc(&ws, words * sizeof(float)) != cudaSuccess) return GAMMA_ERR_CUDA;
-  float *grad = ws, *m = ws + NPARAM, *v = ws + 2 * NPARAM, *loss = ws + 3 * NPARAM;
+  const int nsm = sm_count();
+  // m, v, per-epoch loss (zeroed), then the blocks' partial sums
+  float *ws = nullptr;
+  const size_t words = 2 * (size_t)NPARAM + (size_t)std::max(tc->epochs, 1);
+  const size_t part_words = (size_t)nsm * gb::mlp::NPART;
+  if (cudaMalloc(&ws, (words + part_words) * sizeof(float)) != cudaSuccess) return GAMMA_ERR_CUDA;
+  float *m = ws, *v = ws + NPARAM, *loss = ws + 2 * NPARAM, *part = ws + words;
   int rc = GAMMA_OK;
   auto check = [&](cudaError_t e) {
     if (e != cudaSuccess && rc == GAMMA_OK) rc = GAMMA_ERR_CUDA;
@@ -159,7 +179,6 @@ GAMMA_API int gamma_mlp_train(float *params, const float *x, const float *y, lon
   check(cudaMemsetAsync(ws, 0, words * sizeof(float), s));
   const size_t smem = sizeof(gb::mlp::TrainSmem);
   check(cudaFuncSetAttribute(gb::mlp::grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int nsm = sm_count();
   const long long steps_per_epoch = (n + tc->batch - 1) / tc->batch;
   const long long total_steps = steps_per_epoch * tc->epochs;
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
@@ -181,18 +200,17 @@ GAMMA_API int gamma_mlp_train(float *params, const float *x, const float *y, lon
     for (long long b = 0; b < steps_per_epoch && rc == GAMMA_OK; ++b, ++step) {
       const long long start = b * tc->batch;
       const int cnt = (int)std::min<long long>(tc->batch, n - start);
-      check(cudaMemsetAsync(grad, 0, NPARAM * sizeof(float), s));
-      const int grid = std::max(1, std::min((cnt + gb::mlp::TB - 1) / gb::mlp::TB, nsm));
-      gb::mlp::grad_kernel<<<grid, gb::mlp::TB, smem, s>>>(params, x, y, n, mul, add, start, cnt, grad, loss + e);
-      check(cudaGetLastError());
+      const int grid = std::max(1, std::min((cnt + gb::mlp::TILE - 1) / gb::mlp::TILE, nsm));
+      check(launch_chained(grid, gb::mlp::TRAIN_THREADS, smem, s, gb::mlp::grad_kernel, params, x, y, n, mul, add,
+                           start, cnt, part, (float *)nullptr, (float *)nullptr));
       // cosine decay from lr to lr_final over all steps
       const double frac = total_steps > 1 ? (double)step / (double)(total_steps - 1) : 0.;
       const float lr = (float)(tc->lr_final + 0.5 * (tc->lr - tc->lr_final) * (1. + std::cos(M_PI * frac)));
       pb1 *= b1;
       pb2 *= b2;
-      gb::mlp::adam_kernel<<<(NPARAM + 255) / 256, 256, 0, s>>>(params, grad, m, v, lr, b1, b2, eps, 1.f - pb1,
-                                                                 1.f - pb2);
-      check(cudaGetLastError());
+      check(launch_chained((NPARAM + 1 + gb::mlp::ADAM_PARAMS - 1) / gb::mlp::ADAM_PARAMS, 256, 0, s,
+                           gb::mlp::adam_kernel, params, part, grid, m, v, lr, b1, b2, eps, 1.f - pb1, 1.f - pb2,
+                           loss + e));
     }
   }
   if (rc == GAMMA_OK && loss_per_epoch && tc->epochs > 0) {
@@ -217,9 +235,9 @@ GAMMA_API int gamma_mlp_loss_grad(const float *params, const float *x, const flo
     return GAMMA_ERR_CUDA;
   if (cudaMemsetAsync(grad, 0, NPARAM * sizeof(float), s) != cudaSuccess) return GAMMA_ERR_CUDA;
   if (loss && cudaMemsetAsync(loss, 0, sizeof(float), s) != cudaSuccess) return GAMMA_ERR_CUDA;
-  const int grid = std::max(1, std::min((n + gb::mlp::TB - 1) / gb::mlp::TB, sm_count()));
+  const int grid = std::max(1, std::min((n + gb::mlp::TILE - 1) / gb::mlp::TILE, sm_count()));
   // the samples in order (multiplier 1, offset 0), one mini-batch of n
-  gb::mlp::grad_kernel<<<grid, gb::mlp::TB, smem, s>>>(params, x, y, n, 1, 0, 0, n, grad, loss);
+  gb::mlp::grad_kernel<<<grid, gb::mlp::TRAIN_THREADS, smem, s>>>(params, x, y, n, 1, 0, 0, n, nullptr, grad, loss);
   return cudaGetLastError() == cudaSuccess ? GAMMA_OK : GAMMA_ERR_CUDA;
 }
 

@@ -39,10 +39,6 @@ constexpr int OFF_B3 = OFF_W3 + 2 * H;   // [2]
 constexpr int NPARAM = OFF_B3 + 2;       // 4546
 
 __device__ __forceinline__ float silu(float z) { return z / (1.f + __expf(-z)); }
-__device__ __forceinline__ float dsilu(float z) {
-  const float s = 1.f / (1.f + __expf(-z));
-  return s + z * s * (1.f - s);
-}
 
 // network inputs of a conserved state (D, tau, S_r): the ratios and the
 // thermal part in FP64 (the thermal part cancels), the logarithms in FP32
@@ -73,18 +69,14 @@ __device__ __forceinline__ double guess_pressure(double D, float y0) {
 // than it saves where poor warm starts are rare.
 constexpr double kGuessPolicy = 0.25;
 
-// FP32 forward of one sample; optional pre-activations and activations for
-// the backward pass (h1, h2 may be strided rows of shared memory)
-__device__ __forceinline__ void forward(const float *P, const float x[3], float out[2], float *z1 = nullptr,
-                                        float *h1 = nullptr, float *z2 = nullptr, float *h2 = nullptr) {
+// FP32 forward of one sample
+__device__ __forceinline__ void forward(const float *P, const float x[3], float out[2]) {
   float a1[H];
 #pragma unroll 4
   for (int o = 0; o < H; ++o) {
     const float z = P[OFF_B1 + o] + P[OFF_W1 + 3 * o] * x[0] + P[OFF_W1 + 3 * o + 1] * x[1] +
                     P[OFF_W1 + 3 * o + 2] * x[2];
-    if (z1) z1[o] = z;
     a1[o] = silu(z);
-    if (h1) h1[o] = a1[o];
   }
   float o0 = P[OFF_B3], o1 = P[OFF_B3 + 1];
 #pragma unroll 2
@@ -92,9 +84,7 @@ __device__ __forceinline__ void forward(const float *P, const float x[3], float 
     float z = P[OFF_B2 + o];
 #pragma unroll 16
     for (int i = 0; i < H; ++i) z += P[OFF_W2 + H * o + i] * a1[i];
-    if (z2) z2[o] = z;
     const float a = silu(z);
-    if (h2) h2[o] = a;
     o0 += P[OFF_W3 + o] * a;
     o1 += P[OFF_W3 + H + o] * a;
   }

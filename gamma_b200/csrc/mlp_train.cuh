@@ -75,135 +75,278 @@ __global__ void pairs_kernel(Phys ph, const double *prim, long long n, long long
 
 // ---------------------------------------------------------------------------
 // Training: loss = sum over a mini-batch and both outputs of (out - y)^2 / (2 m).
-// One thread per sample does the forward and backward pass; per-sample deltas
-// and activations are staged in shared memory (rows padded to H+1 floats), and
-// every thread then owns a fixed set of parameter gradients, which it sums over
-// the block's samples and adds to the global gradient once.  Sample j of the
-// mini-batch is pair (perm_mul * (start + j) + perm_add) mod n_total, a
-// bijection when gcd(perm_mul, n_total) = 1 (the host checks).
+// Sample j of the mini-batch is pair (perm_mul * (start + j) + perm_add) mod
+// n_total, a bijection when gcd(perm_mul, n_total) = 1 (the host checks).
+//
+// A block takes tiles of 64 samples through the forward and backward pass as
+// 64 x 64 x 64 products in FP32 from shared memory, 4 x 4 outputs per thread:
+// z2 = h1 W2^T, dL/dh1 = d2 W2 and dL/dW2 = d2^T h1.  Thread (tx, ty) of 16 x 16
+// holds rows ty + 16 i and columns tx + 16 j; every operand is kept with the
+// summed index last (so W2, h1 and d2 also transposed), rows padded to 68 floats:
+// a quarter warp's 16-byte loads of consecutive rows then touch all 32 banks.
+// The block's gradient goes to its own row of partial sums, which adam_kernel
+// adds up in a fixed order, so that training repeats bit for bit.
+// A mini-batch of 8,192 is 128 tiles, one per SM; the products are 0.8 MFLOP of
+// FMA per tile, ~3 us of the SM's FP32 rate, which bounds it (a sample per thread
+// with its activations in local memory took 128 us per mini-batch; now 11 us).
 
-constexpr int TB = 128;  // samples per chunk = threads per block
-constexpr int HP = H + 1;
+constexpr int TILE = 64;              // samples per tile
+constexpr int TRAIN_THREADS = 256;
+constexpr int LD = H + 4;             // padded row
+constexpr int NPART = NPARAM + 2;     // a block's partial sums: gradient, loss, padding
 
 struct TrainSmem {
-  float P[NPARAM];
-  float x[TB][3];
-  float d1[TB][HP];  // dL/dz1
-  float h1[TB][HP];
-  float d2[TB][HP];  // dL/dz2
-  float h2[TB][HP];
-  float d3[TB][2];   // dL/dout
+  float W2[H][LD], W2T[H][LD];        // [o][i] and [i][o]
+  float h1[TILE][LD], h1T[H][LD];     // [sample][unit] and [unit][sample]
+  float d2[TILE][LD], d2T[H][LD];     // dL/dz2, likewise
+  float x[TILE][4], y[TILE][2];
+  float W1[H][3], b1[H], b2[H], W3[2][H], b3[2];
+  float red[TRAIN_THREADS / 32][28][16];
+  float red3[TRAIN_THREADS / 32][3];
 };
 
-__global__ void __launch_bounds__(TB) grad_kernel(const float *Pg, const float *x, const float *y, long long n_total,
-                                                  long long perm_mul, long long perm_add, long long start, int m,
-                                                  float *grad, float *loss) {
+// The kernels of a training run follow one another in a stream, each launched
+// while the one before still runs (programmatic stream serialization): a kernel
+// lets the next one be launched as it starts, does what needs no results of the
+// one before, and waits for those here.
+__device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// acc[i][j] += sum_k A[ty + 16 i][k] B[tx + 16 j][k]
+__device__ __forceinline__ void tile_product(const float (*A)[LD], const float (*B)[LD], int tx, int ty,
+                                             float acc[4][4]) {
+#pragma unroll 4
+  for (int k = 0; k < H; k += 4) {
+    float4 a[4], b[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      a[i] = *reinterpret_cast<const float4 *>(&A[ty + 16 * i][k]);
+      b[i] = *reinterpret_cast<const float4 *>(&B[tx + 16 * i][k]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        acc[i][j] = fmaf(a[i].x, b[j].x, acc[i][j]);
+        acc[i][j] = fmaf(a[i].y, b[j].y, acc[i][j]);
+        acc[i][j] = fmaf(a[i].z, b[j].z, acc[i][j]);
+        acc[i][j] = fmaf(a[i].w, b[j].w, acc[i][j]);
+      }
+  }
+}
+
+// part != nullptr: the block's sums go to part[blockIdx.x][NPART]; else they are
+// added to grad and loss (zeroed by the caller).
+__global__ void __launch_bounds__(TRAIN_THREADS, 1)
+    grad_kernel(const float *Pg, const float *x, const float *y, long long n_total, long long perm_mul,
+                long long perm_add, long long start, int m, float *part, float *grad, float *loss) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TrainSmem &sm = *reinterpret_cast<TrainSmem *>(smem_raw);
-  const int tid = threadIdx.x;
-  for (int i = tid; i < NPARAM; i += TB) sm.P[i] = Pg[i];
-  __syncthreads();
-  constexpr int PER = (NPARAM + TB - 1) / TB;
-  float acc[PER];
-#pragma unroll
-  for (int j = 0; j < PER; ++j) acc[j] = 0.f;
-  const float inv_m = 1.f / (float)m;
-  float lsum = 0.f;
-
-  for (int base = blockIdx.x * TB; base < m; base += gridDim.x * TB) {
-    const int j = base + tid;
-    const bool valid = j < m;
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  launch_next();
+  // sample s of the block's tile at base: its pair (zeros past the mini-batch)
+  auto load_pair = [&](int base, int s) {
+    const int j = base + s;
     float xi[3] = {0.f, 0.f, 0.f}, yi[2] = {0.f, 0.f};
-    if (valid) {
+    if (j < m) {
       const long long k = (long long)(((unsigned long long)perm_mul * (unsigned long long)(start + j) +
                                        (unsigned long long)perm_add) % (unsigned long long)n_total);
-      xi[0] = x[3 * k];
-      xi[1] = x[3 * k + 1];
-      xi[2] = x[3 * k + 2];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) xi[c] = x[3 * k + c];
       yi[0] = y[2 * k];
       yi[1] = y[2 * k + 1];
     }
-    float z1[H], z2[H], out[2];
-    forward(sm.P, xi, out, z1, sm.h1[tid], z2, sm.h2[tid]);
-    float dout[2] = {0.f, 0.f};
-    if (valid) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) sm.x[s][c] = xi[c];
+    sm.y[s][0] = yi[0];
+    sm.y[s][1] = yi[1];
+  };
+  if (tid < TILE) load_pair(blockIdx.x * TILE, tid);
+  wait_previous();  // the parameters
+#pragma unroll
+  for (int k = tid; k < H * H; k += TRAIN_THREADS) {
+    const float w = Pg[OFF_W2 + k];
+    sm.W2[k / H][k % H] = w;
+    sm.W2T[k % H][k / H] = w;
+  }
+  for (int k = tid; k < 3 * H; k += TRAIN_THREADS) sm.W1[k / 3][k % 3] = Pg[OFF_W1 + k];
+  if (tid < H) {
+    sm.b1[tid] = Pg[OFF_B1 + tid];
+    sm.b2[tid] = Pg[OFF_B2 + tid];
+  }
+  if (tid < 2 * H) sm.W3[tid / H][tid % H] = Pg[OFF_W3 + tid];
+  if (tid < 2) sm.b3[tid] = Pg[OFF_B3 + tid];
+
+  // gradients of this thread: W2[ty + 16 i][tx + 16 j]; summed over its rows'
+  // samples, of unit tx + 16 j: b1, b2, W1[.][3], W3[2][.]; b3, and the loss
+  float gW2[4][4] = {}, gb1[4] = {}, gb2[4] = {}, gW1[4][3] = {}, gW3[2][4] = {}, gb3[2] = {0.f, 0.f}, lsum = 0.f;
+  const float inv_m = 1.f / (float)m;
+
+  for (int base = blockIdx.x * TILE; base < m; base += gridDim.x * TILE) {
+    if (base != blockIdx.x * TILE) {
+      __syncthreads();  // the tile before is done with
+      if (tid < TILE) load_pair(base, tid);
+    }
+    __syncthreads();
+    float ds1[4][4], z2[4][4];  // silu'(z1), z2
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int s = ty + 16 * i, o = tx + 16 * j;
+        const float z = sm.b1[o] + sm.W1[o][0] * sm.x[s][0] + sm.W1[o][1] * sm.x[s][1] + sm.W1[o][2] * sm.x[s][2];
+        const float sg = 1.f / (1.f + __expf(-z)), h = z * sg;
+        ds1[i][j] = sg + h * (1.f - sg);
+        sm.h1[s][o] = h;
+        sm.h1T[o][s] = h;
+        z2[i][j] = sm.b2[o];
+      }
+    __syncthreads();
+    tile_product(sm.h1, sm.W2, tx, ty, z2);
+    // output layer: sums over the 16 threads of a row
+    float out[4][2], sg2[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      out[i][0] = out[i][1] = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        sg2[i][j] = 1.f / (1.f + __expf(-z2[i][j]));
+        z2[i][j] *= sg2[i][j];  // h2 from here on
+        out[i][0] += sm.W3[0][tx + 16 * j] * z2[i][j];
+        out[i][1] += sm.W3[1][tx + 16 * j] * z2[i][j];
+      }
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+#pragma unroll
+        for (int d = 8; d > 0; d >>= 1) out[i][q] += __shfl_xor_sync(0xffffffffu, out[i][q], d);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int s = ty + 16 * i;
+      float dout[2];
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
-        const float e = out[q] - yi[q];
-        lsum += e * e;
+        const float e = base + s < m ? out[i][q] + sm.b3[q] - sm.y[s][q] : 0.f;
         dout[q] = e * inv_m;
+        if (tx == 0) {
+          lsum += e * e;
+          gb3[q] += dout[q];
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int o = tx + 16 * j;
+        const float h2 = z2[i][j];
+        gW3[0][j] += dout[0] * h2;
+        gW3[1][j] += dout[1] * h2;
+        // dL/dz2 = (W3^T dout) * silu'(z2)
+        const float d =
+            (sm.W3[0][o] * dout[0] + sm.W3[1][o] * dout[1]) * (sg2[i][j] + h2 * (1.f - sg2[i][j]));
+        gb2[j] += d;
+        sm.d2[s][o] = d;
+        sm.d2T[o][s] = d;
       }
     }
-    sm.d3[tid][0] = dout[0];
-    sm.d3[tid][1] = dout[1];
-    sm.x[tid][0] = xi[0];
-    sm.x[tid][1] = xi[1];
-    sm.x[tid][2] = xi[2];
-    // dL/dz2 = (W3^T dout) * silu'(z2)
-#pragma unroll 8
-    for (int i = 0; i < H; ++i) {
-      z2[i] = (sm.P[OFF_W3 + i] * dout[0] + sm.P[OFF_W3 + H + i] * dout[1]) * dsilu(z2[i]);
-      sm.d2[tid][i] = z2[i];
-    }
+    __syncthreads();
+    tile_product(sm.d2T, sm.h1T, tx, ty, gW2);
     // dL/dz1 = (W2^T dL/dz2) * silu'(z1)
-#pragma unroll 2
-    for (int i = 0; i < H; ++i) {
-      float s = 0.f;
-#pragma unroll 16
-      for (int o = 0; o < H; ++o) s += sm.P[OFF_W2 + H * o + i] * z2[o];
-      sm.d1[tid][i] = s * dsilu(z1[i]);
-    }
-    __syncthreads();
-    // parameter gradients owned by this thread
+    float d1[4][4] = {};
+    tile_product(sm.d2, sm.W2T, tx, ty, d1);
 #pragma unroll
-    for (int q = 0; q < PER; ++q) {
-      const int g = tid + q * TB;
-      if (g >= NPARAM) break;
-      float s = 0.f;
-      if (g < OFF_B1) {  // W1[o][i]
-        const int o = g / 3, i = g % 3;
-        for (int t = 0; t < TB; ++t) s += sm.d1[t][o] * sm.x[t][i];
-      } else if (g < OFF_W2) {
-        const int o = g - OFF_B1;
-        for (int t = 0; t < TB; ++t) s += sm.d1[t][o];
-      } else if (g < OFF_B2) {  // W2[o][i]
-        const int o = (g - OFF_W2) / H, i = (g - OFF_W2) % H;
-        for (int t = 0; t < TB; ++t) s += sm.d2[t][o] * sm.h1[t][i];
-      } else if (g < OFF_W3) {
-        const int o = g - OFF_B2;
-        for (int t = 0; t < TB; ++t) s += sm.d2[t][o];
-      } else if (g < OFF_B3) {  // W3[r][i]
-        const int r = (g - OFF_W3) / H, i = (g - OFF_W3) % H;
-        for (int t = 0; t < TB; ++t) s += sm.d3[t][r] * sm.h2[t][i];
-      } else {
-        const int r = g - OFF_B3;
-        for (int t = 0; t < TB; ++t) s += sm.d3[t][r];
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float d = d1[i][j] * ds1[i][j];
+        gb1[j] += d;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) gW1[j][c] += d * sm.x[ty + 16 * i][c];
       }
-      acc[q] += s;
-    }
-    __syncthreads();
+  }
+  // sums over the threads of a unit: two rows of a warp, then the warps
+  float v[28];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    v[j] = gb1[j];
+    v[4 + j] = gb2[j];
+    v[8 + j] = gW3[0][j];
+    v[12 + j] = gW3[1][j];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) v[16 + 3 * j + c] = gW1[j][c];
   }
 #pragma unroll
-  for (int q = 0; q < PER; ++q) {
-    const int g = tid + q * TB;
-    if (g < NPARAM) atomicAdd(&grad[g], acc[q]);
+  for (int k = 0; k < 28; ++k) {
+    v[k] += __shfl_xor_sync(0xffffffffu, v[k], 16);
+    if ((tid & 31) < 16) sm.red[tid >> 5][k][tx] = v[k];
   }
+  float w[3] = {gb3[0], gb3[1], lsum};
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-  if (loss && (tid & 31) == 0) atomicAdd(loss, 0.5f * lsum * inv_m);
+  for (int k = 0; k < 3; ++k) {
+    w[k] += __shfl_xor_sync(0xffffffffu, w[k], 16);
+    if ((tid & 31) == 0) sm.red3[tid >> 5][k] = w[k];
+  }
+  __syncthreads();
+  float *row = part ? part + (size_t)blockIdx.x * NPART : nullptr;
+  auto give = [&](int g, float s) {
+    if (row) row[g] = s;
+    else atomicAdd(&grad[g], s);
+  };
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) give(OFF_W2 + (ty + 16 * i) * H + tx + 16 * j, gW2[i][j]);
+  for (int k = tid; k < 28 * 16; k += TRAIN_THREADS) {
+    const int q = k / 16, t = k % 16;
+    float s = 0.f;
+#pragma unroll
+    for (int u = 0; u < TRAIN_THREADS / 32; ++u) s += sm.red[u][q][t];
+    int g;
+    if (q < 4) g = OFF_B1 + t + 16 * q;
+    else if (q < 8) g = OFF_B2 + t + 16 * (q - 4);
+    else if (q < 16) g = OFF_W3 + (q >= 12 ? H : 0) + t + 16 * (q & 3);
+    else g = OFF_W1 + 3 * (t + 16 * ((q - 16) / 3)) + (q - 16) % 3;
+    give(g, s);
+  }
+  if (tid < 3) {
+    float s = 0.f;
+#pragma unroll
+    for (int u = 0; u < TRAIN_THREADS / 32; ++u) s += sm.red3[u][tid];
+    if (tid < 2) give(OFF_B3 + tid, s);
+    else if (row) row[NPARAM] = 0.5f * s * inv_m;
+    else if (loss) atomicAdd(loss, 0.5f * s * inv_m);
+  }
 }
 
-// Adam (Kingma & Ba 2015) with bias corrections bc1 = 1 - b1^t, bc2 = 1 - b2^t
-__global__ void adam_kernel(float *P, const float *grad, float *m, float *v, float lr, float b1, float b2, float eps,
-                            float bc1, float bc2) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < NPARAM; i += gridDim.x * blockDim.x) {
-    const float g = grad[i];
-    const float mi = b1 * m[i] + (1.f - b1) * g;
-    const float vi = b2 * v[i] + (1.f - b2) * g * g;
-    m[i] = mi;
-    v[i] = vi;
-    P[i] -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
+// The gradient from nb blocks' partial sums, then Adam (Kingma & Ba 2015) with
+// bias corrections bc1 = 1 - b1^t, bc2 = 1 - b2^t; the mini-batch's loss is added
+// to *loss.  Eight threads per parameter, one of every eight blocks' sums each.
+constexpr int ADAM_PARAMS = 32;  // parameters per block of 256 threads
+__global__ void __launch_bounds__(256) adam_kernel(float *P, const float *part, int nb, float *m, float *v, float lr,
+                                                   float b1, float b2, float eps, float bc1, float bc2, float *loss) {
+  __shared__ float red[8][ADAM_PARAMS];
+  const int t = threadIdx.x & 31, k = threadIdx.x >> 5;
+  const int i = blockIdx.x * ADAM_PARAMS + t;  // NPARAM: the loss
+  launch_next();
+  wait_previous();
+  float s = 0.f;
+  if (i <= NPARAM) {
+#pragma unroll 8
+    for (int b = k; b < nb; b += 8) s += part[(size_t)b * NPART + i];
   }
+  red[k][t] = s;
+  __syncthreads();
+  if (k != 0 || i > NPARAM) return;
+  float g = red[0][t];
+#pragma unroll
+  for (int u = 1; u < 8; ++u) g += red[u][t];
+  if (i == NPARAM) {
+    *loss += g;
+    return;
+  }
+  const float mi = b1 * m[i] + (1.f - b1) * g;
+  const float vi = b2 * v[i] + (1.f - b2) * g * g;
+  m[i] = mi;
+  v[i] = vi;
+  P[i] -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
 }
 
 // FP32 forward of n samples (x [n][3] -> out [n][2])
