@@ -26,18 +26,25 @@ using namespace gb::d2;
 namespace {
 
 constexpr int kThreads = 256;
-// resident blocks per SM asked of the heavy per-cell passes.  The interface
-// passes are straight-line FP64 code (flat_ops.cuh) that overlaps its own
-// quotients and wants registers: at 512 tracks of 4,000 cells, per stage, the r
-// interfaces took 377 us at 2 blocks (3: 411, 4: 470, 1: 591) and the theta
-// interfaces 440 us at 2 (3: 538, 4: 602, 1: 615).  The transverse gradients
-// wait on loads and want warps: 484 us at 4 (3: 542, 2: 625, 1: 1078); so do the
-// theta gather and the cell update.
+// the interface passes' blocks: a small tile's barriers (r) and a small grid's
+// interfaces (theta) are spread finer (512 tracks: 266 -> 250 us per stage; 16
+// tracks of 400 cells: 17.8 -> 16.9 and 19.1 -> 17.4 us)
+constexpr int kIfaceThreads = 64;
+// resident blocks (of kThreads) per SM asked of the heavy per-cell passes.  The
+// interface passes and the cell update are straight-line FP64 code
+// (flat_ops.cuh) that overlaps its own quotients and wants registers: at 512
+// tracks of 4,000 cells, per stage, the r interfaces took 377 us at 2 blocks (3:
+// 411, 4: 470, 1: 591), the theta interfaces 440 us at 2 (3: 538, 4: 602, 1: 615)
+// and the update 307 us at 2 (4: 330).  The transverse gradients wait on loads
+// and want warps: 403 us at 4 (3: 444); so does the theta gather (174 us at 4).
 #ifndef GB2_MINB_MV
 #define GB2_MINB_MV 2
 #endif
 #ifndef GB2_MINB_TG
 #define GB2_MINB_TG 4
+#endif
+#ifndef GB2_TG_UNROLL
+#define GB2_TG_UNROLL 2
 #endif
 #ifndef GB2_MINB_F1
 #define GB2_MINB_F1 2
@@ -46,7 +53,7 @@ constexpr int kThreads = 256;
 #define GB2_MINB_GA 4
 #endif
 #ifndef GB2_MINB_UP
-#define GB2_MINB_UP 4
+#define GB2_MINB_UP 2
 #endif
 // waves of resident blocks in the grid of a per-cell pass
 #ifndef GB2_PASS_WAVES
@@ -168,32 +175,6 @@ __global__ void k_ghosts_copy(Grid2 G, int reset) {
 
 __global__ void k_ghost_cells(Grid2 G) { ghosts_cells(G, blockIdx.x, threadIdx.x, blockDim.x); }
 
-// Per-cell passes run over the live cells only: pref[j] = cells of tracks < j
-// (rebuilt after every ghost pass, when the track lengths are final for the
-// stage), and a fixed grid strides over [0, pref[NJ]).
-__global__ void k_prefix(Grid2 G) {
-  __shared__ int part[1024];
-  const int t = threadIdx.x, nt = blockDim.x;
-  const int chunk = (G.NJ + nt - 1) / nt;
-  const int j0 = t * chunk, j1 = min(G.NJ, j0 + chunk);
-  int sum = 0;
-  for (int j = j0; j < j1; ++j) sum += G.ntrack[j];
-  part[t] = sum;
-  __syncthreads();
-  for (int off = 1; off < nt; off <<= 1) {  // inclusive scan
-    const int v = t >= off ? part[t - off] : 0;
-    __syncthreads();
-    part[t] += v;
-    __syncthreads();
-  }
-  int run = part[t] - sum;
-  for (int j = j0; j < j1; ++j) {
-    G.pref[j] = run;
-    run += G.ntrack[j];
-  }
-  if (t == nt - 1) G.pref[G.NJ] = part[t];
-}
-
 // the last track j in [0, NJ-1] with pref[j] <= g (pref: a prefix over tracks)
 __device__ __forceinline__ int track_at(const int *pref, int NJ, long long g) {
   int lo = 0, hi = NJ - 1;
@@ -205,13 +186,56 @@ __device__ __forceinline__ int track_at(const int *pref, int NJ, long long g) {
   return lo;
 }
 
-// track_at of every 32nd element (live cell, theta interface), after the
-// prefix is formed: an element's track is then at most a few steps past its
-// group's (one step per track that starts inside the group)
-__global__ void k_group_tracks(const int *pref, int NJ, int *grp) {
-  const long long n = pref[NJ];
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; 32 * k < n; k += (long long)gridDim.x * blockDim.x)
-    grp[k] = track_at(pref, NJ, 32 * k);
+// Per-cell passes run over the live cells only: pref[j] = cells of tracks < j
+// (rebuilt after every ghost pass, when the track lengths are final for the
+// stage), and a fixed grid strides over [0, pref[NJ]); the theta interfaces'
+// passes likewise.  This kernel forms the prefix of count[0..ncount-1] (tracks
+// past ncount hold none) over the tracks, and track_at of every 32nd element: an
+// element's track is then at most a few steps past its group's (one step per
+// track that starts inside the group).  Each block scans the tracks itself, in
+// shared memory, so that one launch does both (a launch is 2 to 3 us of a small
+// grid's step, which has 16 per stage); block 0 keeps the prefix.  With more
+// tracks than fit there (SHARED false) the prefix is one launch of one block
+// (grp null) and the groups another (count null).  clear: a word per track to
+// zero.
+constexpr int kIndexThreads = 1024, kIndexTracks = 11000;
+template <bool SHARED>
+__global__ void __launch_bounds__(kIndexThreads) k_index(const int *count, int ncount, int NJ, int *pref, int *grp,
+                                                         int *clear) {
+  __shared__ int part[kIndexThreads];
+  __shared__ int copy[SHARED ? kIndexTracks + 1 : 1];
+  int *p = SHARED ? copy : pref;
+  const int t = threadIdx.x, nt = kIndexThreads;
+  if (count) {
+    const int chunk = (NJ + nt - 1) / nt;
+    const int j0 = min(NJ, t * chunk), j1 = min(NJ, j0 + chunk);
+    int sum = 0;
+    for (int j = j0; j < j1; ++j) sum += j < ncount ? count[j] : 0;
+    part[t] = sum;
+    __syncthreads();
+    for (int off = 1; off < nt; off <<= 1) {  // inclusive scan
+      const int v = t >= off ? part[t - off] : 0;
+      __syncthreads();
+      part[t] += v;
+      __syncthreads();
+    }
+    int run = part[t] - sum;
+    for (int j = j0; j < j1; ++j) {
+      p[j] = run;
+      if (SHARED && blockIdx.x == 0) pref[j] = run;
+      run += j < ncount ? count[j] : 0;
+      if (clear && blockIdx.x == 0) clear[j] = 0;
+    }
+    if (t == nt - 1) {
+      p[NJ] = part[t];
+      if (SHARED && blockIdx.x == 0) pref[NJ] = part[t];
+    }
+    __syncthreads();
+  }
+  if (!grp) return;
+  const long long n = p[NJ];
+  for (long long k = blockIdx.x * (long long)nt + t; 32 * k < n; k += (long long)gridDim.x * nt)
+    grp[k] = track_at(p, NJ, 32 * k);
 }
 
 // track_at(pref, NJ, g) from the group table
@@ -233,26 +257,46 @@ __device__ __forceinline__ void cell_at(const Grid2 &G, long long g, int *j, int
        g_ += (long long)gridDim.x * blockDim.x)                                                     \
     if (int j = 0, i = 0; cell_at((G), g_, &j, &i), true)
 
-__global__ void __launch_bounds__(kThreads, GB2_MINB_MV) k_mv(const __grid_constant__ Phys ph, const __grid_constant__ Params2 P, const __grid_constant__ Grid2 G) {
-  const long long it = *G.it;
-  FOR_LIVE_CELLS(G, j, i) mv_interface(ph, P, G, j, i, it);
+__global__ void __launch_bounds__(kIfaceThreads, GB2_MINB_MV * kThreads / kIfaceThreads)
+    k_mv(const __grid_constant__ Phys ph, const __grid_constant__ Params2 P, const __grid_constant__ Grid2 G) {
+  __shared__ MvTile<kIfaceThreads> sm;
+  const long long it = *G.it, n = G.pref[G.NJ];
+  constexpr int OWN = MvTile<kIfaceThreads>::OWN;
+  for (long long base = (long long)blockIdx.x * OWN; base < n; base += (long long)gridDim.x * OWN) {
+    const long long c = base - 1 + threadIdx.x;
+    const bool live = c >= 0 && c < n;
+    int j = 0, i = 0;
+    if (live) cell_at(G, c, &j, &i);
+    mv_tile(sm, ph, P, G, live, j, i, it);
+  }
 }
 
 __global__ void k_cellmv(Grid2 G) {
   FOR_LIVE_CELLS(G, j, i) cell_mv(G, j, i);
 }
 
-// foreign stale contributors: clear, then one thread per track appends
-__global__ void k_stale_clear(Grid2 G) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < G.NJ; t += gridDim.x * blockDim.x) G.stale_n[t] = 0;
-}
+// foreign stale contributors: one thread per track appends (k_index cleared them)
 __global__ void k_stale(Grid2 G) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j <= G.NJ - 2) stale_append(G, j);
 }
 
+// PARTS threads per cell, each a share of the slots: whole warps take one share
+// of 32 consecutive cells.
+template <int PARTS>
 __global__ void __launch_bounds__(kThreads, GB2_MINB_TG) k_tgrad(const __grid_constant__ Grid2 G) {
-  FOR_LIVE_CELLS(G, j, i) trans_grad(G, j, i);
+  __shared__ GeoTile<kThreads> sm;
+  constexpr int SLOTS = NQ / PARTS;
+  static_assert(NQ % PARTS == 0, "equal shares");
+  const long long n = G.pref[G.NJ], m = (n + 31) / 32 * 32 * PARTS;
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < m; e += (long long)gridDim.x * blockDim.x) {
+    const long long w = e >> 5, c = w / PARTS * 32 + (e & 31);
+    const int part = (int)(w % PARTS);
+    if (c >= n) continue;
+    int j, i;
+    cell_at(G, c, &j, &i);
+    trans_grad<GB2_TG_UNROLL>(sm, G, j, i, part * SLOTS, (part + 1) * SLOTS);
+  }
 }
 
 // The theta interfaces of track j (one block per track, j <= NJ-2), numbered
@@ -291,33 +335,9 @@ __global__ void k_if_scan(Grid2 G) {
   }
 }
 
-// if_pref: the interfaces of the tracks before j (track NJ-1 owns none)
-__global__ void k_if_pref(Grid2 G) {
-  __shared__ int part[1024];
-  const int t = threadIdx.x, nt = blockDim.x;
-  const int chunk = (G.NJ + nt - 1) / nt;
-  const int j0 = t * chunk, j1 = min(G.NJ, j0 + chunk);
-  auto tot = [&](int j) { return j <= G.NJ - 2 ? G.if_tot[j] : 0; };
-  int sum = 0;
-  for (int j = j0; j < j1; ++j) sum += tot(j);
-  part[t] = sum;
-  __syncthreads();
-  for (int off = 1; off < nt; off <<= 1) {
-    const int v = t >= off ? part[t - off] : 0;
-    __syncthreads();
-    part[t] += v;
-    __syncthreads();
-  }
-  int run = part[t] - sum;
-  for (int j = j0; j < j1; ++j) {
-    G.if_pref[j] = run;
-    run += tot(j);
-  }
-  if (t == nt - 1) G.if_pref[G.NJ] = part[t];
-}
-
 // every theta interface, one per thread (f1_if)
-__global__ void __launch_bounds__(kThreads, GB2_MINB_F1) k_f1if(const __grid_constant__ Phys ph, const __grid_constant__ Grid2 G) {
+__global__ void __launch_bounds__(kIfaceThreads, GB2_MINB_F1 * kThreads / kIfaceThreads)
+    k_f1if(const __grid_constant__ Phys ph, const __grid_constant__ Grid2 G) {
   const long long n = G.if_pref[G.NJ];
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x) {
@@ -326,8 +346,9 @@ __global__ void __launch_bounds__(kThreads, GB2_MINB_F1) k_f1if(const __grid_con
   }
 }
 
-__global__ void __launch_bounds__(kThreads, GB2_MINB_GA) k_f1gather(Phys ph, Grid2 G) {
-  FOR_LIVE_CELLS(G, j, i) f1_gather(ph, G, j, i);
+template <bool SPLIT_SIDES>
+__global__ void __launch_bounds__(kThreads, GB2_MINB_GA) k_f1gather(Grid2 G) {
+  FOR_LIVE_CELLS(G, j, i) f1_gather<SPLIT_SIDES>(G, j, i);
 }
 
 // detectShock and collect_dt: per-block minima, then one block
@@ -431,9 +452,11 @@ struct gamma_2d {
   int NJ = 0, cap = 0;
   long long NC = 0;
   cudaStream_t stream = nullptr;
-  cudaGraph_t graph = nullptr;
+  // a step's graph from either place of the two grad_f1 arrays (Grid2::gf1)
+  cudaGraph_t graph[2] = {};
+  cudaGraphExec_t exec[2] = {};
+  int side = 0;
   bool no_graphs = false;  // gamma_2d_use_graphs(ctx, 0): launch each step's kernels directly
-  cudaGraphExec_t exec = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   std::vector<void *> allocs;
   Grid2 G{};
@@ -444,7 +467,7 @@ struct gamma_2d {
   int nsm = 148;
   // grid of each per-cell pass (set_pass_grids)
   struct {
-    int mv, cellmv, tgrad, f1if, f1gather, dtpart, iface, update, update_guess, groups, if_groups;
+    int mv, cellmv, tgrad, tgrad_parts, f1if, f1gather, dtpart, iface, update, update_guess, groups, if_groups;
   } grid{};
   std::vector<double> tg;  // host copy of the per-track factors
   std::vector<double> theta, dtheta;  // of the active tracks, as given at creation
@@ -498,11 +521,12 @@ int blocks_of(long long n) { return (int)((n + kThreads - 1) / kThreads); }
 // wave, and no more blocks than the cell capacity needs.  The cells a thread
 // takes change with the grid, the arithmetic of each cell does not.
 template <class K>
-int pass_blocks(const gamma_2d *c, K kernel, size_t smem, int waves = kPassWaves) {
+int pass_blocks(const gamma_2d *c, K kernel, int threads, size_t smem = 0, int per_cell = 1) {
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, smem) != cudaSuccess || per_sm < 1)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess || per_sm < 1)
     per_sm = 1;
-  return (int)std::max(1LL, std::min<long long>(blocks_of(c->NC), (long long)c->nsm * per_sm * waves));
+  return (int)std::max(1LL, std::min<long long>((c->NC * per_cell + threads - 1) / threads,
+                                                (long long)c->nsm * per_sm * kPassWaves));
 }
 
 // entries of the theta interfaces' group table: the interfaces are at most
@@ -510,24 +534,47 @@ int pass_blocks(const gamma_2d *c, K kernel, size_t smem, int waves = kPassWaves
 long long if_groups(const gamma_2d *c) { return ((long long)(c->NJ - 1) * (2LL * c->cap + 64)) / 32 + 2; }
 
 void set_pass_grids(gamma_2d *c) {
-  c->grid.mv = pass_blocks(c, k_mv, 0);
-  c->grid.cellmv = pass_blocks(c, k_cellmv, 0);
-  c->grid.tgrad = pass_blocks(c, k_tgrad, 0);
-  c->grid.f1if = pass_blocks(c, k_f1if, 0);
-  c->grid.f1gather = pass_blocks(c, k_f1gather, 0);
+  c->grid.mv = pass_blocks(c, k_mv, kIfaceThreads);
+  c->grid.cellmv = pass_blocks(c, k_cellmv, kThreads);
+  // Threads per cell of the transverse gradients: a grid that leaves the SMs'
+  // threads idle shares a cell's slots out (each share forms the geometry).
+  // Measured us per stage with 1, 2, 5 (live cells): 6,400 24.8, 14.2, 8.6; 48,000
+  // 23.7, 17.5, 20.2; 60,000 25.5, 19.0, 24.0; 200,000 53.7, 52.5, 68; 2.05 M 407, 493,
+  // 632.
+  c->grid.tgrad_parts = c->NC <= c->nsm * 128LL ? 5 : (c->NC <= c->nsm * 1024LL ? 2 : 1);
+  c->grid.tgrad = c->grid.tgrad_parts == 5   ? pass_blocks(c, k_tgrad<5>, kThreads, 0, 5)
+                  : c->grid.tgrad_parts == 2 ? pass_blocks(c, k_tgrad<2>, kThreads, 0, 2)
+                                             : pass_blocks(c, k_tgrad<1>, kThreads);
+  c->grid.f1if = pass_blocks(c, k_f1if, kIfaceThreads);
+  c->grid.f1gather = pass_blocks(c, k_f1gather<false>, kThreads);
   // one wave: every block ends in a block reduction, and k_dtfinal reads
   // one partial per block
-  c->grid.dtpart = pass_blocks(c, k_dtpart, 0, 1);
-  c->grid.iface = pass_blocks(c, k_iface, 0);
-  c->grid.update = pass_blocks(c, k_update<false>, 0);
-  c->grid.update_guess = pass_blocks(c, k_update<true>, sizeof(mlp::InferSmem));
-  c->grid.groups = std::max(1, std::min(blocks_of(c->NC / 32 + 1), c->nsm * 8));
-  c->grid.if_groups = std::max(1, std::min(blocks_of(if_groups(c)), c->nsm * 8));
+  c->grid.dtpart = std::min(blocks_of(c->NC), c->nsm * 8);
+  c->grid.iface = pass_blocks(c, k_iface, kThreads);
+  c->grid.update = pass_blocks(c, k_update<false>, kThreads);
+  c->grid.update_guess = pass_blocks(c, k_update<true>, kThreads, sizeof(mlp::InferSmem));
+  c->grid.groups = (int)std::max(1LL, std::min<long long>((c->NC / 32 + 1) / kIndexThreads, c->nsm));
+  c->grid.if_groups = (int)std::max(1LL, std::min<long long>(if_groups(c) / kIndexThreads, c->nsm));
 }
 
 int ghost_blocks(const gamma_2d *c, bool reset) {
   const long long n = (reset ? c->NC : 0) + 2LL * c->cfg.ngst * c->cap;
   return (int)std::max(1LL, std::min((n + kThreads - 1) / kThreads, 148LL * 8));
+}
+
+void index_tracks(gamma_2d *c, const int *count, int ncount, int *pref, int *grp, int *clear, int blocks) {
+  if (c->NJ <= kIndexTracks) {
+    k_index<true><<<blocks, kIndexThreads, 0, c->stream>>>(count, ncount, c->NJ, pref, grp, clear);
+  } else {
+    k_index<false><<<1, kIndexThreads, 0, c->stream>>>(count, ncount, c->NJ, pref, nullptr, clear);
+    k_index<false><<<blocks, kIndexThreads, 0, c->stream>>>(nullptr, 0, c->NJ, pref, grp, nullptr);
+  }
+}
+
+// This stage's grad_f1 becomes the persistent one.
+void swap_sides(gamma_2d *c) {
+  std::swap(c->G.gf1, c->G.gf1n);
+  c->side ^= 1;
 }
 
 // One step's launches on the context's stream.  upto > 0 stops after the
@@ -536,7 +583,7 @@ int ghost_blocks(const gamma_2d *c, bool reset) {
 int enqueue_step_until(gamma_2d *c, int upto) {
   const Phys ph = phys_of(c->cfg);
   const Params2 P = params_of(c->par);
-  const Grid2 &G = c->G;
+  Grid2 &G = c->G;
   cudaStream_t s = c->stream;
   if (c->guess) k_guess_policy2<<<1, 1, 0, s>>>(c->d_policy, c->d_stats);
   k_regrid_check<<<1, kThreads, 0, s>>>(P, G, c->d_flags, c->cfg.ngst);
@@ -549,22 +596,22 @@ int enqueue_step_until(gamma_2d *c, int upto) {
   for (int stage = 1; stage <= nstage; ++stage) {
     k_ghosts_copy<<<ghost_blocks(c, stage == 1), kThreads, 0, s>>>(G, stage == 1);
     k_ghost_cells<<<c->NJ, 32, 0, s>>>(G);
-    k_prefix<<<1, 1024, 0, s>>>(G);
-    k_group_tracks<<<c->grid.groups, kThreads, 0, s>>>(G.pref, G.NJ, G.gtrk);
-    k_mv<<<c->grid.mv, kThreads, 0, s>>>(ph, P, G);
+    index_tracks(c, G.ntrack, G.NJ, G.pref, G.gtrk, G.stale_n, c->grid.groups);
+    k_mv<<<c->grid.mv, kIfaceThreads, 0, s>>>(ph, P, G);
     k_cellmv<<<c->grid.cellmv, kThreads, 0, s>>>(G);
-    k_stale_clear<<<(c->NJ + 255) / 256, 256, 0, s>>>(G);
     k_stale<<<(c->NJ + 127) / 128, 128, 0, s>>>(G);
-    k_tgrad<<<c->grid.tgrad, kThreads, 0, s>>>(G);
+    if (c->grid.tgrad_parts == 5) k_tgrad<5><<<c->grid.tgrad, kThreads, 0, s>>>(G);
+    else if (c->grid.tgrad_parts == 2) k_tgrad<2><<<c->grid.tgrad, kThreads, 0, s>>>(G);
+    else k_tgrad<1><<<c->grid.tgrad, kThreads, 0, s>>>(G);
     k_if_scan<<<c->NJ - 1, kThreads, 0, s>>>(G);
-    k_if_pref<<<1, 1024, 0, s>>>(G);
-    k_group_tracks<<<c->grid.if_groups, kThreads, 0, s>>>(G.if_pref, G.NJ, G.iftrk);
-    k_f1if<<<c->grid.f1if, kThreads, 0, s>>>(ph, G);
-    k_f1gather<<<c->grid.f1gather, kThreads, 0, s>>>(ph, G);
+    index_tracks(c, G.if_tot, G.NJ - 1, G.if_pref, G.iftrk, nullptr, c->grid.if_groups);  // track NJ-1 owns none
+    k_f1if<<<c->grid.f1if, kIfaceThreads, 0, s>>>(ph, G);
     if (stage == upto) {
+      k_f1gather<true><<<c->grid.f1gather, kThreads, 0, s>>>(G);
       G2_CUDA(c, cudaGetLastError());
       return GAMMA_OK;
     }
+    k_f1gather<false><<<c->grid.f1gather, kThreads, 0, s>>>(G);
     if (stage == 1) {
       k_dtpart<<<c->grid.dtpart, kThreads, 0, s>>>(G);
       k_dtfinal<<<1, kThreads, 0, s>>>(G, c->grid.dtpart, c->cfg.cfl);
@@ -574,6 +621,7 @@ int enqueue_step_until(gamma_2d *c, int upto) {
     k_update<false><<<c->grid.update, kThreads, 0, s>>>(ph, P, G, stage, c->d_stats, nullptr, pol);
     if (c->guess)
       k_update<true><<<c->grid.update_guess, kThreads, sizeof(mlp::InferSmem), s>>>(ph, P, G, stage, c->d_stats, c->guess, pol);
+    swap_sides(c);
   }
   k_advance<<<1, 32, 0, s>>>(G, c->d_stats);
   G2_CUDA(c, cudaGetLastError());
@@ -734,11 +782,11 @@ GAMMA_API int gamma_2d_layout(const gamma_2d_t *ctx, int *ntracks, int *cap) {
 
 // the graph holds the launch arguments: capture again on the next step
 static void drop_graph(gamma_2d *ctx) {
-  if (ctx->exec) {
-    cudaGraphExecDestroy(ctx->exec);
-    cudaGraphDestroy(ctx->graph);
-    ctx->exec = nullptr;
-    ctx->graph = nullptr;
+  for (int k = 0; k < 2; ++k) {
+    if (ctx->exec[k]) cudaGraphExecDestroy(ctx->exec[k]);
+    if (ctx->graph[k]) cudaGraphDestroy(ctx->graph[k]);
+    ctx->exec[k] = nullptr;
+    ctx->graph[k] = nullptr;
   }
 }
 
@@ -837,19 +885,30 @@ GAMMA_API int gamma_2d_step(gamma_2d_t *ctx, int nsteps, gamma_step_stats_t *sta
       const int rc = enqueue_step(c);
       if (rc != GAMMA_OK) return rc;
     }
-  } else if (!c->exec && nsteps > 0) {
-    G2_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    const int rc = enqueue_step(c);
-    cudaGraph_t g = nullptr;
-    const cudaError_t e = cudaStreamEndCapture(c->stream, &g);
-    if (rc != GAMMA_OK) return rc;
-    if (e != cudaSuccess) return fail(c, e, "cudaStreamEndCapture");
-    c->graph = g;
-    G2_CUDA(c, cudaGraphInstantiate(&c->exec, c->graph, 0));
-  }
-  if (!c->no_graphs) {
+  } else {
+    // a step has an odd number of stages: steps alternate between the two sides
+    for (int k = 0; k < std::min(nsteps, 2); ++k) {
+      const int side = c->side ^ k;
+      if (c->exec[side]) continue;
+      if (k) swap_sides(c);
+      G2_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+      const int rc = enqueue_step(c);
+      cudaGraph_t g = nullptr;
+      const cudaError_t e = cudaStreamEndCapture(c->stream, &g);
+      while (c->side != (side ^ k)) swap_sides(c);  // as before the capture
+      if (rc != GAMMA_OK) {
+        if (g) cudaGraphDestroy(g);
+        return rc;
+      }
+      if (e != cudaSuccess) return fail(c, e, "cudaStreamEndCapture");
+      c->graph[side] = g;
+      G2_CUDA(c, cudaGraphInstantiate(&c->exec[side], g, 0));
+    }
     G2_CUDA(c, cudaEventRecord(c->ev0, c->stream));
-    for (int k = 0; k < nsteps; ++k) G2_CUDA(c, cudaGraphLaunch(c->exec, c->stream));
+    for (int k = 0; k < nsteps; ++k) {
+      G2_CUDA(c, cudaGraphLaunch(c->exec[c->side], c->stream));
+      swap_sides(c);
+    }
   }
   G2_CUDA(c, cudaEventRecord(c->ev1, c->stream));
   if (stats) {
@@ -1044,8 +1103,7 @@ GAMMA_API int gamma_2d_load(gamma_2d_t *ctx, const char *path) {
 GAMMA_API void gamma_2d_destroy(gamma_2d_t *ctx) {
   if (!ctx) return;
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-  if (ctx->exec) cudaGraphExecDestroy(ctx->exec);
-  if (ctx->graph) cudaGraphDestroy(ctx->graph);
+  drop_graph(ctx);
   for (void *p : ctx->allocs) cudaFree(p);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);

@@ -927,10 +927,21 @@ GB_HD bool compute_Sd(Ar &ar, const Phys &ph, const FState<Cfg> &S1, const FStat
   double Da = ar.quo(4. * g * p1 * ((g - 1) * p2 + p1), ar.by(gm12 * (p1 - p2) * (p1 - p2)));
   double Db = ar.quo(h2 * (p2 - p1), by_rho2) - h2 * h2;
   double Dd = 1. - Da * Db;
+  // the root of a negative number is NaN, and so is then all that follows
+  if (!(Dd >= 0.)) {
+    *Sd = nan("");
+    *pspec = P_SPEC;
+    return true;
+  }
   double h3 = ar.quo((ar.root(Dd) - 1) * gm1 * (p1 - p2), ar.by(2 * (gm1 * p2 + p1)));
   double J232a = ar.quo(-g, bgm1) * (p1 - p2);
   double J232b = ar.quo(h3 * (h3 - 1), by_p1) - ar.quo(h2 * (h2 - 1), ar.by(p2));
   double J232 = ar.quo(J232a, ar.by(J232b));
+  if (!(J232 >= 0.)) {
+    *Sd = nan("");
+    *pspec = P_SPEC;
+    return true;
+  }
   double J23 = ar.root(J232);
   double Vsa = rho22 * lfac22 * vx2 + fabs(J23) * ar.root(J232 + rho22 * lfac22 * (1. - vx22));
   double Vsb = rho22 * lfac22 + J232;

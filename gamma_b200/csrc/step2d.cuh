@@ -38,6 +38,9 @@
 namespace gb {
 namespace d2 {
 
+#ifndef GB2_TG_KGEO
+#define GB2_TG_KGEO 6
+#endif
 constexpr int KMAX_STALE = 8;  // foreign stale contributors per target track
 // a theta interface's results: flux[NQ], forward Sd, reverse Sd, flags (1: the
 // forward test reached the spectral index, 2: the reverse one)
@@ -62,10 +65,12 @@ struct Grid2 {
   double *x, *dx;     // r and dr (Cell::G)
   double *dtl, *sd, *pspec;
   uint8_t *shocked;
-  double *gmv, *gf1, *gf1n;  // [NQ][NC] grad_mv, grad_f1 (persistent), grad_f1 of this stage
+  // [NQ][NC] grad_mv, grad_f1 (persistent), grad_f1 of this stage; the last two
+  // change places at the end of a stage (every live cell has a new one)
+  double *gmv, *gf1, *gf1n;
   int *nbr;                  // [4][NC]: first id and count towards track j-1, then j+1
   double *cons0, *dV0;       // [NQ][NC], [NC]: S0.cons and G0.dV (copyState0)
-  double *f1lo, *f1hi;       // [NQ][NC]: flux[0][F1], flux[1][F1]
+  double *f1lo, *f1hi;       // [NQ][NC]: flux[0][F1] - flux[1][F1]; for diagnostics each of them
   // interfaces
   double *xI, *xI0, *xIm;    // position, step-start position, position after the stage's move
   double *v, *lL, *lR;
@@ -231,41 +236,13 @@ GB_HD void cell_state(Ar &ar, const Phys &ph, const Grid2 &G, long long g, int d
   fill(ar, ph, S, dim, G.x[g]);
 }
 
-// The interface with the operators Ar.  False (the interface's own outputs not
-// written) where an operand left their range.
+// The interface between its two states.  False (nothing written) where an
+// operand left the range of Ar.
 template <class Ar>
-GB_HD bool mv_interface_ops(const Phys &ph, const Params2 &P, const Grid2 &G, int j, int i, long long it) {
-  Ar ar;
+GB_HD bool mv_solve(Ar &ar, const Phys &ph, const Params2 &P, const Grid2 &G, int j, int i, long long it, double xI,
+                    const St &L, const St &R) {
   const int n = G.ntrack[j];
-  const long long o = (long long)j * G.cap, g = o + i;
-  const double xI = G.xI[g];
-  St L, R;
-  if (i == 0 || i == n - 2) {
-    cell_state(ar, ph, G, g, MV, L);
-    cell_state(ar, ph, G, g + 1, MV, R);
-  } else {
-    const double cLL = cen_r(ar, G.x[g - 1], G.dx[g - 1]), cL = cen_r(ar, G.x[g], G.dx[g]);
-    const double cR = cen_r(ar, G.x[g + 1], G.dx[g + 1]), cRR = cen_r(ar, G.x[g + 2], G.dx[g + 2]);
-    const auto dL = ar.by(cL - cLL), dN = ar.by(cR - cL), dR = ar.by(cRR - cR);
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-      const double qLL = G.prim[q * G.NC + g - 1], qL = G.prim[q * G.NC + g];
-      const double qR = G.prim[q * G.NC + g + 1], qRR = G.prim[q * G.NC + g + 2];
-      double gL = ar.quo0(qL - qLL, dL);
-      const double gN = ar.quo0(qR - qL, dN);
-      double gR = ar.quo0(qRR - qR, dR);
-      gL = minmod(gL, gN);
-      gR = minmod(gR, gN);
-      // grad_mv stored in the cells; cell i from its right interface, except
-      // the last reconstructed cell n-2, which only has its left one
-      G.gmv[q * G.NC + g] = gL;
-      if (i == n - 3) G.gmv[q * G.NC + g + 1] = gR;
-      L.prim[q] = qL + gL * (xI - cL);
-      R.prim[q] = qR + gR * (xI - cR);
-    }
-    fill(ar, ph, L, MV, xI);
-    fill(ar, ph, R, MV, xI);
-  }
+  const long long g = (long long)j * G.cap + i;
   const Waves w = compute_lambda(ar, ph, L, R, MV, xI);
   double v = ph.vi * w.lS;
   if (i >= n - 1 - G.ngst) v = outer_velocity(G, P, it);
@@ -286,13 +263,114 @@ GB_HD bool mv_interface_ops(const Phys &ph, const Params2 &P, const Grid2 &G, in
   G.sd[g] = fmax(G.sd[g], Sd);
   return true;
 }
+
+// The whole interface with the plain operators, from the cells in memory.
 GB_HD_OUTLINE void mv_interface_plain(const Phys &ph, const Params2 &P, const Grid2 &G, int j, int i, long long it) {
-  mv_interface_ops<PlainOps>(ph, P, G, j, i, it);
+  PlainOps ar;
+  const int n = G.ntrack[j];
+  const long long g = (long long)j * G.cap + i;
+  const double xI = G.xI[g];
+  St L, R;
+  if (i == 0 || i == n - 2) {
+    cell_state(ar, ph, G, g, MV, L);
+    cell_state(ar, ph, G, g + 1, MV, R);
+  } else {
+    const double cLL = cen_r(ar, G.x[g - 1], G.dx[g - 1]), cL = cen_r(ar, G.x[g], G.dx[g]);
+    const double cR = cen_r(ar, G.x[g + 1], G.dx[g + 1]), cRR = cen_r(ar, G.x[g + 2], G.dx[g + 2]);
+    for (int q = 0; q < NQ; ++q) {
+      const double qLL = G.prim[q * G.NC + g - 1], qL = G.prim[q * G.NC + g];
+      const double qR = G.prim[q * G.NC + g + 1], qRR = G.prim[q * G.NC + g + 2];
+      double gL = qdiv(qL - qLL, cL - cLL);
+      const double gN = qdiv(qR - qL, cR - cL);
+      double gR = qdiv(qRR - qR, cRR - cR);
+      gL = minmod(gL, gN);
+      gR = minmod(gR, gN);
+      G.gmv[q * G.NC + g] = gL;
+      if (i == n - 3) G.gmv[q * G.NC + g + 1] = gR;
+      L.prim[q] = qL + gL * (xI - cL);
+      R.prim[q] = qR + gR * (xI - cR);
+    }
+    fill(ar, ph, L, MV, xI);
+    fill(ar, ph, R, MV, xI);
+  }
+  mv_solve(ar, ph, P, G, j, i, it, xI, L, R);
 }
-GB_HD void mv_interface(const Phys &ph, const Params2 &P, const Grid2 &G, int j, int i, long long it) {
-  if (i > G.ntrack[j] - 2) return;
-  if (!mv_interface_ops<FlatOps>(ph, P, G, j, i, it)) mv_interface_plain(ph, P, G, j, i, it);
+
+#ifdef __CUDACC__
+// The r interfaces of a block's tile of consecutive live cells: BS slots, slot t
+// of thread t, which is flat live cell base - 1 + t; slots 1 .. BS-3 own their
+// right interface.  The tile's cells are read once into shared memory, all of a
+// thread's loads at once, and each pair of neighbours' gradient is divided once
+// and used by the three interfaces around it.
+template <int BS>
+struct MvTile {
+  static constexpr int OWN = BS - 3;
+  double p[NQ][BS], cen[BS], gp[NQ][BS];  // primitives, centroid, gradient to the next slot
+};
+
+// live: thread t's slot holds cell (j, i)
+template <int BS>
+__device__ __forceinline__ void mv_tile(MvTile<BS> &sm, const Phys &ph, const Params2 &P, const Grid2 &G, bool live,
+                                        int j, int i, long long it) {
+  const int t = threadIdx.x;
+  const int n = live ? G.ntrack[j] : 0;
+  const long long g = (long long)j * G.cap + i;
+  double x = 0.;
+  if (live) {
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) sm.p[q][t] = G.prim[q * G.NC + g];
+    x = G.x[g];
+    const double dx = G.dx[g];
+    FlatOps ar;
+    double cen = cen_r(ar, x, dx);
+    if (ar.bad()) cen = cen_r(x, dx);
+    sm.cen[t] = cen;
+  }
+  __syncthreads();
+  const bool pair = live && t < BS - 1 && i <= n - 2;  // slot t+1 holds cell (j, i+1)
+  if (pair) {
+    FlatOps ar;
+    const auto by = ar.by(sm.cen[t + 1] - sm.cen[t]);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) sm.gp[q][t] = ar.quo0(sm.p[q][t + 1] - sm.p[q][t], by);
+    if (ar.bad())
+      for (int q = 0; q < NQ; ++q) sm.gp[q][t] = qdiv(sm.p[q][t + 1] - sm.p[q][t], sm.cen[t + 1] - sm.cen[t]);
+  }
+  __syncthreads();
+  if (pair && t >= 1 && t <= BS - 3) {
+    FlatOps ar;
+    const double xI = G.xI[g];
+    St L, R;
+    if (i == 0 || i == n - 2) {  // piecewise constant, each at its own centre
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        L.prim[q] = sm.p[q][t];
+        R.prim[q] = sm.p[q][t + 1];
+      }
+      fill(ar, ph, L, MV, x);
+      fill(ar, ph, R, MV, G.x[g + 1]);
+    } else {
+      const double dL = xI - sm.cen[t], dR = xI - sm.cen[t + 1];
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        const double gN = sm.gp[q][t];
+        const double gL = minmod(sm.gp[q][t - 1], gN);
+        const double gR = minmod(sm.gp[q][t + 1], gN);
+        // grad_mv stored in the cells; cell i from its right interface, except
+        // the last reconstructed cell n-2, which only has its left one
+        G.gmv[q * G.NC + g] = gL;
+        if (i == n - 3) G.gmv[q * G.NC + g + 1] = gR;
+        L.prim[q] = sm.p[q][t] + gL * dL;
+        R.prim[q] = sm.p[q][t + 1] + gR * dR;
+      }
+      fill(ar, ph, L, MV, xI);
+      fill(ar, ph, R, MV, xI);
+    }
+    if (!mv_solve(ar, ph, P, G, j, i, it, xI, L, R)) mv_interface_plain(ph, P, G, j, i, it);
+  }
+  __syncthreads();  // the next tile overwrites this one's slots
 }
+#endif  // __CUDACC__
 
 // ---------------------------------------------------------------------------
 // Per cell after the interfaces: update_dt(MV) (cell.cpp:47-74) and the
@@ -407,16 +485,23 @@ GB_HD double neighbour_grad(Ar &ar, const Grid2 &G, int q, long long gn, const N
 // neighbour's gradient in the reference's order (an order-dependent chain:
 // minmod(x, x) = 0).  Every slot's chain uses its own gradients only, so the
 // slots run one after another over geometry formed once: the first KGEO
-// neighbours' geometry and one slot's gradients stay in registers, and
-// neighbours past KGEO recompute theirs for each slot.  Per slot the
-// operations and their order are those of the reference's loops.
-constexpr int KGEO = 4;
+// neighbours' is kept in shared memory (a column per thread; neighbours past
+// KGEO, which are rare, recompute theirs for each slot), one slot's first KKEEP
+// gradients in registers.  Per slot the operations and their order are those of
+// the reference's loops.
+constexpr int KGEO = GB2_TG_KGEO, KKEEP = 4;
+
+template <int BS>
+struct GeoTile {
+  double g[KGEO][3][BS];
+};
 
 // False where an operand left the range of Ar (grad_f1 of the cell is then to
 // be formed again).
-template <class Ar>
-GB_HD bool trans_grad_ops(const Grid2 &G, int j, int i) {
+template <class Ar, int UNROLL, int BS>
+__device__ __forceinline__ bool trans_grad_ops(GeoTile<BS> &sm, const Grid2 &G, int j, int i, int q0, int q1) {
   Ar ar;
+  const int t = threadIdx.x;
   const long long g0 = (long long)j * G.cap + i;
   const double cr0 = cen_r(ar, G.x[g0], G.dx[g0]);
   const TrackGeo t0 = tgeo(G, j);
@@ -426,66 +511,72 @@ GB_HD bool trans_grad_ops(const Grid2 &G, int j, int i) {
   const int nn = c0 + c1;
   // neighbour kn: the lower list's cells, then the upper list's; the theta of
   // the interface is th - dth/2 below and th (unmoved) above
-#define TG_NBR(kn) ((kn) < c0 ? (long long)f0 + (kn) : (long long)f1 + ((kn) - c0))
-#define TG_S(kn) ((kn) < c0 ? t0.s_lo : t0.s_mid)
-#define TG_D(kn) ((kn) < c0 ? d0 : d1)
+  auto nbr = [&](int kn) { return kn < c0 ? f0 + kn : f1 + (kn - c0); };
   // theta distances to the two lists' tracks (1 where a list is empty)
   const auto d0 = ar.by(c0 > 0 ? tgeo(G, track_of(G, f0)).cen_t - ct0 : 1.);
   const auto d1 = ar.by(c1 > 0 ? tgeo(G, track_of(G, f1)).cen_t - ct0 : 1.);
-  NbrGeo geo[KGEO];
+  auto make = [&](int kn) { return neighbour_geo(ar, G, g0, nbr(kn), cr0, kn < c0 ? t0.s_lo : t0.s_mid); };
+  auto geo = [&](int kn) {
+    return kn < KGEO ? NbrGeo{sm.g[kn][0][t], sm.g[kn][1][t], sm.g[kn][2][t]} : make(kn);
+  };
   double dAtot = 0.;
-#pragma unroll
-  for (int kn = 0; kn < KGEO; ++kn)
-    if (kn < nn) {
-      geo[kn] = neighbour_geo(ar, G, g0, TG_NBR(kn), cr0, TG_S(kn));
-      dAtot += geo[kn].dA;
+#pragma unroll 2
+  for (int kn = 0; kn < nn; ++kn) {
+    const NbrGeo e = make(kn);
+    if (kn < KGEO) {
+      sm.g[kn][0][t] = e.dxmL;
+      sm.g[kn][1][t] = e.dxmR;
+      sm.g[kn][2][t] = e.dA;
     }
-  for (int kn = KGEO; kn < nn; ++kn) dAtot += neighbour_geo(ar, G, g0, TG_NBR(kn), cr0, TG_S(kn)).dA;
-  if (nn == 0) {  // no neighbours: the reference's 0 / 0
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) G.gf1n[q * G.NC + g0] = nan("");
+    dAtot += e.dA;
+  }
+  // No overlap (the copied lists of a track's end cells): the reference's
+  // average is 0 / 0 (areas are not negative), and minmod of a NaN and anything
+  // is 0.  The plain operators divide.
+  if (Ar::FLAT && dAtot == 0.) {
+    for (int q = q0; q < q1; ++q) G.gf1n[q * G.NC + g0] = nn == 0 ? nan("") : 0.;
     return true;
   }
   const auto by_tot = ar.by(dAtot);
-#pragma unroll 1
-  for (int q = 0; q < NQ; ++q) {
+#pragma unroll UNROLL
+  for (int q = q0; q < q1; ++q) {
     const double p0 = G.prim[q * G.NC + g0], m0 = G.gmv[q * G.NC + g0];
-    double avg = 0., kept[KGEO];
+    double avg = 0., kept[KKEEP];
+    auto grad = [&](int kn, const NbrGeo &e) { return neighbour_grad(ar, G, q, nbr(kn), e, kn < c0 ? d0 : d1, p0, m0); };
 #pragma unroll
-    for (int kn = 0; kn < KGEO; ++kn)
+    for (int kn = 0; kn < KKEEP; ++kn)
       if (kn < nn) {
-        kept[kn] = neighbour_grad(ar, G, q, TG_NBR(kn), geo[kn], TG_D(kn), p0, m0);
-        avg += kept[kn] * geo[kn].dA;
+        const NbrGeo e = geo(kn);
+        kept[kn] = grad(kn, e);
+        avg += kept[kn] * e.dA;
       }
-    for (int kn = KGEO; kn < nn; ++kn) {
-      const NbrGeo e = neighbour_geo(ar, G, g0, TG_NBR(kn), cr0, TG_S(kn));
-      avg += neighbour_grad(ar, G, q, TG_NBR(kn), e, TG_D(kn), p0, m0) * e.dA;
+    for (int kn = KKEEP; kn < nn; ++kn) {
+      const NbrGeo e = geo(kn);
+      avg += grad(kn, e) * e.dA;
     }
     avg = ar.quo0(avg, by_tot);
 #pragma unroll
-    for (int kn = 0; kn < KGEO; ++kn)
+    for (int kn = 0; kn < KKEEP; ++kn)
       if (kn < nn) avg = minmod(avg, kept[kn]);
-    for (int kn = KGEO; kn < nn; ++kn) {
-      const NbrGeo e = neighbour_geo(ar, G, g0, TG_NBR(kn), cr0, TG_S(kn));
-      avg = minmod(avg, neighbour_grad(ar, G, q, TG_NBR(kn), e, TG_D(kn), p0, m0));
-    }
+    for (int kn = KKEEP; kn < nn; ++kn) avg = minmod(avg, grad(kn, geo(kn)));
     G.gf1n[q * G.NC + g0] = avg;
   }
-#undef TG_NBR
-#undef TG_S
-#undef TG_D
   return !ar.bad();
 }
-GB_HD_OUTLINE void trans_grad_plain(const Grid2 &G, int j, int i) { trans_grad_ops<PlainOps>(G, j, i); }
-GB_HD void trans_grad(const Grid2 &G, int j, int i) {
+template <int BS>
+__device__ __noinline__ void trans_grad_plain(GeoTile<BS> &sm, const Grid2 &G, int j, int i, int q0, int q1) {
+  trans_grad_ops<PlainOps, 1>(sm, G, j, i, q0, q1);
+}
+// Slots [q0, q1) of the cell's gradient.
+template <int UNROLL, int BS>
+__device__ __forceinline__ void trans_grad(GeoTile<BS> &sm, const Grid2 &G, int j, int i, int q0, int q1) {
   if (i >= G.ntrack[j]) return;
   if (j == G.NJ - 1) {  // never recomputed: keeps its copied value
     const long long g0 = (long long)j * G.cap + i;
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) G.gf1n[q * G.NC + g0] = G.gf1[q * G.NC + g0];
+    for (int q = q0; q < q1; ++q) G.gf1n[q * G.NC + g0] = G.gf1[q * G.NC + g0];
     return;
   }
-  if (!trans_grad_ops<FlatOps>(G, j, i)) trans_grad_plain(G, j, i);
+  if (!trans_grad_ops<FlatOps, UNROLL>(sm, G, j, i, q0, q1)) trans_grad_plain(sm, G, j, i, q0, q1);
 }
 
 // ---------------------------------------------------------------------------
@@ -610,29 +701,32 @@ GB_HD void stale_table(const Grid2 &G) {
 
 // Cell cn after f1_if: its own side (flux[1][F1], forward shocks over its
 // upper list) and its other side (flux[0][F1] and reverse shocks, summed over
-// the cells whose upper list holds cn, in the reference's (j, i) order).
-GB_HD void f1_gather(const Phys &ph, const Grid2 &G, int t, int k) {
-  (void)ph;
+// the cells whose upper list holds cn, in the reference's (j, i) order).  The
+// update takes their difference; SPLIT_SIDES keeps each (for diagnostics).
+template <bool SPLIT_SIDES>
+GB_HD void f1_gather(const Grid2 &G, int t, int k) {
   if (k >= G.ntrack[t]) return;
   const long long gn = (long long)t * G.cap + k;
   const long long IC = if_cap(G), IS = (long long)G.NJ * IC;
   double sd = G.sd[gn], ps = G.pspec[gn];
   // the cell's own side: flux[1][F1] and the forward shock tests over its
   // upper list, in order (tracks 0..NJ-2)
+  double hi[NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) hi[q] = 0.;
   if (t <= G.NJ - 2) {
     const int cnt = G.nbr[3 * G.NC + gn], off = G.if_off[gn];
     const long long sl0 = (long long)t * IC + off;
-    double hi[NQ];
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) hi[q] = 0.;
     for (int m = 0; m < cnt && off + m < IC; ++m) {
 #pragma unroll
       for (int q = 0; q < NQ; ++q) hi[q] += G.ifs[q * IS + sl0 + m];
       sd = fmax(sd, G.ifs[NQ * IS + sl0 + m]);
       if (((int)G.ifs[(NQ + 2) * IS + sl0 + m] & 1) && P_SPEC > ps) ps = P_SPEC;
     }
+    if (SPLIT_SIDES) {
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) G.f1hi[q * G.NC + gn] = hi[q];
+      for (int q = 0; q < NQ; ++q) G.f1hi[q * G.NC + gn] = hi[q];
+    }
   }
   double acc[NQ];
 #pragma unroll
@@ -704,7 +798,7 @@ GB_HD void f1_gather(const Phys &ph, const Grid2 &G, int t, int k) {
     if (j >= t) add(j, g0);
   }
 #pragma unroll
-  for (int q = 0; q < NQ; ++q) G.f1lo[q * G.NC + gn] = acc[q];
+  for (int q = 0; q < NQ; ++q) G.f1lo[q * G.NC + gn] = SPLIT_SIDES ? acc[q] : acc[q] - hi[q];
   G.sd[gn] = sd;
   G.pspec[gn] = ps;
 }
@@ -748,8 +842,7 @@ GB_HD void iface_move(const Grid2 &G, int j, int i, int stage) {
 
 // Cell::update (cell.cpp:102-127) of an active cell, the stage's combine and
 // cons2prim; at the last stage (3, or 1 with the Euler module) the particle
-// injection of every cell (run after evolve by Simu::run).  Every cell copies this stage's grad_f1 into the
-// persistent one.
+// injection of every cell (run after evolve by Simu::run).
 // The starting pressure of cons2prim: the cell's previous pressure (the
 // reference's warm start).  With a learned guess (Guess::ON), cons2prim stops
 // at a poor warm start (C2PStats::deferred) and those cells search again from
@@ -816,7 +909,7 @@ GB_HD void cell_advance(Ar &ar, const Phys &ph, const Params2 &P, const Grid2 &G
 #pragma unroll
   for (int q = 0; q < NQ; ++q) c.cons[q] += (G.flx[q * G.NC + g - 1] - G.flx[q * G.NC + g]) * c.dt;
 #pragma unroll
-  for (int q = 0; q < NQ; ++q) c.cons[q] += (G.f1lo[q * G.NC + g] - G.f1hi[q * G.NC + g]) * c.dt;
+  for (int q = 0; q < NQ; ++q) c.cons[q] += G.f1lo[q * G.NC + g] * c.dt;
   c.tj = tgeo(G, j);
   source_terms(ar, ph, c.prim, G0, c.tj, c.dt, c.cons);
   {  // Cell::radiativeSourceTerms
@@ -954,8 +1047,6 @@ GB_HD void update_cell(const Phys &ph, const Params2 &P, const Grid2 &G, int j, 
 #pragma unroll
     for (int q = 0; q < NQ; ++q) G.prim[q * G.NC + g] = prim[q];
   }
-#pragma unroll
-  for (int q = 0; q < NQ; ++q) G.gf1[q * G.NC + g] = G.gf1n[q * G.NC + g];
 }
 
 // ---------------------------------------------------------------------------
