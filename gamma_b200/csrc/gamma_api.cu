@@ -177,10 +177,18 @@ int configure_launch(gamma_ctx *c, int v, bool guess) {
   return GAMMA_OK;
 }
 
+// A batch of states, a root search per thread.  Its warps wait for their own
+// chains of quotients and roots (and for the longest search among their lanes),
+// so warps count more than registers: with 8 blocks per SM (64 registers)
+// 4,194,307 cold starts take 1,092 us and as many warm ones 215 us, unbounded
+// 1,281 and 262 us.  (With the copies of the inputs a cold job takes 1,308 us at
+// 8 blocks, 1,329 at 6, 1,383 at 5, 1,480 at 4, 1,497 unbounded.)
+constexpr int kC2PThreads = 128, kC2PBlocks = 8;
 template <class Cfg>
-__global__ void cons2prim_kernel(const __grid_constant__ gb::Phys ph, double *cons, double *prim, int n, int *iters) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
-    gb::cons2prim_at<Cfg>(ph, cons, prim, n, k, iters, -1.);  // warm start from prim[PPP]
+__global__ void __launch_bounds__(kC2PThreads, kC2PBlocks)
+    cons2prim_kernel(const __grid_constant__ gb::Phys ph, double *cons, double *prim, int n, int *iters) {
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x)
+    gb::cons2prim_at<Cfg>(ph, cons, prim, n, (int)k, iters, -1.);  // warm start from prim[PPP]
 }
 
 // Grid::printCols' side effect with shock detection (text1d.cpp:135-141):
@@ -566,11 +574,11 @@ GAMMA_API int gamma_gpu_cons2prim(const gamma_config_t *cfg, double *cons, doubl
   if (modules < 0 || !cons || !prim || n < 0) return GAMMA_ERR_INVALID;
   if (n == 0) return GAMMA_OK;
   cudaStream_t s = (cudaStream_t)stream;
-  const int bs = 128;
+  const int bs = kC2PThreads;
   int dev = 0, nsm = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const int grid = std::min((n + bs - 1) / bs, nsm * 16);
+  const int grid = (int)std::min((n + (long long)bs - 1) / bs, nsm * kC2PBlocks * 8LL);
   if (modules == gamma_problem::MODULES_SPHERICAL1D)
     cons2prim_kernel<gb::CfgSph><<<grid, bs, 0, s>>>(phys_of(*cfg), cons, prim, n, iters);
   else if (modules == gamma_problem::MODULES_CARTESIAN_REL_CYL)
