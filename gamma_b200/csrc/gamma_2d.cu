@@ -30,21 +30,22 @@ constexpr int kThreads = 256;
 // interfaces (theta) are spread finer (512 tracks: 266 -> 250 us per stage; 16
 // tracks of 400 cells: 17.8 -> 16.9 and 19.1 -> 17.4 us)
 constexpr int kIfaceThreads = 64;
+// The transverse gradients wait on the loads of a slot's neighbours: their
+// registers hold one slot's loads in flight.  Per stage at 512 tracks, with a
+// thread per cell: 376 us with 6 blocks per SM (80 registers; 4: 432, 5: 393, 7:
+// 451; one slot after another with loads only of neighbours that exist, 64
+// registers: 403); with shares of a cell per thread (16 tracks of 3,000 cells)
+// 17.1 us with 4 (3: 21.5, 5: 19.1).
+constexpr int kGradThreads = 128, kGradBlocks = 6, kGradPartBlocks = 4;
 // resident blocks (of kThreads) per SM asked of the heavy per-cell passes.  The
 // interface passes and the cell update are straight-line FP64 code
 // (flat_ops.cuh) that overlaps its own quotients and wants registers: at 512
 // tracks of 4,000 cells, per stage, the r interfaces took 377 us at 2 blocks (3:
 // 411, 4: 470, 1: 591), the theta interfaces 440 us at 2 (3: 538, 4: 602, 1: 615)
-// and the update 307 us at 2 (4: 330).  The transverse gradients wait on loads
-// and want warps: 403 us at 4 (3: 444); so does the theta gather (174 us at 4).
+// and the update 307 us at 2 (4: 330).  The theta gather waits on loads and wants
+// warps: 174 us at 4 (2: 203, 3: 185, 5: 221).
 #ifndef GB2_MINB_MV
 #define GB2_MINB_MV 2
-#endif
-#ifndef GB2_MINB_TG
-#define GB2_MINB_TG 4
-#endif
-#ifndef GB2_TG_UNROLL
-#define GB2_TG_UNROLL 2
 #endif
 #ifndef GB2_MINB_F1
 #define GB2_MINB_F1 2
@@ -284,8 +285,8 @@ __global__ void k_stale(Grid2 G) {
 // PARTS threads per cell, each a share of the slots: whole warps take one share
 // of 32 consecutive cells.
 template <int PARTS>
-__global__ void __launch_bounds__(kThreads, GB2_MINB_TG) k_tgrad(const __grid_constant__ Grid2 G) {
-  __shared__ GeoTile<kThreads> sm;
+__global__ void __launch_bounds__(kGradThreads, PARTS == 1 ? kGradBlocks : kGradPartBlocks) k_tgrad(const __grid_constant__ Grid2 G) {
+  __shared__ GeoTile<kGradThreads> sm;
   constexpr int SLOTS = NQ / PARTS;
   static_assert(NQ % PARTS == 0, "equal shares");
   const long long n = G.pref[G.NJ], m = (n + 31) / 32 * 32 * PARTS;
@@ -295,7 +296,7 @@ __global__ void __launch_bounds__(kThreads, GB2_MINB_TG) k_tgrad(const __grid_co
     if (c >= n) continue;
     int j, i;
     cell_at(G, c, &j, &i);
-    trans_grad<GB2_TG_UNROLL>(sm, G, j, i, part * SLOTS, (part + 1) * SLOTS);
+    trans_grad(sm, G, j, i, part * SLOTS, (part + 1) * SLOTS);
   }
 }
 
@@ -538,13 +539,13 @@ void set_pass_grids(gamma_2d *c) {
   c->grid.cellmv = pass_blocks(c, k_cellmv, kThreads);
   // Threads per cell of the transverse gradients: a grid that leaves the SMs'
   // threads idle shares a cell's slots out (each share forms the geometry).
-  // Measured us per stage with 1, 2, 5 (live cells): 6,400 24.8, 14.2, 8.6; 48,000
-  // 23.7, 17.5, 20.2; 60,000 25.5, 19.0, 24.0; 200,000 53.7, 52.5, 68; 2.05 M 407, 493,
-  // 632.
+  // Measured us per stage with 1, 2, 5 (live cells): 6,400 17.5, 10.4, 7.0; 48,000
+  // 18.2, 16.9, 20.2; 60,000 20.2, 17.1, 23.6; 200,000 42.5, 52.9, 67.9; 2.05 M 375,
+  // 496, 712.
   c->grid.tgrad_parts = c->NC <= c->nsm * 128LL ? 5 : (c->NC <= c->nsm * 1024LL ? 2 : 1);
-  c->grid.tgrad = c->grid.tgrad_parts == 5   ? pass_blocks(c, k_tgrad<5>, kThreads, 0, 5)
-                  : c->grid.tgrad_parts == 2 ? pass_blocks(c, k_tgrad<2>, kThreads, 0, 2)
-                                             : pass_blocks(c, k_tgrad<1>, kThreads);
+  c->grid.tgrad = c->grid.tgrad_parts == 5   ? pass_blocks(c, k_tgrad<5>, kGradThreads, 0, 5)
+                  : c->grid.tgrad_parts == 2 ? pass_blocks(c, k_tgrad<2>, kGradThreads, 0, 2)
+                                             : pass_blocks(c, k_tgrad<1>, kGradThreads);
   c->grid.f1if = pass_blocks(c, k_f1if, kIfaceThreads);
   c->grid.f1gather = pass_blocks(c, k_f1gather<false>, kThreads);
   // one wave: every block ends in a block reduction, and k_dtfinal reads
@@ -600,9 +601,9 @@ int enqueue_step_until(gamma_2d *c, int upto) {
     k_mv<<<c->grid.mv, kIfaceThreads, 0, s>>>(ph, P, G);
     k_cellmv<<<c->grid.cellmv, kThreads, 0, s>>>(G);
     k_stale<<<(c->NJ + 127) / 128, 128, 0, s>>>(G);
-    if (c->grid.tgrad_parts == 5) k_tgrad<5><<<c->grid.tgrad, kThreads, 0, s>>>(G);
-    else if (c->grid.tgrad_parts == 2) k_tgrad<2><<<c->grid.tgrad, kThreads, 0, s>>>(G);
-    else k_tgrad<1><<<c->grid.tgrad, kThreads, 0, s>>>(G);
+    if (c->grid.tgrad_parts == 5) k_tgrad<5><<<c->grid.tgrad, kGradThreads, 0, s>>>(G);
+    else if (c->grid.tgrad_parts == 2) k_tgrad<2><<<c->grid.tgrad, kGradThreads, 0, s>>>(G);
+    else k_tgrad<1><<<c->grid.tgrad, kGradThreads, 0, s>>>(G);
     k_if_scan<<<c->NJ - 1, kThreads, 0, s>>>(G);
     index_tracks(c, G.if_tot, G.NJ - 1, G.if_pref, G.iftrk, nullptr, c->grid.if_groups);  // track NJ-1 owns none
     k_f1if<<<c->grid.f1if, kIfaceThreads, 0, s>>>(ph, G);

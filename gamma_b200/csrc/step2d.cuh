@@ -487,8 +487,9 @@ GB_HD double neighbour_grad(Ar &ar, const Grid2 &G, int q, long long gn, const N
 // slots run one after another over geometry formed once: the first KGEO
 // neighbours' is kept in shared memory (a column per thread; neighbours past
 // KGEO, which are rare, recompute theirs for each slot), one slot's first KKEEP
-// gradients in registers.  Per slot the operations and their order are those of
-// the reference's loops.
+// gradients in registers.  Those neighbours' loads are issued together, whether
+// or not the cell has that many (its own values stand in for the rest).  Per slot
+// the operations and their order are those of the reference's loops.
 constexpr int KGEO = GB2_TG_KGEO, KKEEP = 4;
 
 template <int BS>
@@ -498,7 +499,7 @@ struct GeoTile {
 
 // False where an operand left the range of Ar (grad_f1 of the cell is then to
 // be formed again).
-template <class Ar, int UNROLL, int BS>
+template <class Ar, int BS>
 __device__ __forceinline__ bool trans_grad_ops(GeoTile<BS> &sm, const Grid2 &G, int j, int i, int q0, int q1) {
   Ar ar;
   const int t = threadIdx.x;
@@ -538,16 +539,25 @@ __device__ __forceinline__ bool trans_grad_ops(GeoTile<BS> &sm, const Grid2 &G, 
     return true;
   }
   const auto by_tot = ar.by(dAtot);
-#pragma unroll UNROLL
+  int at[KKEEP];
+#pragma unroll
+  for (int kn = 0; kn < KKEEP; ++kn) at[kn] = kn < nn ? nbr(kn) : (int)g0;
+#pragma unroll 1
   for (int q = q0; q < q1; ++q) {
     const double p0 = G.prim[q * G.NC + g0], m0 = G.gmv[q * G.NC + g0];
     double avg = 0., kept[KKEEP];
     auto grad = [&](int kn, const NbrGeo &e) { return neighbour_grad(ar, G, q, nbr(kn), e, kn < c0 ? d0 : d1, p0, m0); };
+    double pk[KKEEP], mk[KKEEP];
+#pragma unroll
+    for (int kn = 0; kn < KKEEP; ++kn) {
+      pk[kn] = G.prim[q * G.NC + at[kn]];
+      mk[kn] = G.gmv[q * G.NC + at[kn]];
+    }
 #pragma unroll
     for (int kn = 0; kn < KKEEP; ++kn)
       if (kn < nn) {
         const NbrGeo e = geo(kn);
-        kept[kn] = grad(kn, e);
+        kept[kn] = ar.quo0(pk[kn] + mk[kn] * e.dxmR - (p0 + m0 * e.dxmL), kn < c0 ? d0 : d1);
         avg += kept[kn] * e.dA;
       }
     for (int kn = KKEEP; kn < nn; ++kn) {
@@ -565,10 +575,10 @@ __device__ __forceinline__ bool trans_grad_ops(GeoTile<BS> &sm, const Grid2 &G, 
 }
 template <int BS>
 __device__ __noinline__ void trans_grad_plain(GeoTile<BS> &sm, const Grid2 &G, int j, int i, int q0, int q1) {
-  trans_grad_ops<PlainOps, 1>(sm, G, j, i, q0, q1);
+  trans_grad_ops<PlainOps>(sm, G, j, i, q0, q1);
 }
 // Slots [q0, q1) of the cell's gradient.
-template <int UNROLL, int BS>
+template <int BS>
 __device__ __forceinline__ void trans_grad(GeoTile<BS> &sm, const Grid2 &G, int j, int i, int q0, int q1) {
   if (i >= G.ntrack[j]) return;
   if (j == G.NJ - 1) {  // never recomputed: keeps its copied value
@@ -576,7 +586,7 @@ __device__ __forceinline__ void trans_grad(GeoTile<BS> &sm, const Grid2 &G, int 
     for (int q = q0; q < q1; ++q) G.gf1n[q * G.NC + g0] = G.gf1[q * G.NC + g0];
     return;
   }
-  if (!trans_grad_ops<FlatOps, UNROLL>(sm, G, j, i, q0, q1)) trans_grad_plain(sm, G, j, i, q0, q1);
+  if (!trans_grad_ops<FlatOps>(sm, G, j, i, q0, q1)) trans_grad_plain(sm, G, j, i, q0, q1);
 }
 
 // ---------------------------------------------------------------------------
