@@ -367,8 +367,9 @@ void *gamma_gpu_stream(gamma_ctx_t *ctx);
 /* ---- Launch shapes of the step kernel, and their autotuner ------------------
  * No counterpart in the reference (its 1D step is one thread's loop).  A
  * variant fixes the threads that advance one run (the CTA size) and the cells
- * each thread takes per sweep chunk; variant 0 is the default (128 threads,
- * one cell).  Every variant computes every cell the same way, so results are
+ * each thread takes per sweep chunk; variant 0 is the default (one cell per
+ * thread; 128 threads in large batches, more threads, and clusters of CTAs, per
+ * run where runs are few).  Every variant computes every cell the same way, so results are
  * identical; only the speed depends on the batch (track lengths, run count).
  * The step with the learned guess (gamma_gpu_set_guess) has every variant too;
  * the context's variant applies to whichever step runs. */
