@@ -168,12 +168,13 @@ GAMMA_API int gamma_mlp_train(float *params, const float *x, const float *y, lon
     return GAMMA_ERR_INVALID;
   cudaStream_t s = (cudaStream_t)stream;
   const int nsm = sm_count();
-  // m, v, per-epoch loss (zeroed), then the blocks' partial sums
+  // per-epoch loss (64-bit), m, v (zeroed), then the blocks' partial sums
   float *ws = nullptr;
-  const size_t words = 2 * (size_t)NPARAM + (size_t)std::max(tc->epochs, 1);
+  const size_t words = 2 * (size_t)std::max(tc->epochs, 1) + 2 * (size_t)NPARAM;
   const size_t part_words = (size_t)nsm * gb::mlp::NPART;
   if (cudaMalloc(&ws, (words + part_words) * sizeof(float)) != cudaSuccess) return GAMMA_ERR_CUDA;
-  float *m = ws, *v = ws + NPARAM, *loss = ws + 2 * NPARAM, *part = ws + words;
+  double *loss = reinterpret_cast<double *>(ws);
+  float *part = ws + words, *m = part - 2 * NPARAM, *v = part - NPARAM;
   int rc = GAMMA_OK;
   auto check = [&](cudaError_t e) {
     if (e != cudaSuccess && rc == GAMMA_OK) rc = GAMMA_ERR_CUDA;
@@ -183,8 +184,8 @@ GAMMA_API int gamma_mlp_train(float *params, const float *x, const float *y, lon
   check(cudaFuncSetAttribute(gb::mlp::grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const long long steps_per_epoch = (n + tc->batch - 1) / tc->batch;
   const long long total_steps = steps_per_epoch * tc->epochs;
-  const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-  float pb1 = 1.f, pb2 = 1.f;
+  const double b1 = 0.9, b2 = 0.999;
+  double pb1 = 1., pb2 = 1.;
   long long step = 0;
   // multipliers coprime with n (sample order of each epoch)
   static const long long kMul[] = {1000003, 999983, 999979, 999961, 999959, 999953, 999931, 999917};
@@ -210,17 +211,17 @@ GAMMA_API int gamma_mlp_train(float *params, const float *x, const float *y, lon
       const float lr = (float)(tc->lr_final + 0.5 * (tc->lr - tc->lr_final) * (1. + std::cos(M_PI * frac)));
       pb1 *= b1;
       pb2 *= b2;
-      check(launch_chained((NPARAM + 1 + gb::mlp::ADAM_PARAMS - 1) / gb::mlp::ADAM_PARAMS, 256, 0, s,
-                           gb::mlp::adam_kernel, params, part, grid, m, v, lr, b1, b2, eps, 1.f - pb1, 1.f - pb2,
+      check(launch_chained(gb::mlp::ADAM_BLOCKS, 256, 0, s, gb::mlp::adam_kernel, params, part, grid, m, v, lr,
+                           (float)(1. - b1), (float)(1. - b2), 1e-8f, (float)(1. - pb1), (float)(1. - pb2), 0.5 / cnt,
                            loss + e));
     }
   }
   if (rc == GAMMA_OK && loss_per_epoch && tc->epochs > 0) {
-    std::vector<float> h(tc->epochs);
-    check(cudaMemcpyAsync(h.data(), loss, tc->epochs * sizeof(float), cudaMemcpyDeviceToHost, s));
+    std::vector<double> h(tc->epochs);
+    check(cudaMemcpyAsync(h.data(), loss, tc->epochs * sizeof(double), cudaMemcpyDeviceToHost, s));
     check(cudaStreamSynchronize(s));
     // each step added its mini-batch mean loss: the epoch value is their mean
-    for (int e = 0; e < tc->epochs; ++e) loss_per_epoch[e] = h[e] / (float)steps_per_epoch;
+    for (int e = 0; e < tc->epochs; ++e) loss_per_epoch[e] = (float)(h[e] / (double)steps_per_epoch);
   }
   check(cudaStreamSynchronize(s));
   cudaFree(ws);

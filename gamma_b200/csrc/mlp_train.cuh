@@ -85,7 +85,9 @@ __global__ void pairs_kernel(Phys ph, const double *prim, long long n, long long
 // summed index last (so W2, h1 and d2 also transposed), rows padded to 68 floats:
 // a quarter warp's 16-byte loads of consecutive rows then touch all 32 banks.
 // The block's gradient goes to its own row of partial sums, which adam_kernel
-// adds up in a fixed order, so that training repeats bit for bit.
+// adds up in a fixed order, so that training repeats bit for bit.  The loss, the
+// mean of up to millions of squares, is summed in 64 bits from a thread's eight
+// of a tile on.
 // A mini-batch of 8,192 is 128 tiles, one per SM; the products are 0.8 MFLOP of
 // FMA per tile, ~3 us of the SM's FP32 rate, which bounds it (a sample per thread
 // with its activations in local memory took 128 us per mini-batch; now 11 us).
@@ -93,7 +95,8 @@ __global__ void pairs_kernel(Phys ph, const double *prim, long long n, long long
 constexpr int TILE = 64;              // samples per tile
 constexpr int TRAIN_THREADS = 256;
 constexpr int LD = H + 4;             // padded row
-constexpr int NPART = NPARAM + 2;     // a block's partial sums: gradient, loss, padding
+constexpr int NPART = NPARAM + 2;     // a block's partial sums: gradient, then the squared errors (a double)
+static_assert(NPARAM % 2 == 0, "every row's double is 8-byte aligned");
 
 struct TrainSmem {
   float W2[H][LD], W2T[H][LD];        // [o][i] and [i][o]
@@ -102,7 +105,8 @@ struct TrainSmem {
   float x[TILE][4], y[TILE][2];
   float W1[H][3], b1[H], b2[H], W3[2][H], b3[2];
   float red[TRAIN_THREADS / 32][28][16];
-  float red3[TRAIN_THREADS / 32][3];
+  float red3[TRAIN_THREADS / 32][2];
+  double redl[TRAIN_THREADS / 32];
 };
 
 // The kernels of a training run follow one another in a stream, each launched
@@ -179,7 +183,8 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 1)
 
   // gradients of this thread: W2[ty + 16 i][tx + 16 j]; summed over its rows'
   // samples, of unit tx + 16 j: b1, b2, W1[.][3], W3[2][.]; b3, and the loss
-  float gW2[4][4] = {}, gb1[4] = {}, gb2[4] = {}, gW1[4][3] = {}, gW3[2][4] = {}, gb3[2] = {0.f, 0.f}, lsum = 0.f;
+  float gW2[4][4] = {}, gb1[4] = {}, gb2[4] = {}, gW1[4][3] = {}, gW3[2][4] = {}, gb3[2] = {0.f, 0.f};
+  double lsum = 0.;
   const float inv_m = 1.f / (float)m;
 
   for (int base = blockIdx.x * TILE; base < m; base += gridDim.x * TILE) {
@@ -204,7 +209,7 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 1)
     __syncthreads();
     tile_product(sm.h1, sm.W2, tx, ty, z2);
     // output layer: sums over the 16 threads of a row
-    float out[4][2], sg2[4][4];
+    float out[4][2], sg2[4][4], sq = 0.f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       out[i][0] = out[i][1] = 0.f;
@@ -229,7 +234,7 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 1)
         const float e = base + s < m ? out[i][q] + sm.b3[q] - sm.y[s][q] : 0.f;
         dout[q] = e * inv_m;
         if (tx == 0) {
-          lsum += e * e;
+          sq += e * e;
           gb3[q] += dout[q];
         }
       }
@@ -247,6 +252,7 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 1)
         sm.d2T[o][s] = d;
       }
     }
+    lsum += sq;
     __syncthreads();
     tile_product(sm.d2T, sm.h1T, tx, ty, gW2);
     // dL/dz1 = (W2^T dL/dz2) * silu'(z1)
@@ -278,12 +284,13 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 1)
     v[k] += __shfl_xor_sync(0xffffffffu, v[k], 16);
     if ((tid & 31) < 16) sm.red[tid >> 5][k][tx] = v[k];
   }
-  float w[3] = {gb3[0], gb3[1], lsum};
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    w[k] += __shfl_xor_sync(0xffffffffu, w[k], 16);
-    if ((tid & 31) == 0) sm.red3[tid >> 5][k] = w[k];
+  for (int k = 0; k < 2; ++k) {
+    gb3[k] += __shfl_xor_sync(0xffffffffu, gb3[k], 16);
+    if ((tid & 31) == 0) sm.red3[tid >> 5][k] = gb3[k];
   }
+  lsum += __shfl_xor_sync(0xffffffffu, lsum, 16);
+  if ((tid & 31) == 0) sm.redl[tid >> 5] = lsum;
   __syncthreads();
   float *row = part ? part + (size_t)blockIdx.x * NPART : nullptr;
   auto give = [&](int g, float s) {
@@ -306,44 +313,72 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 1)
     else g = OFF_W1 + 3 * (t + 16 * ((q - 16) / 3)) + (q - 16) % 3;
     give(g, s);
   }
-  if (tid < 3) {
+  if (tid < 2) {
     float s = 0.f;
 #pragma unroll
     for (int u = 0; u < TRAIN_THREADS / 32; ++u) s += sm.red3[u][tid];
-    if (tid < 2) give(OFF_B3 + tid, s);
-    else if (row) row[NPARAM] = 0.5f * s * inv_m;
-    else if (loss) atomicAdd(loss, 0.5f * s * inv_m);
+    give(OFF_B3 + tid, s);
+  }
+  if (tid == 2) {
+    double s = 0.;
+#pragma unroll
+    for (int u = 0; u < TRAIN_THREADS / 32; ++u) s += sm.redl[u];
+    if (row) *reinterpret_cast<double *>(row + NPARAM) = s;
+    else if (loss) atomicAdd(loss, (float)(0.5 * s / (double)m));
   }
 }
 
-// The gradient from nb blocks' partial sums, then Adam (Kingma & Ba 2015) with
-// bias corrections bc1 = 1 - b1^t, bc2 = 1 - b2^t; the mini-batch's loss is added
-// to *loss.  Eight threads per parameter, one of every eight blocks' sums each.
+// The gradient from nb blocks' partial sums, then Adam (Kingma & Ba 2015); the
+// mini-batch's loss, inv_2m = 1 / (2 m) times its squared errors, is added to
+// *loss.  c1 = 1 - b1, c2 = 1 - b2 and the bias corrections bc1 = 1 - b1^t,
+// bc2 = 1 - b2^t come from the host, each rounded once from 64 bits: formed in 32
+// bits, 1 - 0.999 is off by 1.3e-5 of itself and the products b2^t by as much in
+// the first steps, the same way in every training.
+// The moments move by c (g - m) for the same reason: b2 itself, in 32 bits, is
+// 1.3e-8 off, 1.3e-5 of its distance from 1.  (The epochs' losses against 64 bits,
+// 700 to 150,007 pairs in batches of 64 to 150,007: off by 2e-7 to 1.4e-6 with the
+// constants formed in 32 bits, by up to 1.3e-7 so.)
+// Eight threads per parameter, one of every eight blocks' sums each; the last block
+// takes the loss (in a parameter's block, its loads would follow theirs: 3% of an
+// epoch's time).
 constexpr int ADAM_PARAMS = 32;  // parameters per block of 256 threads
+constexpr int ADAM_BLOCKS = (NPARAM + ADAM_PARAMS - 1) / ADAM_PARAMS + 1;
 __global__ void __launch_bounds__(256) adam_kernel(float *P, const float *part, int nb, float *m, float *v, float lr,
-                                                   float b1, float b2, float eps, float bc1, float bc2, float *loss) {
+                                                   float c1, float c2, float eps, float bc1, float bc2,
+                                                   double inv_2m, double *loss) {
   __shared__ float red[8][ADAM_PARAMS];
+  __shared__ double redl[8];
   const int t = threadIdx.x & 31, k = threadIdx.x >> 5;
-  const int i = blockIdx.x * ADAM_PARAMS + t;  // NPARAM: the loss
+  const int i = blockIdx.x * ADAM_PARAMS + t;
   launch_next();
   wait_previous();
+  if (blockIdx.x == ADAM_BLOCKS - 1) {
+    double s = 0.;
+    for (int b = threadIdx.x; b < nb; b += 256)
+      s += *reinterpret_cast<const double *>(part + (size_t)b * NPART + NPARAM);
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+    if (t == 0) redl[k] = s;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+#pragma unroll
+    for (int u = 1; u < 8; ++u) s += redl[u];
+    *loss += s * inv_2m;
+    return;
+  }
   float s = 0.f;
-  if (i <= NPARAM) {
+  if (i < NPARAM) {
 #pragma unroll 8
     for (int b = k; b < nb; b += 8) s += part[(size_t)b * NPART + i];
   }
   red[k][t] = s;
   __syncthreads();
-  if (k != 0 || i > NPARAM) return;
+  if (k != 0 || i >= NPARAM) return;
   float g = red[0][t];
 #pragma unroll
   for (int u = 1; u < 8; ++u) g += red[u][t];
-  if (i == NPARAM) {
-    *loss += g;
-    return;
-  }
-  const float mi = b1 * m[i] + (1.f - b1) * g;
-  const float vi = b2 * v[i] + (1.f - b2) * g * g;
+  const float mi = m[i] + c1 * (g - m[i]);
+  const float vi = v[i] + c2 * (g * g - v[i]);
   m[i] = mi;
   v[i] = vi;
   P[i] -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
