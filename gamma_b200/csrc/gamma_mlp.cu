@@ -203,7 +203,7 @@ GAMMA_API int gamma_mlp_train(float *params, const float *x, const float *y, lon
     for (long long b = 0; b < steps_per_epoch && rc == GAMMA_OK; ++b, ++step) {
       const long long start = b * tc->batch;
       const int cnt = (int)std::min<long long>(tc->batch, n - start);
-      const int grid = std::max(1, std::min((cnt + gb::mlp::TILE - 1) / gb::mlp::TILE, nsm));
+      const int grid = (int)std::min<long long>(gb::tile_count(cnt, gb::mlp::TILE), nsm);
       check(launch_chained(grid, gb::mlp::TRAIN_THREADS, smem, s, gb::mlp::grad_kernel, params, x, y, n, mul, add,
                            start, cnt, part, (float *)nullptr, (float *)nullptr));
       // cosine decay from lr to lr_final over all steps
@@ -238,7 +238,7 @@ GAMMA_API int gamma_mlp_loss_grad(const float *params, const float *x, const flo
     return GAMMA_ERR_CUDA;
   if (cudaMemsetAsync(grad, 0, NPARAM * sizeof(float), s) != cudaSuccess) return GAMMA_ERR_CUDA;
   if (loss && cudaMemsetAsync(loss, 0, sizeof(float), s) != cudaSuccess) return GAMMA_ERR_CUDA;
-  const int grid = std::max(1, std::min((n + gb::mlp::TILE - 1) / gb::mlp::TILE, sm_count()));
+  const int grid = (int)std::min<long long>(gb::tile_count(n, gb::mlp::TILE), sm_count());
   // the samples in order (multiplier 1, offset 0), one mini-batch of n
   gb::mlp::grad_kernel<<<grid, gb::mlp::TRAIN_THREADS, smem, s>>>(params, x, y, n, 1, 0, 0, n, nullptr, grad, loss);
   return cudaGetLastError() == cudaSuccess ? GAMMA_OK : GAMMA_ERR_CUDA;

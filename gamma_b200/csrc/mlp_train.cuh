@@ -4,6 +4,7 @@
 #pragma once
 
 #include "mlp.cuh"
+#include "tiles.h"
 
 namespace gb {
 namespace mlp {
@@ -149,8 +150,8 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 1)
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   launch_next();
   // sample s of the block's tile at base: its pair (zeros past the mini-batch)
-  auto load_pair = [&](int base, int s) {
-    const int j = base + s;
+  auto load_pair = [&](long long base, int s) {
+    const long long j = base + s;
     float xi[3] = {0.f, 0.f, 0.f}, yi[2] = {0.f, 0.f};
     if (j < m) {
       const long long k = (long long)(((unsigned long long)perm_mul * (unsigned long long)(start + j) +
@@ -165,7 +166,8 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 1)
     sm.y[s][0] = yi[0];
     sm.y[s][1] = yi[1];
   };
-  if (tid < TILE) load_pair(blockIdx.x * TILE, tid);
+  Tiles tile(m, TILE, blockIdx.x, gridDim.x);
+  if (tid < TILE) load_pair(tile.base, tid);
   wait_previous();  // the parameters
 #pragma unroll
   for (int k = tid; k < H * H; k += TRAIN_THREADS) {
@@ -187,10 +189,10 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 1)
   double lsum = 0.;
   const float inv_m = 1.f / (float)m;
 
-  for (int base = blockIdx.x * TILE; base < m; base += gridDim.x * TILE) {
-    if (base != blockIdx.x * TILE) {
+  for (bool first = true; tile.more(); tile.next(), first = false) {
+    if (!first) {
       __syncthreads();  // the tile before is done with
-      if (tid < TILE) load_pair(base, tid);
+      if (tid < TILE) load_pair(tile.base, tid);
     }
     __syncthreads();
     float ds1[4][4], z2[4][4];  // silu'(z1), z2
@@ -231,7 +233,7 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 1)
       float dout[2];
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
-        const float e = base + s < m ? out[i][q] + sm.b3[q] - sm.y[s][q] : 0.f;
+        const float e = tile.base + s < m ? out[i][q] + sm.b3[q] - sm.y[s][q] : 0.f;
         dout[q] = e * inv_m;
         if (tx == 0) {
           sq += e * e;

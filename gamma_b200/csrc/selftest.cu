@@ -4,6 +4,7 @@
 
 #include "physics.cuh"
 #include "search.cuh"
+#include "tiles.h"
 
 namespace {
 
@@ -131,6 +132,15 @@ __attribute__((visibility("default"))) int gb_selftest_partition_from(unsigned s
     if (got != ref) ++bad;
   }
   return bad;
+}
+
+// gb::Tiles on the host: the tiles that block `block` of `blocks` takes of n
+// items, or -1 where one starts out of range or out of turn.
+__attribute__((visibility("default"))) long long gb_selftest_tiles(int n, int tile, int block, int blocks) {
+  long long taken = 0;
+  for (gb::Tiles t(n, tile, block, blocks); t.more(); t.next(), ++taken)
+    if (t.base != ((long long)block + taken * blocks) * tile || t.base >= n) return -1;
+  return taken;
 }
 
 }  // extern "C"
