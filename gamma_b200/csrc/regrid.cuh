@@ -20,7 +20,8 @@
 //      (a run of original cells, or one new cell).  A merged cell is never
 //      examined itself, so the replay only notes its two cells, and takes its
 //      high-pressure mark to be theirs (where they differ, it is formed at
-//      once);
+//      once; where a merged cell has to be formed during the replay and its mark
+//      is not as assumed, the replay runs again as below);
 //   C. all threads form the merged cells (a merged cell's victim may be a merged
 //      cell: rounds) and compare their marks with the assumed ones; if one
 //      differs, the replay runs again and forms each merged cell as it goes;
@@ -335,8 +336,19 @@ __device__ int regrid_track(double *prim, long long N, double *x, double *dx, do
   const long long noff = 2 * off;
   unsigned long long walk_splits = 0, walk_merges = 0;
 
-  // ---- B. sequential replay (thread 0); eager: each merged cell formed at once
-  auto walk = [&](bool eager) {
+  // the mark of an original or of a split's half, assumed of a cell merged from it
+  auto mark_of = [&](int d) {
+    if (d >= 0) return bit_of(hpw, d);
+    double p[NQ];
+#pragma unroll
+    for (int s = 0; s < NQS; ++s) p[s < 3 ? s : s + 1] = S.nprim[s * 2 * S.N + noff + (-d - 1)];
+    p[UU2] = 0.;
+    return Hooks::regrid_marker(par, p);
+  };
+  // ---- B. sequential replay (thread 0); eager: each merged cell formed at once.
+  // False, and the replay is given up, where a merged cell that has to be formed
+  // in it does not have the mark assumed of it.
+  auto walk = [&](bool eager) -> bool {
     int *seg_start = S.seg_start + 4 * off;
     int *seg_src = S.seg_src + 4 * off;
     int nseg = 0, out = 0, nid = 0;
@@ -379,15 +391,21 @@ __device__ int regrid_track(double *prim, long long N, double *x, double *dx, do
       }
       return c.dx;
     };
-    // form new cell d if it waits (its victim first, and so on down)
-    auto form = [&](int d) {
+    // form new cell d if it waits (its victim first, and so on down); whether
+    // the marks are as assumed
+    auto form = [&](int d) -> bool {
+      bool as_assumed = true;
       while (d < 0 && S.nstate[noff + (-d - 1)] < 0) {
         int t = d;
         for (int v; (v = S.nvic[noff + (-t - 1)]) < 0 && S.nstate[noff + (-v - 1)] < 0;) t = v;
         const long long gid = noff + (-t - 1);
-        form_merged<Cfg, Hooks>(ph, V, S, noff, -t - 1, S.ncur[gid], S.nvic[gid], S.nstate[gid] == kMergeLeft, par);
+        const int c = S.ncur[gid];
+        if (form_merged<Cfg, Hooks>(ph, V, S, noff, -t - 1, c, S.nvic[gid], S.nstate[gid] == kMergeLeft, par) !=
+            mark_of(c))
+          as_assumed = false;
         S.nstate[gid] = 0;
       }
+      return as_assumed;
     };
     auto add_new = [&](const RCell<Cfg> &c) {  // a half of a split cell
       const int id = nid++;
@@ -461,7 +479,7 @@ __device__ int regrid_track(double *prim, long long N, double *x, double *dx, do
       }
 
       if (action == SPLIT && ntrack < cap - 1) {
-        form(prev.d);
+        if (!form(prev.d)) return false;
         RCell<Cfg> A, B;
         split_cells<Cfg>(whole_cell(V, S, noff, prev.d), whole_cell(V, S, noff, curc.d), whole_cell(V, S, noff, k), A,
                          B);
@@ -485,7 +503,7 @@ __device__ int regrid_track(double *prim, long long N, double *x, double *dx, do
         S.nstate[gid] = left ? kMergeLeft : kMergeRight;
         WalkCell M{-(id + 1), width(curc) + width(vic), true, curc.hp};
         if (eager || curc.hp != vic.hp) {
-          form(vic.d);
+          if (!form(vic.d)) return false;
           M.hp = form_merged<Cfg, Hooks>(ph, V, S, noff, id, curc.d, vic.d, left, par);
           S.nstate[gid] = 0;
         }
@@ -518,23 +536,14 @@ __device__ int regrid_track(double *prim, long long N, double *x, double *dx, do
     s_nseg = nseg;
     s_first = first_change;
     s_nid = nid;
-  };
-  // the mark assumed of a merged cell: that of its two cells
-  auto mark_of = [&](int d) {
-    if (d >= 0) return bit_of(hpw, d);
-    double p[NQ];
-#pragma unroll
-    for (int s = 0; s < NQS; ++s) p[s < 3 ? s : s + 1] = S.nprim[s * 2 * S.N + noff + (-d - 1)];
-    p[UU2] = 0.;
-    return Hooks::regrid_marker(par, p);
+    return true;
   };
   for (bool eager = false;; eager = true) {
-    if (threadIdx.x == 0) walk(eager);
-    __syncthreads();
+    bool differs = threadIdx.x == 0 && !walk(eager);
+    if (__syncthreads_or(differs)) continue;
     if (eager) break;
     // ---- C. the merged cells, and whether their marks are as assumed
     const int nid = s_nid;
-    bool differs = false;
     for (int round = 1;; ++round) {
       bool waits = false;
       for (int id = threadIdx.x; id < nid; id += BS) {
