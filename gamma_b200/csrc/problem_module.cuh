@@ -55,9 +55,7 @@ inline int default_shape(int nsm, int nruns, int cells) {
   while (c < 8 && 2LL * c * nruns <= nsm) c *= 2;
   int threads = 128;
   while (threads < most && c * threads < cells) threads *= 2;  // no more than the cells of a run
-  for (int v = 0; v < tune::kVariants; ++v)
-    if (tune::kShapes[v].threads == threads && tune::kShapes[v].cells_per_thread == 1) return v;
-  return 0;
+  return tune::shape_of(threads);
 }
 
 struct ProblemEntry {
@@ -115,6 +113,14 @@ struct ModuleKernel {
     if (GUESS) b = ((b + 15u) & ~size_t(15)) + sizeof(mlp::InferSmem);
     return b;
   }
+  // whether a CTA's shared memory holds it with the regrid words of max_cap cells
+  static bool fits(int dev, int max_cap) {
+    int most = 0;
+    cudaFuncAttributes a{};
+    return cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
+           cudaFuncGetAttributes(&a, (const void *)fn) == cudaSuccess &&
+           smem(max_cap) + a.sharedSizeBytes <= (size_t)most;
+  }
   static cudaError_t configure(int nruns, int cells, int max_cap, LaunchShape *L) {
     L->smem = smem(max_cap);
     cudaError_t e = raise_smem_limit((const void *)fn, L->smem);
@@ -165,6 +171,19 @@ struct ModuleKernel {
 static_assert(tune::kVariants == 8, "GB_MODULE_SHAPES lists every launch shape");
 
 template <class C, class Hooks>
+bool module_fits(int v, bool guess, int dev, int max_cap) {
+  switch (v) {
+#define GB_CASE(k)                                                            \
+  case k:                                                                     \
+    return guess ? ModuleKernel<C, Hooks, k, true>::fits(dev, max_cap) \
+                 : ModuleKernel<C, Hooks, k, false>::fits(dev, max_cap);
+    GB_MODULE_SHAPES(GB_CASE)
+#undef GB_CASE
+  }
+  return false;
+}
+
+template <class C, class Hooks>
 cudaError_t module_configure(int v, bool guess, int nruns, int cells, int max_cap, LaunchShape *L) {
   if (v == 0) {
     int dev = 0, nsm = 0;
@@ -172,6 +191,9 @@ cudaError_t module_configure(int v, bool guess, int nruns, int cells, int max_ca
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
     v = default_shape(nsm, nruns, cells);
+    // A long track's regrid words leave a large CTA no room (512 threads of the
+    // spherical step take 144 KB, 128 take 37 KB): the largest that fits.
+    while (v != 0 && !module_fits<C, Hooks>(v, guess, dev, max_cap)) v = tune::shape_of(tune::kShapes[v].threads / 2);
   }
   switch (v) {
 #define GB_CASE(k)                                                                       \

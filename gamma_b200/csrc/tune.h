@@ -21,6 +21,13 @@ struct Shape {
 // threads per run and cells per thread of each variant
 constexpr Shape kShapes[kVariants] = {{128, 1}, {64, 1}, {256, 1}, {128, 2}, {64, 2}, {128, 4}, {512, 1}, {256, 2}};
 
+// the variant of this many threads with one cell each (0 where there is none)
+constexpr int shape_of(int threads) {
+  for (int v = 0; v < kVariants; ++v)
+    if (kShapes[v].threads == threads && kShapes[v].cells_per_thread == 1) return v;
+  return 0;
+}
+
 // The register cap of each variant keeps the default's resident warps per SM,
 // with at least two CTAs of 256 threads: a run's chunk barriers then stall
 // half an SM, not all of it (the spherical step, 3 x 128 by default, would
