@@ -99,7 +99,7 @@ struct ModuleCfg<gamma_problem::MODULES_CARTESIAN_REL_CYL> {
 // with a refinement criterion only), then the learned guess's weights.
 template <class Hooks>
 __host__ __device__ constexpr unsigned module_words_bytes(int max_cap) {
-  return Hooks::REGRID ? 4u * 4u * (unsigned)regrid_words(max_cap) : 0u;
+  return Hooks::REGRID ? 4u * kRegridMarks * (unsigned)regrid_words(max_cap) : 0u;
 }
 
 template <class C, class Hooks, int V, bool GUESS>

@@ -261,11 +261,13 @@ struct WalkCell {
   bool has_dx, hp;
 };
 
-// Shared-memory words needed by regrid_track for a track of capacity cap.
+// Bit words of one mark per cell of a track of capacity cap, and how many marks
+// regrid_track keeps in shared memory (high-pressure, split, merge).
 __host__ __device__ constexpr int regrid_words(int cap) { return (cap + 31) / 32; }
+constexpr int kRegridMarks = 3;
 
 // Regrid one track; returns the new ntrack.  Called by all threads of the CTA.
-// words: 4 * regrid_words(cap) uint32 of shared memory.
+// words: kRegridMarks * regrid_words(cap) uint32 of shared memory.
 //
 // The criterion: Hooks::check_cell_for_regrid(par, dx, prim, i, iS, rOut) for
 // the cell at live position i, where iS is the live position of the rightmost
@@ -294,7 +296,7 @@ __device__ int regrid_track(double *prim, long long N, double *x, double *dx, do
 
   // ---- A. high-pressure bits and the original shock index
   if (threadIdx.x == 0) s_hpmax = -1;
-  for (int w = threadIdx.x; w < 4 * nw; w += BS) words[w] = 0u;
+  for (int w = threadIdx.x; w < kRegridMarks * nw; w += BS) words[w] = 0u;
   __syncthreads();
   for (int base = 0; base < n; base += BS) {
     const int k = base + threadIdx.x;
