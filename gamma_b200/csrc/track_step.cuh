@@ -922,6 +922,10 @@ __global__ void __launch_bounds__(BS, MINB)
       if (T.run[r].status != 0) break;
       TS::step(T, ph, sm, tm, words, r, st, regrid_only != 0, inf);
     }
+    if (st.status) {  // this run's; the next one starts without it
+      atomicMax(&stats->status, st.status);
+      st.status = 0;
+    }
   }
   // fold the per-thread statistics into the launch totals
   __syncthreads();
@@ -939,7 +943,6 @@ __global__ void __launch_bounds__(BS, MINB)
     if (st.splits) atomicAdd(&stats->splits, st.splits);
     if (st.merges) atomicAdd(&stats->merges, st.merges);
   }
-  if (st.status) atomicMax(&stats->status, st.status);
 }
 
 }  // namespace gb
