@@ -453,7 +453,8 @@ struct gamma_2d {
   int NJ = 0, cap = 0;
   long long NC = 0;
   cudaStream_t stream = nullptr;
-  // a step's graph from either place of the two grad_f1 arrays (Grid2::gf1)
+  // a step's graph from either place of the two grad_f1 arrays: side 0 as in G,
+  // side 1 exchanged (grid_at); side: where the persistent one is now
   cudaGraph_t graph[2] = {};
   cudaGraphExec_t exec[2] = {};
   int side = 0;
@@ -479,6 +480,7 @@ namespace {
 
 int fail(gamma_2d *c, cudaError_t e, const char *what) {
   if (c) c->err = std::string(what) + ": " + cudaGetErrorString(e);
+  (void)cudaGetLastError();  // reported: the next launch's check is not to find it
   return GAMMA_ERR_CUDA;
 }
 #define G2_CUDA(ctx, call)                              \
@@ -572,19 +574,24 @@ void index_tracks(gamma_2d *c, const int *count, int ncount, int *pref, int *grp
   }
 }
 
-// This stage's grad_f1 becomes the persistent one.
-void swap_sides(gamma_2d *c) {
-  std::swap(c->G.gf1, c->G.gf1n);
-  c->side ^= 1;
+// The grid with its persistent grad_f1 in the place of `side`.
+Grid2 grid_at(const gamma_2d *c, int side) {
+  Grid2 G = c->G;
+  if (side) std::swap(G.gf1, G.gf1n);
+  return G;
 }
 
-// One step's launches on the context's stream.  upto > 0 stops after the
-// flux passes of stage `upto` (everything before that stage's collect_dt or
-// update): the diagnostics of gamma_2d_prepare_stage.
-int enqueue_step_until(gamma_2d *c, int upto) {
+// Timestep/euler.cpp or rk3.cpp
+int stages_of(const gamma_2d *c) { return c->cfg.timestep == GAMMA_TS_EULER ? 1 : 3; }
+
+// One step's launches on the context's stream, from `side` on (each stage's
+// grad_f1 becomes the persistent one).  upto > 0 stops after the flux passes of
+// stage `upto` (everything before that stage's collect_dt or update): the
+// diagnostics of gamma_2d_prepare_stage.
+int enqueue_step_until(gamma_2d *c, int side, int upto) {
   const Phys ph = phys_of(c->cfg);
   const Params2 P = params_of(c->par);
-  Grid2 &G = c->G;
+  Grid2 G = grid_at(c, side);
   cudaStream_t s = c->stream;
   if (c->guess) k_guess_policy2<<<1, 1, 0, s>>>(c->d_policy, c->d_stats);
   k_regrid_check<<<1, kThreads, 0, s>>>(P, G, c->d_flags, c->cfg.ngst);
@@ -593,7 +600,7 @@ int enqueue_step_until(gamma_2d *c, int upto) {
     k_regrid_check<<<c->cfg.ntheta - 1, kThreads, 0, s>>>(P, G, c->d_flags, c->cfg.ngst + 1);
     k_regrid<<<c->cfg.ntheta - 1, kThreads, 0, s>>>(ph, P, G, c->d_stats, c->d_flags, c->cfg.ngst + 1, 0);
   }
-  const int nstage = c->cfg.timestep == GAMMA_TS_EULER ? 1 : 3;  // Timestep/euler.cpp or rk3.cpp
+  const int nstage = stages_of(c);
   for (int stage = 1; stage <= nstage; ++stage) {
     k_ghosts_copy<<<ghost_blocks(c, stage == 1), kThreads, 0, s>>>(G, stage == 1);
     k_ghost_cells<<<c->NJ, 32, 0, s>>>(G);
@@ -622,14 +629,15 @@ int enqueue_step_until(gamma_2d *c, int upto) {
     k_update<false><<<c->grid.update, kThreads, 0, s>>>(ph, P, G, stage, c->d_stats, nullptr, pol);
     if (c->guess)
       k_update<true><<<c->grid.update_guess, kThreads, sizeof(mlp::InferSmem), s>>>(ph, P, G, stage, c->d_stats, c->guess, pol);
-    swap_sides(c);
+    std::swap(G.gf1, G.gf1n);
   }
   k_advance<<<1, 32, 0, s>>>(G, c->d_stats);
   G2_CUDA(c, cudaGetLastError());
   return GAMMA_OK;
 }
 
-int enqueue_step(gamma_2d *c) { return enqueue_step_until(c, 0); }
+// An odd number of stages: each step leaves the other side.
+int enqueue_step(gamma_2d *c, int side) { return enqueue_step_until(c, side, 0); }
 
 }  // namespace
 
@@ -826,7 +834,7 @@ GAMMA_API int gamma_2d_upload(gamma_2d_t *ctx, const int *ntrack, const double *
   gamma_2d *c = ctx;
   for (int j = 0; j < c->NJ; ++j)
     if (ntrack[j] > c->cap || ntrack[j] < 2 * c->cfg.ngst + 3) return GAMMA_ERR_CAPACITY;
-  const Grid2 &G = c->G;
+  const Grid2 G = grid_at(c, c->side);
   const size_t NC = (size_t)c->NC, d = sizeof(double);
   cudaStream_t s = c->stream;
   G2_CUDA(c, cudaMemcpyAsync(G.ntrack, ntrack, c->NJ * sizeof(int), cudaMemcpyHostToDevice, s));
@@ -883,32 +891,31 @@ GAMMA_API int gamma_2d_step(gamma_2d_t *ctx, int nsteps, gamma_step_stats_t *sta
   if (c->no_graphs) {  // every launch of every step from the host
     G2_CUDA(c, cudaEventRecord(c->ev0, c->stream));
     for (int k = 0; k < nsteps; ++k) {
-      const int rc = enqueue_step(c);
+      const int rc = enqueue_step(c, c->side);
       if (rc != GAMMA_OK) return rc;
+      c->side ^= 1;
     }
   } else {
-    // a step has an odd number of stages: steps alternate between the two sides
+    // steps alternate between the two sides
     for (int k = 0; k < std::min(nsteps, 2); ++k) {
       const int side = c->side ^ k;
       if (c->exec[side]) continue;
-      if (k) swap_sides(c);
       G2_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-      const int rc = enqueue_step(c);
+      const int rc = enqueue_step(c, side);
       cudaGraph_t g = nullptr;
-      const cudaError_t e = cudaStreamEndCapture(c->stream, &g);
-      while (c->side != (side ^ k)) swap_sides(c);  // as before the capture
-      if (rc != GAMMA_OK) {
+      cudaError_t e = cudaStreamEndCapture(c->stream, &g);
+      if (rc == GAMMA_OK && e == cudaSuccess) e = cudaGraphInstantiate(&c->exec[side], g, 0);
+      if (rc != GAMMA_OK || e != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
-        return rc;
+        c->exec[side] = nullptr;
+        return rc != GAMMA_OK ? rc : fail(c, e, "graph of a step");
       }
-      if (e != cudaSuccess) return fail(c, e, "cudaStreamEndCapture");
       c->graph[side] = g;
-      G2_CUDA(c, cudaGraphInstantiate(&c->exec[side], g, 0));
     }
     G2_CUDA(c, cudaEventRecord(c->ev0, c->stream));
     for (int k = 0; k < nsteps; ++k) {
       G2_CUDA(c, cudaGraphLaunch(c->exec[c->side], c->stream));
-      swap_sides(c);
+      c->side ^= 1;
     }
   }
   G2_CUDA(c, cudaEventRecord(c->ev1, c->stream));
@@ -941,7 +948,7 @@ GAMMA_API int gamma_2d_download(gamma_2d_t *ctx, int *ntrack, double *t, double 
                                 double *grad_f1, int *nbr, double *sd, double *pspec, unsigned char *shocked) {
   if (!ctx) return GAMMA_ERR_INVALID;
   gamma_2d *c = ctx;
-  const Grid2 &G = c->G;
+  const Grid2 G = grid_at(c, c->side);
   const size_t NC = (size_t)c->NC, d = sizeof(double);
   cudaStream_t s = c->stream;
   int st = 0;
@@ -969,9 +976,10 @@ GAMMA_API int gamma_2d_download(gamma_2d_t *ctx, int *ntrack, double *t, double 
 GAMMA_API int gamma_2d_prepare(gamma_2d_t *ctx) { return gamma_2d_prepare_stage(ctx, 1); }
 
 GAMMA_API int gamma_2d_prepare_stage(gamma_2d_t *ctx, int stage) {
-  if (!ctx || stage < 1 || stage > (ctx->cfg.timestep == GAMMA_TS_EULER ? 1 : 3)) return GAMMA_ERR_INVALID;
-  const int rc = enqueue_step_until(ctx, stage);
+  if (!ctx || stage < 1 || stage > stages_of(ctx)) return GAMMA_ERR_INVALID;
+  const int rc = enqueue_step_until(ctx, ctx->side, stage);
   if (rc != GAMMA_OK) return rc;
+  ctx->side ^= (stage - 1) & 1;
   G2_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return GAMMA_OK;
 }
@@ -980,7 +988,7 @@ GAMMA_API int gamma_2d_download_fluxes(gamma_2d_t *ctx, double *v, double *lL, d
                                        double *f1lo, double *f1hi, double *grad_f1_stage) {
   if (!ctx) return GAMMA_ERR_INVALID;
   gamma_2d *c = ctx;
-  const Grid2 &G = c->G;
+  const Grid2 G = grid_at(c, c->side);
   const size_t NC = (size_t)c->NC, d = sizeof(double);
   cudaStream_t s = c->stream;
   if (v) G2_CUDA(c, cudaMemcpyAsync(v, G.v, NC * d, cudaMemcpyDeviceToHost, s));
@@ -1092,7 +1100,7 @@ GAMMA_API int gamma_2d_load(gamma_2d_t *ctx, const char *path) {
     rc = gamma_2d_upload(c, nt.data(), prim.data(), x.data(), dx.data(), dtl.data(), xI.data(), gmv.data(),
                          gf1.data(), nbr.data(), sc[0], it, 0);
   if (rc != GAMMA_OK) return rc;
-  const Grid2 &G = c->G;
+  const Grid2 G = grid_at(c, c->side);
   G2_CUDA(c, cudaMemcpyAsync(G.sd, sd.data(), NC * d, cudaMemcpyHostToDevice, c->stream));
   G2_CUDA(c, cudaMemcpyAsync(G.pspec, ps.data(), NC * d, cudaMemcpyHostToDevice, c->stream));
   G2_CUDA(c, cudaMemcpyAsync(G.shocked, sh.data(), NC, cudaMemcpyHostToDevice, c->stream));
