@@ -458,6 +458,12 @@ struct gamma_2d {
   cudaGraph_t graph[2] = {};
   cudaGraphExec_t exec[2] = {};
   int side = 0;
+  // What gamma_2d_download_fluxes finds.  After a step its last stage's grad_f1 is
+  // the persistent one, and f1lo holds the difference of the two theta fluxes,
+  // which a second gather takes apart when they are asked for, or before an upload
+  // replaces the lists that it goes by (keeping them apart in each step's last stage
+  // would cost 1.1% of the 512-track jet's step).
+  bool stage_persists = false, f1_joined = false;
   bool no_graphs = false;  // gamma_2d_use_graphs(ctx, 0): launch each step's kernels directly
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   std::vector<void *> allocs;
@@ -633,6 +639,15 @@ int enqueue_step_until(gamma_2d *c, int side, int upto) {
   }
   k_advance<<<1, 32, 0, s>>>(G, c->d_stats);
   G2_CUDA(c, cudaGetLastError());
+  return GAMMA_OK;
+}
+
+// f1lo and f1hi of the last step's last stage, each by itself
+int take_f1_apart(gamma_2d *c) {
+  if (!c->f1_joined) return GAMMA_OK;
+  k_f1gather<true><<<c->grid.f1gather, kThreads, 0, c->stream>>>(c->G);
+  G2_CUDA(c, cudaGetLastError());
+  c->f1_joined = false;
   return GAMMA_OK;
 }
 
@@ -834,6 +849,12 @@ GAMMA_API int gamma_2d_upload(gamma_2d_t *ctx, const int *ntrack, const double *
   gamma_2d *c = ctx;
   for (int j = 0; j < c->NJ; ++j)
     if (ntrack[j] > c->cap || ntrack[j] < 2 * c->cfg.ngst + 3) return GAMMA_ERR_CAPACITY;
+  if (c->stage_persists) {  // the last stage's stays beside the new persistent one
+    c->side ^= 1;
+    c->stage_persists = false;
+  }
+  const int rc = take_f1_apart(c);
+  if (rc != GAMMA_OK) return rc;
   const Grid2 G = grid_at(c, c->side);
   const size_t NC = (size_t)c->NC, d = sizeof(double);
   cudaStream_t s = c->stream;
@@ -894,6 +915,7 @@ GAMMA_API int gamma_2d_step(gamma_2d_t *ctx, int nsteps, gamma_step_stats_t *sta
       const int rc = enqueue_step(c, c->side);
       if (rc != GAMMA_OK) return rc;
       c->side ^= 1;
+      c->stage_persists = c->f1_joined = true;
     }
   } else {
     // steps alternate between the two sides
@@ -916,6 +938,7 @@ GAMMA_API int gamma_2d_step(gamma_2d_t *ctx, int nsteps, gamma_step_stats_t *sta
     for (int k = 0; k < nsteps; ++k) {
       G2_CUDA(c, cudaGraphLaunch(c->exec[c->side], c->stream));
       c->side ^= 1;
+      c->stage_persists = c->f1_joined = true;
     }
   }
   G2_CUDA(c, cudaEventRecord(c->ev1, c->stream));
@@ -980,6 +1003,7 @@ GAMMA_API int gamma_2d_prepare_stage(gamma_2d_t *ctx, int stage) {
   const int rc = enqueue_step_until(ctx, ctx->side, stage);
   if (rc != GAMMA_OK) return rc;
   ctx->side ^= (stage - 1) & 1;
+  ctx->stage_persists = ctx->f1_joined = false;
   G2_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return GAMMA_OK;
 }
@@ -991,13 +1015,18 @@ GAMMA_API int gamma_2d_download_fluxes(gamma_2d_t *ctx, double *v, double *lL, d
   const Grid2 G = grid_at(c, c->side);
   const size_t NC = (size_t)c->NC, d = sizeof(double);
   cudaStream_t s = c->stream;
+  if (f1lo || f1hi) {
+    const int rc = take_f1_apart(c);
+    if (rc != GAMMA_OK) return rc;
+  }
   if (v) G2_CUDA(c, cudaMemcpyAsync(v, G.v, NC * d, cudaMemcpyDeviceToHost, s));
   if (lL) G2_CUDA(c, cudaMemcpyAsync(lL, G.lL, NC * d, cudaMemcpyDeviceToHost, s));
   if (lR) G2_CUDA(c, cudaMemcpyAsync(lR, G.lR, NC * d, cudaMemcpyDeviceToHost, s));
   if (flux) G2_CUDA(c, cudaMemcpyAsync(flux, G.flx, NQ * NC * d, cudaMemcpyDeviceToHost, s));
   if (f1lo) G2_CUDA(c, cudaMemcpyAsync(f1lo, G.f1lo, NQ * NC * d, cudaMemcpyDeviceToHost, s));
   if (f1hi) G2_CUDA(c, cudaMemcpyAsync(f1hi, G.f1hi, NQ * NC * d, cudaMemcpyDeviceToHost, s));
-  if (grad_f1_stage) G2_CUDA(c, cudaMemcpyAsync(grad_f1_stage, G.gf1n, NQ * NC * d, cudaMemcpyDeviceToHost, s));
+  if (grad_f1_stage)
+    G2_CUDA(c, cudaMemcpyAsync(grad_f1_stage, c->stage_persists ? G.gf1 : G.gf1n, NQ * NC * d, cudaMemcpyDeviceToHost, s));
   G2_CUDA(c, cudaStreamSynchronize(s));
   return GAMMA_OK;
 }

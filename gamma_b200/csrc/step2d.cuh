@@ -70,7 +70,8 @@ struct Grid2 {
   double *gmv, *gf1, *gf1n;
   int *nbr;                  // [4][NC]: first id and count towards track j-1, then j+1
   double *cons0, *dV0;       // [NQ][NC], [NC]: S0.cons and G0.dV (copyState0)
-  double *f1lo, *f1hi;       // [NQ][NC]: flux[0][F1] - flux[1][F1]; for diagnostics each of them
+  // [NQ][NC]: flux[0][F1] - flux[1][F1]; for gamma_2d_download_fluxes each of them
+  double *f1lo, *f1hi;
   // interfaces
   double *xI, *xI0, *xIm;    // position, step-start position, position after the stage's move
   double *v, *lL, *lR;
@@ -712,7 +713,8 @@ GB_HD void stale_table(const Grid2 &G) {
 // Cell cn after f1_if: its own side (flux[1][F1], forward shocks over its
 // upper list) and its other side (flux[0][F1] and reverse shocks, summed over
 // the cells whose upper list holds cn, in the reference's (j, i) order).  The
-// update takes their difference; SPLIT_SIDES keeps each (for diagnostics).
+// update takes their difference; SPLIT_SIDES keeps each.  All else that it
+// writes comes out the same when it runs again after the update.
 template <bool SPLIT_SIDES>
 GB_HD void f1_gather(const Grid2 &G, int t, int k) {
   if (k >= G.ntrack[t]) return;

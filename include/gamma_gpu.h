@@ -354,6 +354,7 @@ int gamma_2d_prepare(gamma_2d_t *ctx);
  * before it complete (updates and combines), then that stage's updateGhosts
  * and prepForUpdate.  stage 1 is gamma_2d_prepare. */
 int gamma_2d_prepare_stage(gamma_2d_t *ctx, int stage);
+/* After gamma_2d_step: those of its last stage. */
 int gamma_2d_download_fluxes(gamma_2d_t *ctx, double *v, double *lL, double *lR, double *flux, double *f1lo,
                              double *f1hi, double *grad_f1_stage);
 
