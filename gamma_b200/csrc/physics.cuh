@@ -502,9 +502,10 @@ GB_HD C2PRoot c2p_pressure_body(Ar &ar, const Phys &ph, double D, double S, doub
     // lfac^2 = E^2 / (E^2 - S^2): certainly not negative, whatever its rounding
     // (lfac carries eps E^2 / (E^2 - S^2)), where D^2 stays that much below
     // E^2 - S^2, as it does unless the gas is colder than p/rho ~ 1e-14 lfac^2;
-    // then f need not be formed (2 quotients and 2 roots of every search).
+    // then f need not be formed (2 quotients and 2 roots of every search).  (The
+    // squares must not lose digits to underflow.)
     bool find_p = true;
-    const bool surely = p_lo == 0. && D * D <= (E - S) * (E + S) - 0x1p-47 * (E * E);
+    const bool surely = p_lo == 0. && E * E >= 0x1p-900 && D * D <= (E - S) * (E + S) - 0x1p-47 * (E * E);
     if (!surely && feval(p_lo, true).f < 0) find_p = false;
     double p_hi;
     if (e0.f < 0) {
