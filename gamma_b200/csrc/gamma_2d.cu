@@ -195,7 +195,7 @@ __device__ __forceinline__ int track_at(const int *pref, int NJ, long long g) {
 // element's track is then at most a few steps past its group's (one step per
 // track that starts inside the group).  Each block scans the tracks itself, in
 // shared memory, so that one launch does both (a launch is 2 to 3 us of a small
-// grid's step, which has 16 per stage); block 0 keeps the prefix.  With more
+// grid's step, which has 13 per stage); block 0 keeps the prefix.  With more
 // tracks than fit there (SHARED false) the prefix is one launch of one block
 // (grp null) and the groups another (count null).  clear: a word per track to
 // zero.
@@ -546,8 +546,10 @@ void set_pass_grids(gamma_2d *c) {
   c->grid.mv = pass_blocks(c, k_mv, kIfaceThreads);
   c->grid.cellmv = pass_blocks(c, k_cellmv, kThreads);
   // Threads per cell of the transverse gradients: a grid that leaves the SMs'
-  // threads idle shares a cell's slots out (each share forms the geometry).
-  // Measured us per stage with 1, 2, 5 (live cells): 6,400 17.5, 10.4, 7.0; 48,000
+  // threads idle shares a cell's slots out (each share forms the geometry).  The
+  // rule goes by the capacity: the live cells, fewer by up to the room left for
+  // splits, are known on the device only.  Measured us per stage with 1, 2, 5 (live
+  // cells, of capacities near them): 6,400 17.5, 10.4, 7.0; 48,000
   // 18.2, 16.9, 20.2; 60,000 20.2, 17.1, 23.6; 200,000 42.5, 52.9, 67.9; 2.05 M 375,
   // 496, 712.
   c->grid.tgrad_parts = c->NC <= c->nsm * 128LL ? 5 : (c->NC <= c->nsm * 1024LL ? 2 : 1);

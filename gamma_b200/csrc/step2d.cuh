@@ -38,9 +38,6 @@
 namespace gb {
 namespace d2 {
 
-#ifndef GB2_TG_KGEO
-#define GB2_TG_KGEO 6
-#endif
 constexpr int KMAX_STALE = 8;  // foreign stale contributors per target track
 // a theta interface's results: flux[NQ], forward Sd, reverse Sd, flags (1: the
 // forward test reached the spectral index, 2: the reverse one)
@@ -85,7 +82,7 @@ struct Grid2 {
                              // 41: a track's theta interfaces exceed if_cap
   double *red;               // partial minima of dt_loc
   int *pref;                 // [NJ+1] cells of tracks before j (the live-cell index)
-  int *gtrk;                 // [NC/32+2] track of live cell 32k (k_group_tracks)
+  int *gtrk;                 // [NC/32+2] track of live cell 32k (k_index)
   // theta interfaces, owned by the cells of track j (j <= NJ-2) through their
   // upper lists, numbered per track in cell order (k_if_scan):
   double *ifs;               // [IF_WORDS][NJ * if_cap]: interface results, track j from j * if_cap
@@ -93,7 +90,7 @@ struct Grid2 {
   int *if_own;               // [NJ * if_cap]: the owning cell (index in its track) of each interface
   int *if_tot;               // [NJ]: interfaces of each track
   int *if_pref;              // [NJ+1]: interfaces of the tracks before j
-  int *iftrk;                // [(NJ-1) if_cap/32 + 2] track of interface 32k (k_if_group_tracks)
+  int *iftrk;                // [(NJ-1) if_cap/32 + 2] track of interface 32k (k_index)
   // regrid scratch (one track of records per track)
   double *rprim, *rgmv, *rgf1;  // [NQ][NC]
   double *rx, *rdx, *rdtl, *rxI;
@@ -491,7 +488,7 @@ GB_HD double neighbour_grad(Ar &ar, const Grid2 &G, int q, long long gn, const N
 // gradients in registers.  Those neighbours' loads are issued together, whether
 // or not the cell has that many (its own values stand in for the rest).  Per slot
 // the operations and their order are those of the reference's loops.
-constexpr int KGEO = GB2_TG_KGEO, KKEEP = 4;
+constexpr int KGEO = 6, KKEEP = 4;
 
 template <int BS>
 struct GeoTile {

@@ -20,9 +20,10 @@
 // chunk starts at the interface on its left, which its neighbour computes too
 // (the same bits); the two cells beyond either end are read before any CTA
 // updates (halo), and the CTAs wait for one another twice per stage.
-// Measured at 20 steps a call, one B200: 12 tubes of 1,001 to 8,191 cells take
-// 1,951 us per step with a CTA each and 102 us with 8, one tube of 500 cells 131
-// and 48 us, one BM1D run of 2,000 initial cells 560 and 107 us.
+// Measured us of the kernel per step, one B200, the same formulas: 12 tubes of
+// 1,001 to 8,191 cells 1,305 with a CTA of 128 threads each and 80 with 8 of 512,
+// one tube of 500 cells 90.6 and 46, one BM1D run of 2,000 initial cells 393 and
+// 103.
 // (A segment per warp, whose warps wait only twice per stage, is slower: 4,096
 // tubes 3.97 against 3.58 ms per step, the BM1D sweep 1.82 against 1.38 ms.  The
 // warps drift apart and no longer share the instruction cache.)
@@ -887,8 +888,8 @@ struct TrackStep {
 // chose this kernel, the one with (nonzero) or without (0) the learned guess.
 template <class Cfg, class Hooks, int BS, bool GUESS = false, int CPT = 1, int MINB = Cfg::MIN_BLOCKS>
 __global__ void __launch_bounds__(BS, MINB)
-    track_step_kernel(const __grid_constant__ Tracks T, const __grid_constant__ Phys ph, int nsteps, const int *order, int nruns, int *queue, StepStats *stats,
-                      int regrid_only, unsigned words_bytes, const int *gate) {
+    track_step_kernel(const __grid_constant__ Tracks T, const __grid_constant__ Phys ph, int nsteps, const int *order,
+                      int nruns, int *queue, StepStats *stats, int regrid_only, unsigned words_bytes, const int *gate) {
   if (gate && ((*gate != 0) != GUESS)) return;
   using TS = TrackStep<Cfg, Hooks, BS, GUESS, CPT>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
