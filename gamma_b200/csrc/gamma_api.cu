@@ -772,6 +772,9 @@ GAMMA_API int gamma_gpu_autotune(gamma_ctx_t *ctx, int nsteps, float *ms, int *c
   const int keep = ctx->variant;
   int best = keep, rc = GAMMA_OK;
   float best_ms = 0.f;
+  // a context's first step with a guess set runs with the network (k_guess_policy):
+  // untimed, lest the first shape alone be charged with it
+  if (e == cudaSuccess && ctx->T.mlp && (rc = run_steps(ctx, 1, nullptr, 0)) == GAMMA_OK) e = copy_all(true);
   for (int v = 0; v < gb::tune::kVariants && rc == GAMMA_OK && e == cudaSuccess; ++v) {
     if ((rc = gamma_gpu_set_variant(ctx, v)) != GAMMA_OK) break;
     // nsteps launches of one step, as a caller stepping one at a time makes them
