@@ -303,12 +303,14 @@ GAMMA_API int gamma_gpu_create(const gamma_config_t *cfg, int nruns, const int *
     GB_ALLOC(S.ndtl, 2 * N * d);
     GB_ALLOC(S.nrifx, 2 * N * d);
     GB_ALLOC(S.nrif, 2 * N * sizeof(int));
-    GB_ALLOC(S.ncur, 2 * N * sizeof(int));
-    GB_ALLOC(S.nvic, 2 * N * sizeof(int));
-    GB_ALLOC(S.nstate, 2 * N * sizeof(int));
     GB_ALLOC(S.seg_start, 4 * N * sizeof(int));
     GB_ALLOC(S.seg_src, 4 * N * sizeof(int));
     GB_ALLOC(S.tprim, nqs * N * d);
+    // the merged cells' notes, done with before the compaction starts, in its first
+    // rows (a run's 2 cap ints from 2 off lie over its own cap doubles from off)
+    S.ncur = reinterpret_cast<int *>(S.tprim);
+    S.nvic = reinterpret_cast<int *>(S.tprim + N);
+    S.nstate = reinterpret_cast<int *>(S.tprim + 2 * N);
     GB_ALLOC(S.tx, N * d);
     GB_ALLOC(S.tdx, N * d);
     GB_ALLOC(S.tdtl, N * d);

@@ -42,8 +42,9 @@ struct RegridScratch {
   int *nrif;                        // [2N] right interface: original index, or -1 (then nrifx)
   int *ncur, *nvic;                 // [2N] a merged cell's two cells: original index, or -(id+1)
   int *nstate;                      // [2N] the round that formed the cell, or kMergeLeft / kMergeRight
+                                    // (these three share memory with tprim)
   int *seg_start, *seg_src;         // [4N] at 4*off[r]: output position; src >= 0 original, else -(id+1)
-  double *tprim;                    // [NQS][N] compaction target
+  double *tprim;                    // [NQS][N] compaction target (step D)
   double *tx, *tdx, *tdtl, *txI;    // [N]
   long long N;
 };
