@@ -370,10 +370,12 @@ void *gamma_gpu_stream(gamma_ctx_t *ctx);
  * variant fixes the threads that advance one run (the CTA size) and the cells
  * each thread takes per sweep chunk; variant 0 is the default (one cell per
  * thread; 128 threads in large batches, more threads, and clusters of CTAs, per
- * run where runs are few).  Every variant computes every cell the same way, so results are
- * identical; only the speed depends on the batch (track lengths, run count).
+ * run where runs are few and the regrid's words leave room for them).  Every
+ * variant computes every cell the same way, so results are identical; only the
+ * speed depends on the batch (track lengths, run count).
  * The step with the learned guess (gamma_gpu_set_guess) has every variant too;
- * the context's variant applies to whichever step runs. */
+ * the context's variant applies to whichever step runs.  gamma_gpu_variant_info
+ * of variant 0 gives the shape that the default takes in large batches. */
 int gamma_gpu_variant_info(int variant, int *threads, int *cells_per_thread);
 int gamma_gpu_set_variant(gamma_ctx_t *ctx, int variant);
 int gamma_gpu_get_variant(const gamma_ctx_t *ctx);
